@@ -15,6 +15,7 @@
 
 #include "ddg.h"
 #include "ddg_kernel.cuh"
+#include "ddg_warp_kernel.cuh"
 
 using namespace ddg;
 
@@ -44,6 +45,7 @@ struct ddg_solver {
   ddg_config cfg;
   int device = 0, lanes = 0, block = 128, sms = 0;
   const KVariant* variant = nullptr;
+  bool by_warp = false;  // searched by warp_kernel (see warp_route), else by the variant's kernel
   TTBucket* tt = nullptr;
   Frame* stacks = nullptr;
   u32* lane_gen = nullptr;
@@ -73,7 +75,7 @@ struct ddg_solver {
   cudaGraphExec_t graph = nullptr;
   const void* graph_key[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   int64_t graph_n = -1;
-  int graph_grid = 0;
+  int graph_grid = 0, graph_block = 0;
 };
 
 extern "C" {
@@ -141,6 +143,18 @@ static const KVariant* find_variant(int block, int minb, int schedule) {
   for (const KVariant& v : kVariants)
     if (v.block == block && v.minb == minb && v.schedule == schedule) return &v;
   return nullptr;
+}
+
+// One warp per search (warp_kernel) unless the configuration asks for helping or names a
+// launch shape, schedule or packing of the lane-per-thread kernels, which only those have.
+static bool warp_route(const ddg_config& c) {
+#ifdef DDG_TT_SIG
+  (void)c;
+  return false;
+#else
+  return c.block == 512 && c.min_blocks == 1 && c.schedule == 0 && !c.help && !c.phase_spread && !c.cheap_limit &&
+         !c.flat_moves && !c.free_below && !c.free_steps && !c.free_pack;
+#endif
 }
 
 static int occupancy_blocks(const KVariant* v) {
@@ -243,8 +257,23 @@ int ddg_solver_create(const ddg_config* cfg_in, ddg_solver** out) {
     return fail(DDG_E_MEMORY, "no room for one block of lanes");
   }
   s->lanes = (int)lanes;
+  s->by_warp = warp_route(cfg);
+#ifndef DDG_TT_SIG
+  if (s->by_warp) {
+    e = cudaFuncSetAttribute((const void*)warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)warp_smem(WARP_MAX));
+    if (e != cudaSuccess) {
+      delete s;
+      return fail(DDG_E_CUDA, "warp kernel: %s", cudaGetErrorString(e));
+    }
+  }
+#endif
   size_t tt_bytes = (size_t)lanes * ((size_t)sizeof(TTBucket) << cfg.tt_log2);
   size_t st_bytes = (size_t)lanes * sizeof(Frame) * STACK_DEPTH;
+#ifndef DDG_TT_SIG
+  if (s->by_warp)  // a searcher's frames leave shared memory only between slices
+    st_bytes = (size_t)std::min<long long>(lanes, (long long)s->sms * WARP_MAX) * sizeof(WarpFrame) * STACK_DEPTH;
+#endif
   e = cudaMalloc(&s->tt, tt_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&s->stacks, st_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&s->lane_gen, (size_t)lanes * 4);
@@ -285,18 +314,34 @@ int ddg_solver_set_job_starts(ddg_solver* s, uint64_t* d_job_start_ns) {
 uint64_t ddg_solver_nodes(const ddg_solver* s) { return s ? s->total_nodes : 0; }
 int64_t ddg_solver_bytes(const ddg_solver* s) { return s ? (int64_t)s->bytes : 0; }
 
-static int launch_batch(ddg_solver* s, const BatchArgs& a, long long n_jobs, cudaStream_t stream,
-                        int* grid_out) {
+// Launches the solve; `block_out` gets the threads per block, `sms` the SMs it may use.
+static int launch_batch(ddg_solver* s, const BatchArgs& a, cudaStream_t stream, int sms, int* grid_out,
+                        int* block_out) {
+  BatchArgs args = a;
+  void* params[] = {&args};
+#ifndef DDG_TT_SIG
+  if (s->by_warp) {
+    // One block per SM, the lanes' TT slices spread over them; a batch with fewer jobs than
+    // that takes fewer searchers (a stream's jobs are yet to come).
+    const long long want = a.ring || a.n_jobs > s->lanes ? s->lanes : a.n_jobs;
+    const int grid = (int)std::min<long long>(sms, want);
+    const int warps = (int)std::min<long long>(WARP_MAX, a.ring ? want / grid : (want + grid - 1) / grid);
+    const int fit = s->lanes / grid;  // every searcher has a lane
+    const int use = warps < fit ? warps : fit;
+    args.rr_jobs = a.ring ? 0 : std::min<long long>(a.n_jobs, (long long)grid * use);
+    *grid_out = grid;
+    *block_out = use * 32;
+    CUDA_TRY(cudaLaunchKernel((const void*)warp_kernel, dim3(grid), dim3(use * 32), params, warp_smem(use), stream));
+    return DDG_OK;
+  }
+#endif
   // Every lane is launched: the first jobs are dealt round-robin over the blocks, so a small
   // batch spreads over all SMs (lanes without a job end at once, or help with helping on).
-  (void)n_jobs;
-  int grid = (int)((s->lanes + s->block - 1) / s->block);
-  if (grid < 1) grid = 1;
-  *grid_out = grid;
-  BatchArgs args = a;
+  const int grid = std::max(1, (s->lanes + s->block - 1) / s->block);
   const long long lanes = (long long)grid * s->block;
   args.rr_jobs = a.ring ? 0 : (a.n_jobs < lanes ? a.n_jobs : lanes);
-  void* params[] = {&args};
+  *grid_out = grid;
+  *block_out = s->block;
   CUDA_TRY(cudaLaunchKernel((const void*)s->variant->fn, dim3(grid), dim3(s->block), params, s->variant->smem,
                             stream));
   return DDG_OK;
@@ -339,7 +384,7 @@ static BatchArgs make_args(ddg_solver* s, const uint64_t* d_hands, int64_t n, co
 }
 
 // Counters of the last launch into `st` (and the solver's node total). Returns the words.
-static int read_stats(ddg_solver* s, int grid, ddg_stats* st, unsigned long long* c) {
+static int read_stats(ddg_solver* s, int grid, int block, ddg_stats* st, unsigned long long* c) {
   CUDA_TRY(cudaMemcpy(c, s->counters, CNT_WORDS * 8, cudaMemcpyDeviceToHost));
   s->total_nodes += c[CNT_NODES];
   if (c[CNT_FAULTS])
@@ -374,8 +419,8 @@ static int read_stats(ddg_solver* s, int grid, ddg_stats* st, unsigned long long
   CUDA_TRY(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
   st->kernel_ms = ms;
   st->grid = grid;
-  st->block = s->block;
-  st->lanes = grid * s->block;
+  st->block = block;
+  st->lanes = s->lanes;
   return DDG_OK;
 }
 
@@ -425,14 +470,14 @@ int ddg_solve_device_ex(ddg_solver* s, const uint64_t* d_hands, int64_t n, const
   if (s->d_job_end_ns) CUDA_TRY(cudaMemsetAsync(s->d_job_end_ns, 0, (size_t)a.n_jobs * 8, stream));
   if (s->d_job_start_ns) CUDA_TRY(cudaMemsetAsync(s->d_job_start_ns, 0, (size_t)a.n_jobs * 8, stream));
   CUDA_TRY(cudaEventRecord(s->ev0, stream));
-  int grid = 0;
-  int rc = launch_batch(s, a, a.n_jobs, stream, &grid);
+  int grid = 0, block = 0;
+  int rc = launch_batch(s, a, stream, s->sms, &grid, &block);
   if (rc) return rc;
   CUDA_TRY(cudaEventRecord(s->ev1, stream));
   rc = wait_launch(s);
   if (rc) return rc;
   unsigned long long c[CNT_WORDS];
-  return read_stats(s, grid, st, c);
+  return read_stats(s, grid, block, st, c);
 }
 
 int ddg_solve_graph(ddg_solver* s, const uint64_t* d_hands, int64_t n, const int8_t* d_seed20, uint8_t* d_out20,
@@ -458,7 +503,7 @@ int ddg_solve_graph(ddg_solver* s, const uint64_t* d_hands, int64_t n, const int
     a.job_end_ns = s->d_job_end_ns;
     a.job_start_ns = s->d_job_start_ns;
     cudaGraph_t g = nullptr;
-    int grid = 0, rc = DDG_OK;
+    int grid = 0, block = 0, rc = DDG_OK;
     cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->counters, 0, CNT_WORDS * 8, cap);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_out20, 0xFF, (size_t)n * 20, cap);
@@ -466,7 +511,7 @@ int ddg_solve_graph(ddg_solver* s, const uint64_t* d_hands, int64_t n, const int
     if (e == cudaSuccess && s->d_job_end_ns) e = cudaMemsetAsync(s->d_job_end_ns, 0, (size_t)a.n_jobs * 8, cap);
     if (e == cudaSuccess && s->d_job_start_ns)
       e = cudaMemsetAsync(s->d_job_start_ns, 0, (size_t)a.n_jobs * 8, cap);
-    if (e == cudaSuccess) rc = launch_batch(s, a, a.n_jobs, cap, &grid);
+    if (e == cudaSuccess) rc = launch_batch(s, a, cap, s->sms, &grid, &block);
     cudaError_t e2 = cudaStreamEndCapture(cap, &g);
     if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess && rc == DDG_OK) e = cudaGraphInstantiate(&s->graph, g, 0);
@@ -484,6 +529,7 @@ int ddg_solve_graph(ddg_solver* s, const uint64_t* d_hands, int64_t n, const int
     s->graph_key[3] = s->d_job_end_ns;
     s->graph_key[4] = s->d_job_start_ns;
     s->graph_grid = grid;
+    s->graph_block = block;
   }
   *(volatile int*)s->h_stop = 0;
   CUDA_TRY(cudaEventRecord(s->ev0, stream));
@@ -492,7 +538,7 @@ int ddg_solve_graph(ddg_solver* s, const uint64_t* d_hands, int64_t n, const int
   int rc = wait_launch(s);
   if (rc) return rc;
   unsigned long long c[CNT_WORDS];
-  return read_stats(s, s->graph_grid, st, c);
+  return read_stats(s, s->graph_grid, s->graph_block, st, c);
 }
 
 int ddg_solve_begin(ddg_solver* s, const uint64_t* d_hands, int64_t n, const int8_t* d_seed20, uint8_t* d_out20,
@@ -546,13 +592,13 @@ int ddg_solve_continue(ddg_solver* s, double seconds, const uint64_t* hands_host
   CUDA_TRY(cudaEventRecord(s->ev0, stream));
   if (hands_host)  // the caller's deals again (pinned memory makes this an async copy)
     CUDA_TRY(cudaMemcpyAsync((void*)a.hands, hands_host, (size_t)s->slice_n * 32, cudaMemcpyHostToDevice, stream));
-  int grid = 0;
+  int grid = 0, block = 0;
   if (!s->slice_done) {
     // Every counter but the job queue's head starts again at zero.
     CUDA_TRY(cudaMemsetAsync(s->counters + 1, 0, (CNT_WORDS - 1) * 8, stream));
     *(volatile int*)s->h_stop = 0;
     a.slice_ns = (u64)(seconds * 1e9);
-    int rc = launch_batch(s, a, a.n_jobs, stream, &grid);
+    int rc = launch_batch(s, a, stream, s->sms, &grid, &block);
     if (rc) return rc;
   }
   if (out20_host)
@@ -566,7 +612,7 @@ int ddg_solve_continue(ddg_solver* s, double seconds, const uint64_t* hands_host
   }
   s->slice_args.resume = 1;
   unsigned long long c[CNT_WORDS];
-  rc = read_stats(s, grid, st, c);
+  rc = read_stats(s, grid, block, st, c);
   if (rc) return rc;
   if ((long long)c[CNT_BLOCKS_DONE] == grid) s->slice_done = true;
   if (finished) *finished = s->slice_done ? 1 : 0;
@@ -656,8 +702,8 @@ static int stream_kernel(ddg_stream* st) {
     a.hint20 = st->d_hint;
   }
   *(volatile int*)s->h_stop = 0;
-  int grid = 0;
-  int rc = launch_batch(s, a, (long long)s->lanes, st->kstream, &grid);
+  int grid = 0, block = 0;
+  int rc = launch_batch(s, a, st->kstream, st->guide ? s->sms - 2 : s->sms, &grid, &block);
   if (rc) return rc;
   CUDA_TRY(cudaEventRecord(st->kdone, st->kstream));
   st->launched = true;
@@ -930,14 +976,14 @@ static int solve_one(ddg_solver* s, const uint64_t* hands4, int strain, int decl
   if (s->tasks) CUDA_TRY(cudaMemset(s->tasks, 0, s->tasks_bytes));
   *(volatile int*)s->h_stop = 0;
   CUDA_TRY(cudaEventRecord(s->ev0, nullptr));
-  int grid = 0;
-  rc = launch_batch(s, a, 1, nullptr, &grid);
+  int grid = 0, block = 0;
+  rc = launch_batch(s, a, nullptr, s->sms, &grid, &block);
   if (rc) return rc;
   CUDA_TRY(cudaEventRecord(s->ev1, nullptr));
   rc = wait_launch(s);
   if (rc) return rc;
   unsigned long long c[CNT_WORDS];
-  rc = read_stats(s, grid, nullptr, c);
+  rc = read_stats(s, grid, block, nullptr, c);
   if (rc) return rc;
   CUDA_TRY(cudaMemcpy(out20, s->d_out, 20, cudaMemcpyDeviceToHost));
   return DDG_OK;

@@ -155,6 +155,24 @@ __device__ __forceinline__ bool stop_requested(const BatchArgs& a, u64 t_end) {
   return (a.stop && *a.stop) || (t_end && global_ns() > t_end);
 }
 
+// Stream: counts a finished job of `deal`; the last one writes the deal's completion record.
+__device__ __noinline__ void stream_deal_done(const BatchArgs& a, long long deal) {
+  const long long slot = deal & a.ring_mask;
+  __threadfence();  // this job's answers before the count
+  if (atomicAdd(a.deal_done + slot, 1) != a.jpd - 1) return;
+  __threadfence();  // every job's answers are visible now
+  const volatile uint8_t* o = a.out20 + slot * 20;
+  const unsigned long long idx = atomicAdd(a.comp_tail, 1ull);
+  volatile CompRec* r = a.comp + (idx & (unsigned long long)a.ring_mask);
+  r->seq = (unsigned long long)deal;
+  for (int k = 0; k < 20; k++) r->tricks[k] = o[k];
+  // The slot's count is reset before the flag lets the host free the slot: a job of the
+  // next deal in this slot must not find the old count.
+  a.deal_done[slot] = 0;
+  __threadfence_system();  // the record and the reset before the flag
+  r->flag = (unsigned)idx + 1u;
+}
+
 struct DevEnv {
   const BatchArgs* a;
   Frame* stack;
@@ -284,24 +302,7 @@ struct DevEnv {
     if (a->job_nodes) a->job_nodes[L.job] = c->s.nodes - c->start_nodes;
     if (a->job_end_ns) a->job_end_ns[L.job] = global_ns();
     c->jobs_done++;
-    if (a->ring) stream_job_done(L);
-  }
-  // Stream: the lane that finishes a deal's last job writes its completion record.
-  __device__ __noinline__ void stream_job_done(const Lane& L) {
-    const long long slot = L.deal & a->ring_mask;
-    __threadfence();  // this job's answers before the count
-    if (atomicAdd(a->deal_done + slot, 1) != a->jpd - 1) return;
-    __threadfence();  // every job's answers are visible now
-    const volatile uint8_t* o = a->out20 + slot * 20;
-    const unsigned long long idx = atomicAdd(a->comp_tail, 1ull);
-    volatile CompRec* r = a->comp + (idx & (unsigned long long)a->ring_mask);
-    r->seq = (unsigned long long)L.deal;
-    for (int k = 0; k < 20; k++) r->tricks[k] = o[k];
-    // The slot's count is reset before the flag lets the host free the slot: a job of the
-    // next deal in this slot must not find the old count.
-    a->deal_done[slot] = 0;
-    __threadfence_system();  // the record and the reset before the flag
-    r->flag = (unsigned)idx + 1u;
+    if (a->ring) stream_deal_done(*a, L.deal);
   }
 };
 

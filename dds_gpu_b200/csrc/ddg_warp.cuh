@@ -1,0 +1,1185 @@
+// The search of one job by one warp: every node's work is spread over the 32 threads.
+//
+// A position is held suit by suit. Thread t stands for suit s = t & 3 and seat
+// p = (t >> 2) & 3 (the upper half-warp repeats the lower one) and keeps the 13-bit mask
+// of the cards seat p holds in suit s; sets of cards (relevant, tried, in play) are kept
+// as one 13-bit mask per suit, the same in every thread of that suit. So suit lengths are
+// one popcount for all sixteen holdings, playing a card is one masked XOR, a set is one
+// 32-bit register, and nothing but the transposition table's key needs 64-bit words. What
+// a node does per suit (owner codes, top cards, widening the relevant cards), per table
+// way (tags, entries) or per candidate (weights, skipping small cards) runs side by side
+// in the threads that stand for it; what is one decision (trick winner, bounds, the next
+// move) is the same scalar code in all threads. The stack of frames lies in shared memory.
+//
+// Decisions, their order and the table's contents are those of ddg_search.cuh (and of the
+// reference, src/dd.h:613-939), so node counts per job are equal, node for node; a host
+// emulation of the warp (tests/native/warp_replay.cpp) checks it on the CPU.
+#pragma once
+#include "ddg_search.cuh"
+
+#ifndef DDG_TT_SIG
+
+namespace ddg {
+
+#ifdef __CUDACC__
+#define DDG_W __device__ __forceinline__
+DDG_W u32 w_ballot(bool p) { return __ballot_sync(0xFFFFFFFFu, p); }
+DDG_W u32 w_shfl(u32 v, int src) { return __shfl_sync(0xFFFFFFFFu, v, src); }
+DDG_W u32 w_shfl_up1(u32 v) { return __shfl_up_sync(0xFFFFFFFFu, v, 1); }
+DDG_W u32 w_or(u32 v) { return __reduce_or_sync(0xFFFFFFFFu, v); }
+DDG_W u32 w_max(u32 v) { return __reduce_max_sync(0xFFFFFFFFu, v); }
+DDG_W u32 w_min(u32 v) { return __reduce_min_sync(0xFFFFFFFFu, v); }
+DDG_W u32 w_add(u32 v) { return __reduce_add_sync(0xFFFFFFFFu, v); }
+DDG_W void w_sync() { __syncwarp(); }
+DDG_W int w_top(u32 x) { return 31 - __clz((int)x); }   // highest set bit, -1 for 0
+DDG_W int w_low(u32 x) { return __ffs((int)x) - 1; }    // lowest set bit, -1 for 0
+DDG_W int w_popc(u32 x) { return __popc(x); }
+#else  // the host emulation provides the collectives (warp_emu.hpp)
+#define DDG_W static inline
+DDG_W int w_top(u32 x) { return x ? 31 - __builtin_clz(x) : -1; }
+DDG_W int w_low(u32 x) { return x ? __builtin_ctz(x) : -1; }
+DDG_W int w_popc(u32 x) { return __builtin_popcount(x); }
+#endif
+
+// One level of the search in shared memory.
+struct alignas(16) WarpFrame {
+  struct {
+    u32 at;    // relevant cards gathered so far | cards tried << 16
+    u32 code;  // owner code before this frame's card was played
+  } suit[4];
+  u32 trick, info;  // the trick before this frame's card; w_open_info()
+  uint16_t all[4];  // a frame that completed a trick: the cards in play at the trick's start
+  uint8_t mv[16];   // candidates, best first
+};
+static_assert(sizeof(WarpFrame) == 64, "a frame is two 32-byte halves");
+
+// Counters, one to a thread.
+enum { WCNT_PROBES = 0, WCNT_HITS = 1, WCNT_STORES = 2, WCNT_READS = 3, WCNT_BYTES = 4, WCNT_BOUNDS = 5, WCNT_COUNT = 6 };
+
+// A searcher's job, root search and totals: read and written at root searches only.
+struct WarpJob {
+  long long job, deal;
+  u64 start_nodes, nodes;  // node totals at the job's start / now (flushed)
+  u64 total[WCNT_COUNT];   // the threads' counters (flushed)
+  u32 jobs_done;
+  int8_t strain, decl, last_decl, mode, lo, hi, cards, stage;
+};
+
+struct WarpMem {
+  WarpFrame fr[STACK_DEPTH];
+  uint8_t scratch[16];  // candidates before they are ordered
+  WarpJob job;
+};
+
+// Registers of a searcher. The same in all threads, unless marked: [s] per suit, [sp] per
+// (suit, seat), [t] per thread.
+struct WarpState {
+  u32 m;      // [sp] cards of the seat in the suit
+  u32 all;    // [s] cards in play at the start of the trick
+  u32 now;    // [s] cards still in a hand
+  u32 code;   // [s] owners of those, two bits each, the highest card's at the top of the word
+  u32 rel;    // [s] relevant cards of the node just finished
+  u32 at;     // [s] top frame's relevant cards | tried cards << 16
+  u32 cnt;    // [t] counter of thread WCNT_*
+  u32 trick;  // cards of the trick, a byte each (bytes from nplayed on are 0)
+  u32 info;   // top frame's info word
+  int trump, leader, nplayed, left;
+  int need;      // tricks NS still need
+  int sp;        // depth of the top frame
+  u32 nodes;     // nodes since the last flush
+  u32 gen;
+};
+
+struct WarpIds {  // what a thread stands for
+  int t, s, p;
+};
+
+DDG_W void w_count(WarpState& w, const WarpIds& id, int what, u32 k) {
+  if (id.t == what) w.cnt += k;
+}
+
+// ---- key and owner codes -------------------------------------------------------------------
+
+struct WarpKey {
+  u64 q;
+  u32 lens_hi, lens_lo;  // length_key()
+  u32 bucket, tag;
+};
+
+// Suit lengths of all hands and their hash (make_key): one popcount for the 16 holdings,
+// two OR reductions for the 64-bit word.
+DDG_W WarpKey w_key(const WarpState& w, const WarpIds& id, u32 mask) {
+  WarpKey k;
+  const u32 part = (u32)w_popc(w.m) << (28 - 16 * (id.p & 1) - 4 * id.s);
+  k.lens_hi = w_or(id.p < 2 ? part : 0);
+  k.lens_lo = w_or(id.p >= 2 ? part : 0);
+  const u64 x = key_hash((u64)k.lens_hi << 32 | k.lens_lo, w.leader);
+  k.bucket = (u32)x & mask;
+  k.q = (x >> 9) & ((1ull << Q_BITS) - 1);
+  k.tag = ((u32)(x >> 32) & 0xFFFF0000u) | ((u32)w.left << 12) | (w.gen << 2) | (u32)w.leader;
+  return k;
+}
+
+// Owner code of this thread's suit from the hands (a job's start; then w_play keeps it).
+DDG_W u32 w_build_code(const WarpState& w, const WarpIds& id) {
+  u32 h[4], code = 0;
+  for (int q = 0; q < 4; q++) h[q] = w_shfl(w.m, 4 * q + id.s);
+  int at = 32;
+  for (int r = 12; r >= 0; r--)
+    for (u32 q = 0; q < 4; q++)
+      if (h[q] >> r & 1 && at > 0) code |= q << (at -= 2);
+  return code;
+}
+// The owners of the highest n cards, lowest card in the low bits (n = 0: 0).
+DDG_W u32 w_pattern(u32 code, int n) { return (code >> 1) >> (31 - 2 * n); }
+
+// The top n cards of a suit.
+DDG_W u32 w_top_n(u32 all, int n) {
+  int r = 0;
+#pragma unroll
+  for (int step = 8; step; step >>= 1)
+    if (w_popc(all >> (r + step)) >= n) r += step;
+  return (all >> r) << r;
+}
+
+// ---- transposition table -------------------------------------------------------------------
+
+// The probe (tt_probe): thread t looks at tag t & 15; those that match read and check
+// their entries side by side. Returns 1, 0 (rel set) or -1 (hint set).
+DDG_W int w_probe(WarpState& w, const WarpIds& id, const TTBucket* b, u32 tagw, const WarpKey& k, u32 code, int need,
+                  int& hint) {
+  hint = -1;
+  const bool match = id.t < TT_WAYS && (tagw & ~0xF00u) == k.tag;
+  const u32 mm = w_ballot(match);
+  w_count(w, id, WCNT_PROBES, 1);
+  if (!mm) return -1;
+  u32 codes[4];
+#pragma unroll
+  for (int s = 0; s < 4; s++) codes[s] = w_shfl(code, s);
+  bool same = false, decides = false, holds = false;
+  int best = 63;
+  u32 counts = 0;
+  if (match) {
+    u64 w0, w1;
+    entry_load(b, (int)((tagw >> 8) & 15), w0, w1);
+    counts = (u32)w1 & 0xFFFFu;
+    // Tag, bucket and q are the whole hash of the suit lengths, a bijection, so an entry
+    // with this q has these lengths: its counts are no longer than the suits.
+    const int n0 = (int)(counts & 15), n1 = (int)(counts >> 4 & 15), n2 = (int)(counts >> 8 & 15);
+    u64 mine = w_pattern(codes[3], (int)(counts >> 12));
+    mine = mine << (2 * n2) | w_pattern(codes[2], n2);
+    mine = mine << (2 * n1) | w_pattern(codes[1], n1);
+    mine = mine << (2 * n0) | w_pattern(codes[0], n0);
+    same = (w0 & ((1ull << Q_BITS) - 1)) == k.q && mine == ((w1 >> 16) | ((w0 >> 53) << 48));
+    const int lb = (int)((w0 >> Q_BITS) & 15), ub = (int)((w0 >> (Q_BITS + 4)) & 15);
+    best = (int)((w0 >> (Q_BITS + 8)) & 63);
+    holds = lb >= need;
+    decides = same && (holds || ub < need);
+  }
+  const u32 dec = w_ballot(decides), up = w_ballot(decides && holds);
+  const u32 before = dec ? (dec & (0u - dec)) - 1 : 0xFFFFu;  // the ways read ahead of the deciding one
+  const u32 hints = w_ballot(same && best != 63) & before;
+  w_count(w, id, WCNT_READS, (u32)w_popc(mm & (before << 1 | 1)));
+  if (dec) {
+    const int at = w_low(dec);
+    const u32 c = w_shfl(counts, at);
+    w.rel = w_top_n(w.all, (int)(c >> (4 * id.s)) & 15);
+    w_count(w, id, WCNT_HITS, 1);
+    return (int)((up >> at) & 1);
+  }
+  if (hints) hint = (int)w_shfl((u32)best, w_top(hints));
+  return -1;
+}
+
+// The store (tt_store) of bounds [lb, ub] for the class of positions that share the
+// relevant cards `rel`: each suit's thread makes its owner pattern, each way's thread
+// checks its entry, and the tag line shifts by one shuffle.
+DDG_W void w_store(WarpState& w, const WarpIds& id, TTBucket* b, u32 tagw, const WarpKey& k, u32 code, u32 rel, int lb,
+                   int ub, int best) {
+  const int above = rel ? w_popc(w.all >> w_low(rel)) : 0;  // cards at or above the lowest relevant one
+  const u32 counts = w_or((u32)above << (4 * id.s));
+  const int n0 = (int)(counts & 15), n1 = (int)(counts >> 4 & 15), n2 = (int)(counts >> 8 & 15);
+  if (n0 + n1 + n2 + (int)(counts >> 12) > MAX_REL) return;
+  const int off = (id.s > 0 ? n0 : 0) + (id.s > 1 ? n1 : 0) + (id.s > 2 ? n2 : 0);
+  const u64 mine = (u64)w_pattern(code, above) << (2 * off);
+  const u64 owners = (u64)w_or((u32)(mine >> 32)) << 32 | w_or((u32)mine);
+  const u64 w1 = (u64)counts | owners << 16;
+  const u32 hi = (u32)(owners >> 48);
+  const bool match = id.t < TT_WAYS && (tagw & ~0xF00u) == k.tag;
+  const u32 mm = w_ballot(match);
+  w_count(w, id, WCNT_STORES, 1);
+  bool same = false;
+  u32 old = 0;
+  if (match) {
+    u64 e0, e1;
+    entry_load(b, (int)((tagw >> 8) & 15), e0, e1);
+    same = (e0 & ((1ull << Q_BITS) - 1)) == k.q && e1 == w1 && (u32)(e0 >> 53) == hi;
+    old = (u32)(e0 >> Q_BITS) & 0x3FFFu;  // lb:4 | ub:4 | best:6
+  }
+  const u32 sm = w_ballot(same);
+  int way;
+  if (sm) {  // the class has an entry: the first one is narrowed in place
+    const int at = w_low(sm);
+    old = w_shfl(old | ((tagw >> 8) & 15) << 16, at);
+    way = (int)(old >> 16);
+    const int olb = (int)(old & 15), oub = (int)(old >> 4 & 15), obest = (int)(old >> 8 & 63);
+    lb = olb > lb ? olb : lb;
+    ub = oub < ub ? oub : ub;
+    best = best < 0 ? obest : best;
+    w_count(w, id, WCNT_BYTES, 64 + 16 * (u32)w_popc(mm & ((sm & (0u - sm)) * 2 - 1)) + 8);
+  } else {
+    w_count(w, id, WCNT_BYTES, 64 + 16 * (u32)w_popc(mm) + 64 + 16);
+    // The way (take_way): the first empty one, else the least 2 * tricks left + age, other
+    // generations first; of equal ones the oldest.
+    const int age = TT_WAYS - 1 - (id.t & 15);
+    const u32 empty = w_ballot(id.t < TT_WAYS && tagw == 0);
+    const u32 v = ((tagw >> 2) & 63) != w.gen ? 0 : 1 + 2 * ((tagw >> 12) & 15) + (u32)age;
+    const int pos = empty ? TT_WAYS - 1 : TT_WAYS - 1 - (int)(w_min(v << 4 | (u32)age) & 15);
+    way = empty ? w_low(empty) : (int)((w_shfl(tagw, pos) >> 8) & 15);
+    const u32 prev = w_shfl_up1(tagw);
+    if (id.t <= pos) b->tag[id.t] = id.t == 0 ? (k.tag | (u32)way << 8) : prev;
+  }
+  if (id.t == TT_WAYS)
+    entry_store(b, way, k.q | (u64)((u32)lb | (u32)ub << 4 | (u32)(best < 0 ? 63 : best) << 8 | hi << 14) << Q_BITS, w1);
+  w_sync();
+}
+
+// ---- the top cards of every suit, relative to the leader ------------------------------------
+
+// Per suit, in its threads: lengths of leader, left, partner, right (4 bits each), holders
+// of the top three cards relative to the leader (0..3, REL_NONE = no such card; 4 bits
+// each from bit 16), and the cards' ranks.
+enum { REL_NONE = 4, REL_L = 1, REL_P = 2, REL_R = 3 };
+struct WarpTop {
+  u32 a, ranks;
+};
+DDG_W int rt_len(u32 a, int who) { return (int)(a >> (4 * who)) & 15; }
+DDG_W int rt_win(u32 a) { return (int)(a >> 16) & 15; }
+DDG_W int rt_sec(u32 a) { return (int)(a >> 20) & 15; }
+DDG_W int rt_thr(u32 a) { return (int)(a >> 24) & 15; }
+DDG_W int rt_rank(u32 r, int k) { return (int)(r >> (4 * k)) & 15; }
+
+DDG_W WarpTop w_make_top(const WarpState& w, const WarpIds& id, const WarpKey& k) {
+  const int sh = 12 - 4 * id.s;  // lengths of seats 0..3 in this suit, then rotated to the leader
+  const u32 l = ((k.lens_hi >> (sh + 16)) & 15) | ((k.lens_hi >> sh) & 15) << 4 | ((k.lens_lo >> (sh + 16)) & 15) << 8 |
+                ((k.lens_lo >> sh) & 15) << 12;
+  WarpTop t;
+  t.a = ((l | l << 16) >> (4 * w.leader)) & 0xFFFFu;
+  t.ranks = 0;
+  u32 a = w.all;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const u32 c = (u32)w_top(a) & 15;
+    const u32 who = a ? ((w.code >> (30 - 2 * j)) - (u32)w.leader) & 3 : (u32)REL_NONE;
+    t.ranks |= c << (4 * j);
+    t.a |= who << (16 + 4 * j);
+    a &= ~(1u << c);
+  }
+  return t;
+}
+
+// ---- QuickTricks and LaterTricks (ddg_bounds.cuh, the same decisions in the same order) ------
+
+struct QtIn {  // one suit as QuickTricks sees it
+  int own, lho, part, rho, win, sec, thr;
+  u32 ranks;
+};
+DDG_W QtIn w_qt_in(u32 a, u32 ranks) {
+  QtIn q;
+  q.own = rt_len(a, 0);
+  q.lho = rt_len(a, REL_L);
+  q.part = rt_len(a, REL_P);
+  q.rho = rt_len(a, REL_R);
+  q.win = rt_win(a);
+  q.sec = rt_sec(a);
+  q.thr = rt_thr(a);
+  q.ranks = ranks;
+  return q;
+}
+
+// One holding side's tricks of a suit whose top card it holds: `a` holds it, `b` is its
+// partner (qt_lead_side / qt_lead_plain for the leader, qt_partner_* over the entry).
+// side: a side suit of a trump contract. draws: cashing draws the opponents' trumps.
+DDG_W int w_qt_suit(const QtIn& c, const WarpIds& id, int suit, bool lead, bool side, bool draws, int cutoff, int& lhoT,
+                    int& rhoT, int comm_suit, u32 entry, int qt, u32& wr, int& res) {
+  const int a = lead ? c.own : c.part, b = lead ? c.part : c.own;
+  const int first = lead ? 0 : REL_P, other = lead ? REL_P : 0;
+  const bool out = lhoT == 0 && rhoT == 0;  // both opponents are out of trumps
+  const bool clear = !side || out;
+  const u32 mine = id.s == suit ? 0xFFFFFFFFu : 0u;
+  res = QT_STOP;
+  if (!side || ((c.lho != 0 || lhoT == 0) && (c.rho != 0 || rhoT == 0))) {
+    wr |= (1u << rt_rank(c.ranks, 0) & mine) | entry;
+    if (++qt >= cutoff) return qt;
+    if (draws) {
+      lhoT = lhoT > 0 ? lhoT - 1 : 0;
+      rhoT = rhoT > 0 ? rhoT - 1 : 0;
+    }
+    if (c.lho <= 1 && c.rho <= 1 && b <= 1 && clear) {
+      qt += a - 1;
+      if (qt >= cutoff) return qt;
+      res = QT_NEXT;
+      return qt;
+    }
+  }
+  const bool run = c.sec == first, both = c.sec == other && a > 1 && b > 1;
+  if (run || both) {
+    if (clear) {
+      wr |= (1u << rt_rank(c.ranks, 1) & mine) | (side ? entry : 0);
+      if (++qt >= cutoff) return qt;
+      if (draws) {
+        lhoT = lhoT > 0 ? lhoT - 1 : 0;
+        rhoT = rhoT > 0 ? rhoT - 1 : 0;
+      }
+      if (c.lho <= 2 && c.rho <= 2 && (b <= 2 || (both && a <= 2))) {
+        qt += (run || a > b ? a : b) - 2;
+        if (qt >= cutoff) return qt;
+        res = QT_NEXT;
+        return qt;
+      }
+    }
+  } else if (!lead && suit == comm_suit && c.sec == REL_L &&
+             (!side || ((c.lho >= 2 || lhoT == 0) && (c.rho >= 2 || rhoT == 0)))) {
+    if (c.thr == REL_P) {
+      wr |= (1u << rt_rank(c.ranks, 2) & mine) | (side ? entry : 0);
+      if (++qt >= cutoff) return qt;
+      if (c.own <= 2 && c.lho <= 2 && c.rho <= 2 && clear) {
+        qt += c.part - 2;
+        if (qt >= cutoff) return qt;
+      }
+    }
+  }
+  res = QT_STAY;
+  return qt;
+}
+
+// QuickTricks (quick_tricks_impl): the leading side's sure tricks against `cutoff`;
+// decided = the answer is known (a count > 0: the leading side makes it).
+DDG_W int w_quick_tricks(const WarpState& w, const WarpIds& id, const WarpTop& top, int cutoff, int cutoff_other, u32& wr,
+                         bool& decided) {
+  const int trump = w.trump;
+  wr = 0;
+  decided = true;
+  const bool has_t = trump >= 0;
+  const u32 ta = has_t ? w_shfl(top.a, trump) : 0;
+  const int tl = rt_len(ta, REL_L), tr = rt_len(ta, REL_R);
+  // The entry to partner: every suit's thread tests its suit, the first in order is taken.
+  const bool safe = !has_t || ((rt_len(top.a, REL_L) != 0 || tl == 0) && (rt_len(top.a, REL_R) != 0 || tr == 0));
+  const bool by_win = rt_win(top.a) == REL_P && rt_len(top.a, 0) != 0;
+  const bool by_sec = rt_sec(top.a) == REL_P && rt_win(top.a) == 0 && rt_len(top.a, 0) >= 2 && rt_len(top.a, REL_P) >= 2;
+  const u32 entries = w_ballot(id.t < 4 && id.s != trump && safe && (by_win || by_sec));
+  int comm_suit = w_low(entries);
+  if (comm_suit < 0 && has_t && rt_len(ta, 0) != 0 && rt_win(ta) == REL_P) comm_suit = trump;
+  const bool comm = comm_suit >= 0;
+  u32 entry = 0;  // [s] the entry card
+  if (id.s == comm_suit) entry = 1u << rt_rank(top.ranks, by_win ? 0 : 1);
+  // in the trump suit the entry is partner's top card, which by_win says as well
+  int qt = 0, suit = has_t ? trump : 0, lhoT = tl, rhoT = tr;
+  bool ruffed = false;
+  for (; suit <= 3; suit = qt_next_suit(suit, trump)) {
+    const QtIn c = w_qt_in(w_shfl(top.a, suit), w_shfl(top.ranks, suit));
+    const bool side = has_t && trump != suit;
+    const bool opps = (c.lho | c.rho) != 0;
+    const bool no_ruff = !side || (lhoT == 0 && rhoT == 0);
+    if (!opps) {
+      if (c.part == 0) {  // only the leader holds the suit
+        if (c.own != 0 && no_ruff) {
+          qt += c.own;
+          if (qt >= cutoff) return qt;
+        }
+        continue;
+      }
+      // The sure length of the partnership's suit may decide at once (qt_blocked_sum).
+      const bool only_part = comm && c.own == 0;
+#pragma unroll
+      for (int pass = 0; pass < 2; pass++) {
+        const bool by_lead = pass == 0;
+        if (!by_lead && (!comm || only_part)) continue;
+        int sum;
+        bool hit = false;
+        if (has_t && suit == trump) {
+          sum = c.own > c.part ? c.own : c.part;
+          const bool longer = by_lead ? c.own >= c.part : c.own <= c.part;
+          const int l0 = rt_len(top.a, 0), l2 = rt_len(top.a, REL_P);
+          const bool shortness = by_lead ? (l0 > 0 && l2 == 0) : (l2 > 0 && l0 == 0);
+          const u32 any = w_ballot(id.s != trump && shortness);
+          if (sum > 0 && longer && any) sum++;
+          hit = sum >= cutoff;
+        } else {
+          sum = c.own < c.part ? c.own : c.part;
+          if (no_ruff) hit = sum >= cutoff;
+        }
+        if (hit) {
+          if (!by_lead && has_t && suit == trump) wr |= entry;
+          return sum;
+        }
+      }
+      if (only_part) {  // only partner holds it: cashed over the entry
+        if (no_ruff) {
+          qt += c.part;
+          wr |= entry;
+          if (qt >= cutoff) return qt;
+        }
+        continue;
+      }
+    }
+    if (c.win == REL_NONE) continue;
+    int res = QT_STAY;
+    if (c.win == 0 || (c.win == REL_P && comm)) {
+      const bool lead = c.win == 0, draws = lead && has_t && trump == suit && suit != comm_suit;
+      qt = w_qt_suit(c, id, suit, lead, side, draws, cutoff, lhoT, rhoT, comm_suit, lead ? 0u : entry, qt, wr, res);
+    }
+    if (res == QT_STOP) return qt;
+    if (res == QT_NEXT) continue;
+    // A ruff by partner.
+    if (side && c.own > 0 && !ruffed && c.part == 0 && rt_len(ta, REL_P) > 0 &&
+        (qt == 0 || (c.win != 0 && c.win != REL_P && rt_win(ta) != 0 && rt_win(ta) != REL_P))) {
+      if ((c.rho > 0 || tr == 0) && (c.lho > 0 || tl == 0)) {
+        ruffed = true;  // nobody can overruff
+        if (1 >= cutoff) return 1;
+        continue;
+      }
+      const u32 pt = w_shfl(w.m, 4 * ((w.leader + 2) & 3) + trump);
+      const u32 lt = w_shfl(w.m, 4 * ((w.leader + 1) & 3) + trump), rt = w_shfl(w.m, 4 * ((w.leader + 3) & 3) + trump);
+      const u32 over = (c.lho == 0 ? lt : 0) | (c.rho == 0 ? rt : 0);
+      if (over < pt) {
+        ruffed = true;
+        if (id.s == trump) wr |= 1u << w_top(pt);
+        if (1 >= cutoff) return 1;
+      }
+      continue;
+    }
+    if (qt >= cutoff) return qt;
+  }
+  if (qt == 0 && (!has_t || rt_win(ta) == REL_NONE)) {
+    // No quick trick: the opponents win the first trick with a top card.
+    if (rt_win(top.a) != REL_NONE && rt_len(top.a, 0) > 0) wr = 1u << rt_rank(top.ranks, 0);
+    if (1 >= cutoff_other) return 0;
+  }
+  decided = false;
+  return qt;
+}
+
+// LaterTricks (later_min_impl / later_max_impl): true when the bound decides the node (NS
+// fail when NS lead, NS make it when EW lead). Written for the leader's side: the other
+// side takes at least one trick later.
+DDG_W bool w_later_tricks(const WarpState& w, const WarpIds& id, const WarpTop& top, u32& wr) {
+  const bool ns = ns_side(w.leader);
+  const int dq = w.left - 1, need = w.need;
+  wr = 0;
+  const u32 ta = w.trump >= 0 ? w_shfl(top.a, w.trump) : 0;
+  const bool nt = w.trump < 0 || rt_win(ta) == REL_NONE;
+  if (nt) {
+    // Tricks the leader's side can take with its own top cards' suits.
+    const int win = rt_win(top.a);
+    const bool ours = win == 0 || win == REL_P;
+    const int l0 = rt_len(top.a, 0), l1 = rt_len(top.a, 1), l2 = rt_len(top.a, 2), l3 = rt_len(top.a, 3);
+    const int pair = l0 > l2 ? l0 : l2;
+    const int sum = (int)w_add(id.t < 4 && ours ? (u32)pair : 0u);
+    if (sum <= 0) return false;
+    if (ns) {
+      if (!(sum < need) || dq >= need) return false;
+    } else {
+      if (!(dq + 1 - sum >= need) || 1 < need) return false;
+    }
+    const bool theirs = win == 1 || win == 3;  // a top card of the other side with another hand in the suit
+    const bool others = win == 1 ? (l0 | l2 | l3) != 0 : (l0 | l1 | l2) != 0;
+    if (theirs && others) wr = 1u << rt_rank(top.ranks, 0);
+    return true;
+  }
+  const u32 tk = w_shfl(top.ranks, w.trump);
+  const int win = rt_win(ta), sec = rt_sec(ta), thr = rt_thr(ta);
+  const bool win_ours = win == 0 || win == REL_P;
+  const u32 at_trump = id.s == w.trump ? 0xFFFFFFFFu : 0u;
+  // ns: "not even dq tricks are enough"; ew: "one trick is enough"
+  const bool one = ns ? dq < need : 1 >= need;
+  if (!win_ours) {
+    if (rt_len(ta, 0) == 0 && rt_len(ta, REL_P) == 0) {
+      const int a = rt_len(ta, REL_L), b = rt_len(ta, REL_R);
+      const int m = a > b ? a : b;
+      return ns ? dq + 1 - m < need : m >= need;
+    }
+    if (one) {
+      wr = 1u << rt_rank(tk, 0) & at_trump;
+      return true;
+    }
+    if (ns ? dq == need : 2 >= need) {
+      if (sec == REL_NONE) return false;
+      const bool sec_theirs = sec == 1 || sec == 3;
+      if (sec_theirs && (rt_len(ta, 1) > 1 || rt_len(ta, 3) > 1)) {
+        wr = 1u << rt_rank(tk, 1) & at_trump;
+        return true;
+      }
+    }
+    return false;
+  }
+  if (sec == REL_NONE || sec == 0 || sec == REL_P || rt_len(ta, sec) <= 1) return false;
+  if (win == ((sec + 3) & 3)) {
+    if (one) {
+      wr = 1u << rt_rank(tk, 1) & at_trump;
+      return true;
+    }
+  } else {
+    if (thr == REL_NONE) return false;
+    if ((thr == 1 || thr == 3) && one) {
+      wr = 1u << rt_rank(tk, 2) & at_trump;
+      return true;
+    }
+  }
+  return false;
+}
+
+// The second hand's QuickTricks (quick_tricks_2nd_impl). Neither it nor its partner has
+// played to the trick, so "holds the suit's top card at the trick's start" is a test of
+// its cards.
+DDG_W bool w_quick_2nd(const WarpState& w, const WarpIds& id, u32& wr) {
+  const int lead = (int)(w.trick & 0xFF), ls = card_suit(lead), trump = w.trump;
+  const int hand = lho_of(w.leader), P = partner_of(hand), third = lho_of(hand);
+  const int cutoff = ns_side(hand) ? w.need : w.left - w.need + 1;
+  wr = 0;
+  const u32 me = w_shfl(w.m, 4 * hand + ls), pd = w_shfl(w.m, 4 * P + ls), th = w_shfl(w.m, 4 * third + ls);
+  const u32 ranks = me | pd, bit = 1u << (lead & 15);
+  const bool wins = ranks > (bit | th);
+  bool by_rank = true;
+  if (trump >= 0 && ls != trump) {
+    const u32 T = w_ballot(id.s == trump && w.m != 0);  // seats that hold a trump: bits 4 * seat + trump
+    const bool we_ruff = (!me && (T >> (4 * hand + trump) & 1)) || (!pd && (T >> (4 * P + trump) & 1));
+    const bool they_ruff = !th && (T >> (4 * third + trump) & 1);
+    if (they_ruff) return false;
+    by_rank = !we_ruff;
+  }
+  if (by_rank && !wins) return false;
+  if (by_rank && id.s == ls) wr = 1u << w_top(ranks);
+  if (1 >= cutoff) return true;
+  if (trump >= 0) return false;
+  const int hh = me > pd ? hand : P;
+  const u32 mine = w_shfl(w.m, 4 * hh + id.s);
+  const int c1 = w_top(w.all);
+  const int c2 = w_top(w.all & ~(c1 >= 0 ? 1u << c1 : 0u));
+  const bool has1 = c1 >= 0 && (mine >> c1 & 1);
+  const bool has2 = c2 >= 0 && (mine >> c2 & 1);
+  int q = 1;
+  const u32 top2 = w_ballot(id.t < 4 && id.s == ls && has1 && has2);
+  if (top2) {
+    q++;
+    if (id.s == ls) wr |= 1u << c2;
+    if (q >= cutoff) return true;
+  }
+  // The other suits in order, each adding its tricks; the cards of those up to the one
+  // that reaches the cutoff count.
+  const bool lone = mine != 0 && !(w.now & ~mine);  // nobody else holds the suit
+  const int inc = id.s == ls || !mine ? 0 : lone ? w_popc(mine) : has1 ? 1 : 0;
+  const u32 upto = w_or((u32)inc << (4 * id.s)) * 0x1111u >> (4 * id.s) & 15;  // (at most 13 in all)
+  const u32 reached = w_ballot(id.t < 4 && q + (int)upto >= cutoff);
+  if (!reached) return false;
+  const int until = w_low(reached);
+  if (inc && !lone && id.s <= until) wr |= 1u << c1;
+  return true;
+}
+
+// ---- move generation -----------------------------------------------------------------------
+
+// Cards of a holding that are the top of their run (run_tops for one suit).
+DDG_W u32 w_run_tops(u32 own, u32 all) {
+  u32 open = ~(all & ~own) & 0x1FFFu;
+  u32 fill = own;
+  fill |= open & (fill >> 1);
+  open &= open >> 1;
+  fill |= open & (fill >> 2);
+  open &= open >> 2;
+  fill |= open & (fill >> 4);
+  open &= open >> 4;
+  fill |= open & (fill >> 8);
+  return own & ~(fill >> 1);
+}
+
+// The DDS lead weight (lead_weight) of `card` in this thread; top, hands and lengths of the
+// card's suit come from its threads.
+DDG_W int w_lead_weight(const WarpState& w, const WarpTop& top, int card, int hint) {
+  const int s = card_suit(card), r = card & 15, lead = w.leader, trump = w.trump;
+  const u32 a = w_shfl(top.a, s), tk = w_shfl(top.ranks, s), all = w_shfl(w.all, s);
+  const u32 own = w_shfl(w.m, 4 * lead + s), risL = w_shfl(w.m, 4 * lho_of(lead) + s);
+  const u32 risP = w_shfl(w.m, 4 * partner_of(lead) + s), risR = w_shfl(w.m, 4 * rho_of(lead) + s);
+  u32 ta = 0, hLT = 0, hPT = 0, hRT = 0;
+  if (trump >= 0) {
+    ta = w_shfl(top.a, trump);
+    hLT = w_shfl(w.m, 4 * lho_of(lead) + trump);
+    hPT = w_shfl(w.m, 4 * partner_of(lead) + trump);
+    hRT = w_shfl(w.m, 4 * rho_of(lead) + trump);
+  }
+  const u32 bit = 1u << r;
+  bool tt = false;  // the card, or one alike, is the hint
+  if (hint >= 0 && card_suit(hint) == s) {
+    const int hr = hint & 15, lo = r < hr ? r : hr, hi = r < hr ? hr : r;
+    const u32 between = ((1u << hi) - 1) & ~((2u << lo) - 1);
+    tt = (all & ~own & between) == 0;
+  }
+  const int r_rank = w_popc(all >> r);
+  const u32 below = all & (bit - 1);
+  const bool seq = below && (own >> w_top(below) & 1);
+  const int lenL = rt_len(a, REL_L), lenR = rt_len(a, REL_R), lenP = rt_len(a, REL_P);
+  const u32 cnt = (u32)((lenL == 0 ? w.left : lenL) + (lenR == 0 ? w.left : lenR)) << 2;
+  const int w1 = rt_win(a), w2 = rt_sec(a), w3 = rt_thr(a);
+  const bool is_win = rt_rank(tk, 0) == r, is_sec = w2 != REL_NONE && rt_rank(tk, 1) == r;
+  const bool drop = (lenL == 1 && w1 == REL_L) || (lenR == 1 && w1 == REL_R);
+  const bool p_long = (w2 == 0 && w3 == REL_P && lenP > 1) || (w2 == REL_P && w3 == 0 && lenP > 1);
+  const bool pp = w2 == REL_P && w3 == REL_P;
+  const bool w1_0 = w1 == 0, w1_p = w1 == REL_P, w2_p = w2 == REL_P;
+  const bool tops = risP > (risL | risR), lead_sec = seq & is_sec;
+  int delta, base;
+  bool with_rank;  // weight = delta + base (+ r_rank)
+  if (trump >= 0 && rt_win(ta) != REL_NONE) {
+    const int tP = rt_len(ta, REL_P);
+    const bool side = s != trump;
+    const bool ruffL = (lenL == 0) & (rt_len(ta, REL_L) != 0), ruffR = (lenR == 0) & (rt_len(ta, REL_R) != 0);
+    const u32 over = (ruffL ? hLT : 0) | (ruffR ? hRT : 0);  // trumps of the opponents that can ruff
+    const bool p_ruffs = (lenP == 0) & (tP != 0);
+    delta = -(int)((cnt << 5) / 13);
+    delta += side & (ruffL | ruffR) ? -12 : 0;
+    delta += side & p_ruffs & (lenR > 0) ? 17 : 0;
+    delta += (w1 == REL_R) | (w2 == REL_R) ? (lenR != 1 ? -12 : 0) : (w1 == REL_L) & w2_p & (lenP != 1) ? 27 : 0;
+    delta += side & (rt_len(a, 0) == 1) & (rt_len(ta, 0) > 0) & (lenP > 1) & w1_p ? 19 : 0;
+    const bool ruff_wins = hPT > over;
+    const bool win = is_win | tops ? !side | (is_win & p_ruffs ? ruff_wins : over == 0) : side & p_ruffs & ruff_wins;
+    if (win) {
+      base = drop ? 35 : w1_0 ? (w2_p ? 48 : is_win ? 31 : -3) : w1_p ? (w2 == 0 ? 42 : 28) : lead_sec ? 40 : seq ? 22 : 11;
+      with_rank = drop | (w1_0 ? w2_p | !is_win : w1_p | !lead_sec);
+      base += tt ? 18 : 0;
+    } else {
+      delta += pp ? 20 : p_long ? 13 : 0;
+      base = drop ? 2 : w1_0 ? (w2_p ? 33 : is_win ? 38 : -14) : w1_p ? 34 : lead_sec ? 35 : 15 - r;
+      with_rank = drop | (w1_0 ? w2_p | !is_win : w1_p);
+    }
+    return delta + base + (with_rank ? r_rank : 0);
+  }
+  delta = -(int)((cnt << 5) / 19) - (lenP == 0 ? 9 : 0);
+  if (is_win | tops) {
+    const bool safe = ((w2 != REL_L) | (lenL == 1)) & ((w2 != REL_R) | (lenR == 1));
+    delta += w2 == REL_R ? (lenR != 1 ? -1 : 0) : w2 == REL_L ? (lenL != 1 ? 22 : 16) : 0;
+    return delta + (safe ? 45 : 18) + (tt ? 32 : 0) + r_rank;
+  }
+  delta += (w1 == REL_R) | (w2 == REL_R) ? (lenR != 1 ? -10 : 0) : (w1 == REL_L) & w2_p & (lenP != 1) ? 31 : 0;
+  delta += pp ? 35 : p_long ? 25 : 0;
+  base = drop ? 28 : w1_0 ? -17 : !seq ? 12 : is_sec ? 48 : 29;
+  const int by = drop | w1_0 | !seq ? r_rank : is_sec ? 0 : -r_rank;
+  return delta + base + by + (tt ? 19 : 0);
+}
+
+DDG_W int w_hi(u32 m) { return w_top(m) + 2 - (m == 0); }  // DDS rank of the highest / lowest card, 0 = none
+DDG_W int w_lo(u32 m) { return m ? w_low(m) + 2 : 0; }
+
+// The DDS follow weights (follow_weight) of `card` in this thread; n = cards played. What
+// is the same for all candidates of a node is decided once (the branches); what differs
+// from card to card is chosen by selects, so the warp does not diverge.
+DDG_W int w_follow_weight(const WarpState& w, int n, int seat, bool is_void, int card) {
+  const int lead = w.leader, trump = w.trump;
+  const bool has_t = trump >= 0;
+  const int c0 = (int)(w.trick & 0xFF), ls = card_suit(c0), lead0 = rank2(c0);
+  const int s = card_suit(card), r = card & 15, rank = r + 2;
+  const int P = partner_of(lead), R = rho_of(lead);
+  const u32 hRL = w_shfl(w.m, 4 * R + ls), hRT0 = w_shfl(w.m, 4 * R + (trump & 3)), hRT = has_t ? hRT0 : 0;
+  const u32 all = w_shfl(w.all, s), now = w_shfl(w.now, s), me = w_shfl(w.m, 4 * seat + s);
+  const int r_rank = w_popc(now >> r);
+  const u32 bit = 1u << r, lead_bit = 1u << (c0 & 15);
+  const int c1 = (int)(w.trick >> 8 & 0xFF), c2 = (int)(w.trick >> 16 & 0xFF);
+  const int high1 = n > 1 && beats(c1, c0, trump) ? 1 : 0, move1 = high1 ? c1 : c0;
+  if (!is_void) {  // the 2nd hand (the others' order: w_follow_floor)
+    const u32 hPL = w_shfl(w.m, 4 * P + ls), hPT0 = w_shfl(w.m, 4 * P + (trump & 3)), hPT = has_t ? hPT0 : 0;
+    const u32 hLL = w_shfl(w.m, 4 * lead + ls);
+    const int max3rd = w_hi(hPL), maxpd = w_hi(hRL), min3rd = w_lo(hPL), minpd = w_lo(hRL);
+    const u32 below = all & (bit - 1);
+    const bool seq = (below != 0) & (me >> (w_top(below) & 31) & 1);
+    const bool over = (rank > lead0) & (rank > max3rd), pd_over = maxpd > lead0 && maxpd > max3rd;
+    const bool under = (rank < min3rd) | (rank < minpd);
+    int base;
+    bool by_rank;  // weight = base - rank, else base + r_rank
+    if (has_t) {
+      const bool side = ls != trump, pd_ruffs = maxpd == 0 && hRT;
+      const bool p_follows = max3rd != 0 || !hPT, pd_over_ruffs = hRT > hPT;
+      const bool u1 = !side || p_follows || (pd_ruffs && pd_over_ruffs), u2 = !side || p_follows;
+      const bool u3 = side && pd_ruffs && (p_follows || pd_over_ruffs), u4 = side && pd_ruffs;
+      const bool lead_high = lead0 > maxpd && lead0 > max3rd;
+      const bool win = over ? u1 : pd_over ? u2 : (lead_high & (lead0 > rank)) ? u3 : u4;
+      const bool keep = maxpd > lead0 && hLL > hRL;
+      const int high = rank < maxpd ? 78 : rank > max3rd ? 73 : seq ? 62 : 49;
+      const int on_win = min3rd > rank ? 40 : keep ? 41 : rank > lead0 ? high : maxpd > 0 ? 47 : 40;
+      const int on_loss = under ? -9 : rank < lead0 ? -16 : seq ? 22 : 10;
+      base = win ? on_win : on_loss;
+      by_rank = win ? !((min3rd > rank) | keep) : !(under | (rank < lead0));
+    } else {
+      base = pd_over ? 0 : over ? 81 : under ? -3 : rank < lead0 ? -11 : seq ? 10 : 13;
+      by_rank = pd_over | over | !(under | (rank < lead0) | seq);
+    }
+    return base + (by_rank ? -rank : r_rank);
+  }
+  // Void in the led suit: the discard's length and its top two cards at the trick's start.
+  const u32 sc = (u32)w_popc(me) << 6;
+  const int t1 = w_top(all) & 31, t2 = w_top(all & ~(1u << t1));
+  const bool one = sc == 64 && (me >> t1 & 1), two = sc == 128 && (t2 >= 0) & (me >> (t2 & 31) & 1);
+  const bool ruff = s == trump;
+  if (n == 1) {
+    const u32 hPL = w_shfl(w.m, 4 * P + ls), hPT0 = w_shfl(w.m, 4 * P + (trump & 3)), hPT = has_t ? hPT0 : 0;
+    const bool r_over = hRL > (hPL | lead_bit);  // 4th hand beats the trick
+    if (has_t) {
+      const int low_add = (int)(sc / 36) - (two ? 4 : 0), high_add = (int)(sc / 44);
+      const bool p_in = hPL != 0, r_ruffs = !hRL && hRT;
+      const bool pd_wins = p_in ? r_over || r_ruffs : (!hRL && hRT > hPT) || (!hPT && hRL > lead_bit);
+      const bool safe = p_in || (r_ruffs && hRT > hPT);
+      const bool high = ls == trump ? r_over : ruff ? safe | (bit > hPT) : pd_wins;
+      const int base = ls == trump ? 0 : ruff ? (high ? 24 : 15) : (high ? 60 : -2);
+      return base - rank + (high ? high_add : low_add);
+    }
+    return -rank + (r_over ? (int)(sc / 23) - (two ? 2 : one ? 3 : 0) : (int)(sc / 33) - (two ? 6 : one ? 8 : 0));
+  }
+  if (n == 2) {
+    const int max4th = w_hi(hRL), m1r = rank2(move1), m1s = card_suit(move1);
+    const u32 hLL = w_shfl(w.m, 4 * lead + ls), allL = w_shfl(w.all, ls);
+    if (!has_t) return -rank + (int)(sc / 24) - (two ? 4 : 0) - (one ? 4 : 0);
+    // the second card of the led suit was the leader's at the trick's start
+    const int l2 = w_top(allL & ~(1u << (w_top(allL) & 31)));
+    const bool sec_lead = l2 >= 0 && ((hLL | lead_bit) >> (l2 & 31) & 1);
+    const bool covered = high1 == 0 && lead0 > max4th && (max4th != 0 || !hRT);
+    const bool tops = bit > hRT;
+    const int base = high1 == 0 ? (max4th != 0 ? (sec_lead ? 36 : 48) : tops ? 48 : -12) : max4th != 0 ? 72 : tops ? 48 : 36;
+    const int plain = -rank + (int)(sc / 40);
+    const int ruffing = covered ? -rank - 50 : (m1s == trump) & (rank < m1r) ? -32 + r_rank + (int)(sc / 40) : base - rank + (int)(sc / 50);
+    return (ls == trump) | !ruff ? plain : ruffing;
+  }
+  const bool h2 = beats(c2, move1, trump);
+  const int move2 = h2 ? c2 : move1, m2r = rank2(move2);
+  const bool m2t = card_suit(move2) == trump;
+  if (!has_t) return -rank + (int)(sc / 27) - (two ? 6 : one ? 8 : 0);
+  const int val = (int)(sc / 24) - (two ? 2 : 0);
+  if (ls == trump) return -rank + val;
+  if (!h2 && high1) return (ruff ? 2 : 25) - rank + val;
+  return ruff ? (m2t & (rank <= m2r) ? -13 : 33) + r_rank : 14 - rank + val;
+}
+
+// Orders the candidates by weight (ties: highest card first, as insert_move keeps them)
+// into the frame; the thread of each one counts those ahead of it. Returns the first.
+DDG_W int w_order(const WarpIds& id, WarpFrame& f, u32 who, int card, int weight) {
+  const bool mine = who >> id.t & 1;
+  const u32 key = (u32)(weight + 1024) << 6 | (u32)card;
+  int ahead = 0;
+#pragma unroll 1
+  for (u32 rest = who; rest; rest &= rest - 1) ahead += w_shfl(key, w_low(rest)) > key;
+  if (mine) f.mv[ahead] = (uint8_t)card;
+  return (int)w_shfl((u32)card, w_low(w_ballot(mine && ahead == 0)));
+}
+
+// The 3rd or 4th hand follows suit (`led`, its candidates of the led suit): the DDS weight is
+// up - rank for a card that wins and -rank for one that does not, with `up` above any rank
+// and "wins" a threshold, so the order is the winners from the lowest up, then the others
+// from the lowest up. Returns the threshold: the winners are the cards of at least that
+// rank (13: none).
+DDG_W int w_follow_floor(const WarpState& w, int n, int seat, u32 led) {
+  const int trump = w.trump, c0 = (int)(w.trick & 0xFF), c1 = (int)(w.trick >> 8 & 0xFF), ls = card_suit(c0);
+  const bool high1 = beats(c1, c0, trump);
+  const int move1 = high1 ? c1 : c0;
+  const bool side = trump >= 0 && ls != trump;
+  if (n == 3) {
+    const int c2 = (int)(w.trick >> 16 & 0xFF);
+    const bool h2 = beats(c2, move1, trump);
+    const int move2 = h2 ? c2 : move1;
+    return (!h2 && high1) || (side && card_suit(move2) == trump) ? 13 : (move2 & 15) + 1;
+  }
+  const u32 fourth = w_shfl(w.m, 4 * rho_of(w.leader) + ls);
+  const int max4th = w_top(fourth), min4th = w_low(fourth), r1 = move1 & 15;  // -1: none
+  const int max3rd = w_top(w_shfl(w.m, 4 * seat + ls));
+  (void)led;
+  if (side && card_suit(move1) == trump) return 13;
+  if (side && high1 && max4th < 0) return r1 + 1;
+  if (!high1 && ((c0 & 15) > max4th || (side && max4th < 0))) return 13;
+  if (max3rd < min4th || max3rd < r1) return 13;
+  const int both = (max4th > r1 ? max4th : r1) + 1;
+  if (trump >= 0 && max3rd > max4th) return ls == trump || high1 ? both : max4th + 1;
+  return trump >= 0 && ls == trump ? 13 : both;
+}
+
+// Hands the cards of `cm` ([sp], the threads of `seat`) to threads 0, 1, 2, ...: thread
+// t looks at cards t and t + 32. Returns their number; `card` is this thread's.
+DDG_W int w_compact(const WarpIds& id, WarpMem& sm, u32 cm, int seat, int& card) {
+  const u32 a = w_shfl(cm, 4 * seat + (id.t >> 4)), b = w_shfl(cm, 4 * seat + 2 + (id.t >> 4));
+  const bool ha = a >> (id.t & 15) & 1, hb = b >> (id.t & 15) & 1;
+  const u32 ma = w_ballot(ha), mb = w_ballot(hb), lt = (1u << id.t) - 1;
+  if (ha) sm.scratch[w_popc(ma & lt)] = (uint8_t)id.t;
+  if (hb) sm.scratch[w_popc(ma) + w_popc(mb & lt)] = (uint8_t)(id.t + 32);
+  w_sync();
+  card = sm.scratch[id.t & 15] & 63;
+  const int n = w_popc(ma) + w_popc(mb);
+  w_sync();
+  return n;
+}
+
+// The frame's info word: value when no child cuts:1 | seat:2 | candidates:4 | the one being
+// searched:4 | undo leader:2 | its card:6 | win card:7 (64 = none).
+DDG_W u32 w_open_info(int seat, int n) { return (u32)(!ns_side(seat)) | (u32)seat << 1 | (u32)n << 3; }
+DDG_W int wi_result(u32 info) { return (int)(info & 1); }
+DDG_W int wi_seat(u32 info) { return (int)(info >> 1) & 3; }
+DDG_W int wi_n(u32 info) { return (int)(info >> 3) & 15; }
+DDG_W int wi_i(u32 info) { return (int)(info >> 7) & 15; }
+DDG_W int wi_undo_leader(u32 info) { return (int)(info >> 11) & 3; }
+DDG_W int wi_card(u32 info) { return (int)(info >> 13) & 63; }
+DDG_W int wi_win_card(u32 info) { return (int)(info >> 19) & 127; }
+enum : u32 { WI_NEXT = 1u << 7, WI_KEEP = (1u << 11) - 1 };  // one candidate on; what a play leaves
+
+DDG_W u32 w_tags(const TTBucket* b, const WarpIds& id) { return b->tag[id.t & 15]; }
+
+// A trick start. Entering it (enter_lead): cutoffs, the last trick, the TT probe, the
+// bounds; a bound's result is stored. Finishing it (`fin`, with its value v and relevant
+// cards w.rel, and the cutting card `best` or -1): the result is stored. Both need the
+// position's key and owner codes and end in the same store, so they share the code.
+// Returns the value, or -1 when the node expands (top and hint set).
+template <class Env>
+DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool fin, int v, int best, WarpTop& top, int& hint) {
+  const int need = w.need;
+  if (!fin) {
+    w.rel = 0;
+    if (need <= 0) return 1;
+    if (w.left < need) return 0;
+    if (w.left == 1) {
+      const u32 bt = w_ballot(id.s == w.trump && w.all != 0);
+      const int su = bt ? w.trump : w_low(w_ballot(id.p == w.leader && w.m != 0)) & 3;
+      const u32 in = w_shfl(w.all, su);
+      if (id.s == su && w_popc(in) >= 2) w.rel = 1u << w_top(in);
+      return (int)(~w_shfl(w.code, su) >> 30 & 1);  // the top card's holder is N or S
+    }
+  }
+  const WarpKey k = w_key(w, id, env.mask());
+  TTBucket* b = env.table() + k.bucket;
+  const u32 tagw = w_tags(b, id);
+  if (!fin) {
+    const int hit = w_probe(w, id, b, tagw, k, w.code, need, hint);
+    if (hit >= 0) return hit;
+    top = w_make_top(w, id, k);
+    const bool ns_lead = ns_side(w.leader);
+    const int cut_ns = need, cut_ew = w.left - need + 1;
+    bool decided;
+    u32 wr;
+    const int q = w_quick_tricks(w, id, top, ns_lead ? cut_ns : cut_ew, ns_lead ? cut_ew : cut_ns, wr, decided);
+    if (decided) v = ns_lead ? q != 0 : q == 0;
+    else if (w_later_tricks(w, id, top, wr)) v = !ns_lead;
+    else return -1;
+    w.rel = wr;
+  }
+  w_store(w, id, b, tagw, k, w.code, w.rel, v ? need : 0, v ? w.left : need - 1, best);
+  return v;
+}
+
+// A node expands (gen_moves_lead, gen_moves_follow): its candidates, one per run of alike
+// cards, ordered by the DDS weights into a fresh frame. Returns the first.
+template <class Env>
+DDG_W int w_expand(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, const WarpTop& top, int hint) {
+  const int seat = (w.leader + w.nplayed) & 3, ls = (int)(w.trick >> 4) & 3;
+  const u32 cm = w_run_tops(w.m, w.all);
+  const u32 in_led = w_shfl(cm, 4 * seat + ls);
+  const u32 led = w.nplayed ? in_led : 0;
+  WarpFrame& f = sm.fr[w.sp];
+  u32 who = led;  // the threads that stand for a candidate
+  int n = w_popc(led), card = ls * 16 + (id.t & 15);  // following suit: thread r for rank r
+  if (!led) {
+    n = w_compact(id, sm, cm, seat, card);
+    who = (1u << n) - 1;
+  }
+  w.at = 0;
+  w.info = w_open_info(seat, n);
+  if (n == 1) {
+    card = (int)w_shfl((u32)card, w_low(who));
+    if (id.t == 0) f.mv[0] = (uint8_t)card;
+    return card;
+  }
+  if (led && w.nplayed > 1) {
+    const u32 win = led & (0xFFFFFFFFu << w_follow_floor(w, w.nplayed, seat, led)), lose = led & ~win;
+    const u32 below = (1u << id.t) - 1;
+    const int ahead = win >> id.t & 1 ? w_popc(win & below) : w_popc(win) + w_popc(lose & below);
+    if (led >> id.t & 1) f.mv[ahead] = (uint8_t)card;
+    return ls * 16 + w_low(win ? win : led);
+  }
+  int weight;
+  if (w.nplayed == 0) {
+    if (hint < 0 && w.sp == 0) {  // the root, no TT move: an outside hint, when the leader holds it
+      const int h = env.root_hint(sm.job);
+      if (h >= 0 && h < 64 && (w_shfl(w.m, 4 * seat + (h >> 4)) >> (h & 15) & 1)) hint = h;
+    }
+    weight = w_lead_weight(w, top, card, hint);
+  } else {
+    weight = w_follow_weight(w, w.nplayed, seat, !led, card);
+  }
+  return w_order(id, f, who, card, weight);
+}
+
+// ENTER inside a trick (enter_follow): the second hand's QuickTricks.
+DDG_W int w_enter_follow(WarpState& w, const WarpIds& id) {
+  if (w.nplayed != 1) return -1;
+  u32 wr;
+  if (!w_quick_2nd(w, id, wr)) return -1;
+  w.rel = wr;
+  return ns_side(lho_of(w.leader)) ? 1 : 0;
+}
+
+// Plays `card` from the top frame and pushes the frame (play): at the fourth card the
+// trick is settled and the frame keeps what taking it back needs.
+DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, int card) {
+  WarpFrame& f = sm.fr[w.sp];
+  const int seat = wi_seat(w.info), su = card_suit(card), r = card & 15;
+  const u32 bit = 1u << r, code = w.code, trick = w.trick;
+  u32 info = (w.info & WI_KEEP) | (u32)card << 13;
+  if (id.s == su) {
+    // The card's owner leaves the code: the owners of the cards below move up.
+    const u32 low = 0xFFFFFFFFu >> (2 * w_popc(w.now >> r) - 2);
+    w.code = (code & ~low) | (code << 2 & low);
+    w.at |= bit << 16;
+    w.now ^= bit;
+  }
+  if ((id.t & 15) == seat * 4 + su) w.m ^= bit;
+  w.trick |= (u32)card << (8 * w.nplayed);
+  w.nplayed++;
+  if (w.nplayed == 4) {
+    const int c = (int)(w.trick >> (8 * (id.t & 3))) & 0xFF, cs = card_suit(c);
+    const u32 key = (cs == w.trump ? 512u : cs == card_suit((int)(w.trick & 0xFF)) ? 256u : 0u) | (u32)c << 2 | (u32)(id.t & 3);
+    const u32 best = w_max(key);
+    const int wc = (int)(best >> 2) & 63;
+    const int same = w_popc(w_ballot(cs == card_suit(wc)) & 15);  // at least two: won by rank
+    info |= (u32)w.leader << 11 | (u32)(same >= 2 ? wc : 64) << 19;
+    if (id.t < 4) f.all[id.t] = (uint16_t)w.all;
+    w.all = w.now;
+    w.leader = (w.leader + (int)(best & 3)) & 3;
+    w.trick = 0;
+    w.nplayed = 0;
+    w.left--;
+    w.need -= ns_side(w.leader);
+  }
+  if (id.t < 4) {
+    f.suit[id.t].at = w.at;
+    f.suit[id.t].code = code;
+  }
+  if (id.t == 4) {
+    f.trick = trick;
+    f.info = info;
+  }
+  w.sp++;
+  w_sync();
+}
+
+// Pops the top frame and takes its card back (node_done, unplay); returns the card.
+DDG_W int w_unplay(WarpState& w, const WarpIds& id, WarpMem& sm) {
+  w.sp--;
+  const WarpFrame& f = sm.fr[w.sp];
+  w.at = f.suit[id.s].at;
+  w.code = f.suit[id.s].code;
+  w.trick = f.trick;
+  w.info = f.info;
+  const int card = wi_card(w.info), su = card_suit(card);
+  if (w.nplayed == 0) {  // this ply completed a trick
+    w.all = f.all[id.s];
+    w.need += ns_side(w.leader);
+    w.left++;
+    w.leader = wi_undo_leader(w.info);
+    const int wc = wi_win_card(w.info);
+    if (id.s == card_suit(wc)) w.rel |= 1u << (wc & 15);  // (none: suit 4)
+  }
+  w.nplayed = (w.nplayed - 1) & 3;
+  const u32 bit = 1u << (card & 15);
+  if (id.s == su) w.now ^= bit;
+  if ((id.t & 15) == wi_seat(w.info) * 4 + su) w.m ^= bit;
+  return card;
+}
+
+// The frame's next candidate that is not a small card like one tried before (step_next):
+// every candidate is tested by its thread. -1: none left.
+DDG_W int w_next(WarpState& w, const WarpIds& id, const WarpMem& sm) {
+  const int n = wi_n(w.info), i = wi_i(w.info);
+  if (i >= n) return -1;
+  const int c = sm.fr[w.sp].mv[id.t & 15];
+  const u32 at = w_shfl(w.at, card_suit(c));
+  const u32 acc = at & 0xFFFFu, tried = at >> 16, bit = 1u << (c & 15);
+  const u32 small = (acc & (0u - acc)) - 1;  // below the lowest relevant card (all, when there is none)
+  const bool skip = (small & bit) != 0 && (small & tried) != 0;
+  const u32 open = w_ballot(id.t < n && !skip) >> i << i;
+  if (!open) return -1;
+  const int next = w_low(open);
+  w.info = (w.info & ~(15u << 7)) | (u32)next << 7;
+  return (int)w_shfl((u32)c, next);
+}
+
+// The top frame is done (finish): the relevant cards widen through runs of the hand's own
+// touching cards.
+DDG_W u32 w_widen(const WarpState& w, const WarpIds& id) {
+  const u32 acc = w.at & 0xFFFFu, low = acc & (0u - acc);
+  const u32 own = w_shfl(w.m, 4 * wi_seat(w.info) + id.s);
+  const u32 below = w.all & (low - 1), stop = 2u << (w_top(below & ~own) & 31);  // (no stop: 2 << 31 = 0)
+  return acc | (low & own ? below & (0u - (stop ? stop : 1u)) : 0);
+}
+
+// ---- root searches (start_search, start_lead, root_result) -----------------------------------
+
+DDG_W void w_start_search(WarpState& w, const WarpJob& j) {
+  w.leader = (j.decl + 1) & 3;
+  w.nplayed = 0;
+  w.left = j.cards;
+  w.trick = 0;
+  w.sp = 0;
+}
+
+// Starts the trick count of the current declarer: the binary search at `first`, or the
+// stepping search from the seed `first`. (A deal has at least one card each, so every
+// lead needs a search.)
+DDG_W void w_start_lead(WarpState& w, const WarpIds& id, WarpJob& j, int first) {
+  int lo = 0, hi = 13;
+  if (j.mode == MODE_BISECT) {
+    w.need = first < 1 ? 1 : first > 13 ? 13 : first;
+  } else {
+    lo = first < 0 ? 0 : first > j.cards ? j.cards : first;
+    hi = lo == 0 ? PH_UP : PH_FIRST;
+    w.need = lo == 0 ? 1 : lo;
+  }
+  w_start_search(w, j);
+  w_sync();
+  if (id.t == 0) {
+    j.lo = (int8_t)lo;
+    j.hi = (int8_t)hi;
+  }
+  w_sync();
+}
+
+// A root search at `target` finished with value v: the next target, or -1 with the answer
+// in `lo`.
+DDG_W int w_root_result(int mode, int cards, int target, int v, int& lo, int& hi) {
+  if (mode == MODE_BISECT) {
+    if (v) lo = target;
+    else hi = target - 1;
+    return lo < hi ? (lo + hi + 1) / 2 : -1;
+  }
+  if (hi == PH_DOWN || (hi == PH_FIRST && !v)) {  // going down: lo - 1 is next
+    if (hi == PH_DOWN && v) return -1;
+    hi = PH_DOWN;
+    lo--;
+    return lo > 0 ? lo : -1;
+  }
+  if (hi == PH_UP) {
+    if (!v) return -1;
+    lo++;
+  }
+  hi = PH_UP;
+  return lo < cards ? lo + 1 : -1;
+}
+
+// Totals to shared memory: the node count and every thread's counter.
+DDG_W void w_flush(WarpState& w, const WarpIds& id, WarpMem& sm) {
+  if (id.t < WCNT_COUNT) sm.job.total[id.t] += w.cnt;
+  if (id.t == 0) sm.job.nodes += w.nodes;
+  w.cnt = 0;
+  w.nodes = 0;
+  w_sync();
+}
+
+// A root search is done with value v and the root's cutting card `best` (or -1): the next
+// search of the job, or its end (false).
+template <class Env>
+DDG_W bool w_end_root(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, int v, int best) {
+  WarpJob& j = sm.job;
+  if (best >= 0 && (v != 0) == ns_side(w.leader)) env.root_best(j, best);
+  int lo = j.lo, hi = j.hi;
+  const int next = w_root_result(j.mode, j.cards, w.need, v, lo, hi);
+  w_sync();
+  if (next >= 0) {
+    w.need = next;
+    if (id.t == 0) {
+      j.lo = (int8_t)lo;
+      j.hi = (int8_t)hi;
+    }
+    w_sync();
+    w_start_search(w, j);
+    return true;
+  }
+  env.answer(j, lo);
+  const int decl = j.decl + 1;
+  w_sync();
+  if (decl > j.last_decl) {
+    w_flush(w, id, sm);
+    env.job_done(j);
+    return false;
+  }
+  if (id.t == 0) j.decl = (int8_t)decl;
+  w_sync();
+  // The next lead starts at this answer (binary search) or at its own seed.
+  w_start_lead(w, id, j, j.mode == MODE_BISECT ? lo : env.seed(j));
+  return true;
+}
+
+// Runs jobs until none is left or the environment stops the warp. sm.job.stage: ST_TAKE to
+// start with a job, ST_ENTER to go on inside one (w and the frames as they were saved); on
+// return ST_IDLE (nothing left), ST_TAKE or ST_ENTER (stopped). An Env offers
+//   bool take(w, id, sm)   the next job: position, job record (else stage is set)
+//   bool stop(w, id, sm)   asked every 64 nodes: true ends the warp
+//   int seed(job), root_hint(job); void answer(job, ns), root_best(job, card), job_done(sm)
+//   TTBucket* table(); u32 mask()
+template <class Env>
+DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
+  bool in_job = sm.job.stage == ST_ENTER;
+  for (;;) {
+    if (!in_job) {
+      if (!env.take(w, id, sm)) return;
+      WarpJob& j = sm.job;
+      w_start_lead(w, id, j, env.seed(j));
+      in_job = true;
+    }
+    // One node per turn: entered, then the frames it closes, up to the next card played.
+    for (;;) {
+      if ((w.nodes & 63u) == 63u && env.stop(w, id, sm)) return;
+      w.nodes++;
+      int v = -1, card = -1, best = -1, hint = -1;
+      bool fin = false, done = false;
+      WarpTop top = {0, 0};
+      for (;;) {
+        if (w.nplayed == 0) v = w_lead(w, id, env, fin, v, best, top, hint);
+        else v = w_enter_follow(w, id);
+        if (v < 0) {
+          card = w_expand(w, id, sm, env, top, hint);
+          break;
+        }
+        // The node is decided: its card is taken back, and the frames it completes with it.
+        for (;;) {
+          if (w.sp == 0) {
+            done = true;  // the root search
+            break;
+          }
+          const int c = w_unplay(w, id, sm);
+          best = -1;
+          if (v == (int)ns_side(wi_seat(w.info))) {  // the child cuts
+            w.at = (w.at & 0xFFFF0000u) | w.rel;
+            best = c;
+          } else {
+            w.at |= w.rel;
+            w.info += WI_NEXT;
+            card = w_next(w, id, sm);
+            if (card >= 0) break;
+            v = wi_result(w.info);
+          }
+          w.rel = w_widen(w, id);
+          if (w.nplayed == 0) break;
+        }
+        if (done || card >= 0) break;
+        fin = true;  // a trick start: its result is stored
+      }
+      if (done) {
+        in_job = w_end_root(w, id, sm, env, v, best);
+        if (!in_job) break;
+        continue;
+      }
+#ifdef DDG_BOUNDS_CHECK
+      if (w.sp >= STACK_DEPTH) {  // counted, skipped: the warp stops, its results stay unsolved
+        w_count(w, id, WCNT_BOUNDS, 1);
+        w_flush(w, id, sm);
+        if (id.t == 0) sm.job.stage = ST_IDLE;
+        return;
+      }
+#endif
+      w_play(w, id, sm, card);
+    }
+  }
+}
+
+}  // namespace ddg
+
+#endif  // DDG_TT_SIG
