@@ -260,8 +260,11 @@ int ddg_solver_create(const ddg_config* cfg_in, ddg_solver** out) {
   s->by_warp = warp_route(cfg);
 #ifndef DDG_TT_SIG
   if (s->by_warp) {
-    e = cudaFuncSetAttribute((const void*)warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute((const void*)warp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)warp_smem(WARP_MAX));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute((const void*)warp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)warp_smem(WARP_MAX));
     if (e != cudaSuccess) {
       delete s;
       return fail(DDG_E_CUDA, "warp kernel: %s", cudaGetErrorString(e));
@@ -331,7 +334,8 @@ static int launch_batch(ddg_solver* s, const BatchArgs& a, cudaStream_t stream, 
     args.rr_jobs = a.ring ? 0 : std::min<long long>(a.n_jobs, (long long)grid * use);
     *grid_out = grid;
     *block_out = use * 32;
-    CUDA_TRY(cudaLaunchKernel((const void*)warp_kernel, dim3(grid), dim3(use * 32), params, warp_smem(use), stream));
+    const void* fn = a.ring ? (const void*)warp_kernel<true> : (const void*)warp_kernel<false>;
+    CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(use * 32), params, warp_smem(use), stream));
     return DDG_OK;
   }
 #endif

@@ -156,7 +156,7 @@ __device__ __forceinline__ bool stop_requested(const BatchArgs& a, u64 t_end) {
 }
 
 // Stream: counts a finished job of `deal`; the last one writes the deal's completion record.
-__device__ __noinline__ void stream_deal_done(const BatchArgs& a, long long deal) {
+__device__ __forceinline__ void stream_deal_done(const BatchArgs& a, long long deal) {
   const long long slot = deal & a.ring_mask;
   __threadfence();  // this job's answers before the count
   if (atomicAdd(a.deal_done + slot, 1) != a.jpd - 1) return;

@@ -30,28 +30,40 @@ DDG_W u32 w_or(u32 v) { return __reduce_or_sync(0xFFFFFFFFu, v); }
 DDG_W u32 w_max(u32 v) { return __reduce_max_sync(0xFFFFFFFFu, v); }
 DDG_W u32 w_min(u32 v) { return __reduce_min_sync(0xFFFFFFFFu, v); }
 DDG_W u32 w_add(u32 v) { return __reduce_add_sync(0xFFFFFFFFu, v); }
+DDG_W bool w_any(bool p) { return __any_sync(0xFFFFFFFFu, p); }
+// The same value in all threads, said so to the compiler: ptxas follows uniformity from a
+// vote, a reduction, a shuffle from one thread or a shared-memory load at a uniform
+// address, but not around a loop. Where it cannot tell that a branch is uniform it guards
+// every collective behind it (a divergence test, and a slow path of some ten instructions).
+DDG_W u32 w_uni(u32 v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
 DDG_W void w_sync() { __syncwarp(); }
 DDG_W int w_top(u32 x) { return 31 - __clz((int)x); }   // highest set bit, -1 for 0
 DDG_W int w_low(u32 x) { return __ffs((int)x) - 1; }    // lowest set bit, -1 for 0
 DDG_W int w_popc(u32 x) { return __popc(x); }
 #else  // the host emulation provides the collectives (warp_emu.hpp)
 #define DDG_W static inline
+DDG_W bool w_any(bool p) { return w_ballot(p) != 0; }
+DDG_W u32 w_uni(u32 v) { return v; }
 DDG_W int w_top(u32 x) { return x ? 31 - __builtin_clz(x) : -1; }
 DDG_W int w_low(u32 x) { return x ? __builtin_ctz(x) : -1; }
 DDG_W int w_popc(u32 x) { return __builtin_popcount(x); }
 #endif
 
-// One level of the search in shared memory.
+// One level of the search in shared memory: what taking its move back needs.
 struct alignas(16) WarpFrame {
   struct {
     u32 at;    // relevant cards gathered so far | cards tried << 16
     u32 code;  // owner code before this frame's card was played
   } suit[4];
-  u32 trick, info;  // the trick before this frame's card; w_open_info()
-  uint16_t all[4];  // a frame that completed a trick: the cards in play at the trick's start
-  uint8_t mv[16];   // candidates, best first
+  u32 st, info, trick;  // state word and trick before this frame's card; w_open_info()
+  uint8_t mv[12];       // candidates 1.., best first (the first is played at once)
+  uint16_t all[4];      // a frame that completed a trick: the cards in play at its start
 };
 static_assert(sizeof(WarpFrame) == 64, "a frame is two 32-byte halves");
+
+// The state word: leader:2 | -:1 | cards played to the trick * 8:2 | -:1 | frame offset
+// (depth * 64):6 | tricks left:4 | tricks NS still need:4.
+enum : u32 { SW_LEADER = 3, SW_CARD = 8, SW_NP8 = 0x18, SW_FRAME = 64, SW_OFF = 0xFC0, SW_LEFT = 1u << 12, SW_NEED = 1u << 16 };
 
 // Counters, one to a thread.
 enum { WCNT_PROBES = 0, WCNT_HITS = 1, WCNT_STORES = 2, WCNT_READS = 3, WCNT_BYTES = 4, WCNT_BOUNDS = 5, WCNT_COUNT = 6 };
@@ -81,14 +93,20 @@ struct WarpState {
   u32 rel;    // [s] relevant cards of the node just finished
   u32 at;     // [s] top frame's relevant cards | tried cards << 16
   u32 cnt;    // [t] counter of thread WCNT_*
-  u32 trick;  // cards of the trick, a byte each (bytes from nplayed on are 0)
+  u32 st;     // the state word
+  u32 trick;  // cards of the trick, a byte each (the bytes from the next one on are 0)
   u32 info;   // top frame's info word
-  int trump, leader, nplayed, left;
-  int need;      // tricks NS still need
-  int sp;        // depth of the top frame
-  u32 nodes;     // nodes since the last flush
+  int trump;
+  int leader, nplayed, left, need;  // fields of st, as w_unpack() last read them
+  u32 nodes;  // nodes since the last flush
   u32 gen;
 };
+DDG_W void w_unpack(WarpState& w) {
+  w.leader = (int)(w.st & SW_LEADER);
+  w.nplayed = (int)(w.st >> 3 & 3);
+  w.left = (int)(w.st >> 12 & 15);
+  w.need = (int)(w.st >> 16 & 15);
+}
 
 struct WarpIds {  // what a thread stands for
   int t, s, p;
@@ -101,7 +119,7 @@ DDG_W void w_count(WarpState& w, const WarpIds& id, int what, u32 k) {
 // ---- key and owner codes -------------------------------------------------------------------
 
 struct WarpKey {
-  u64 q;
+  u32 q, q_hi;  // hash bits 9..40 and 41..47
   u32 lens_hi, lens_lo;  // length_key()
   u32 bucket, tag;
 };
@@ -115,7 +133,8 @@ DDG_W WarpKey w_key(const WarpState& w, const WarpIds& id, u32 mask) {
   k.lens_lo = w_or(id.p >= 2 ? part : 0);
   const u64 x = key_hash((u64)k.lens_hi << 32 | k.lens_lo, w.leader);
   k.bucket = (u32)x & mask;
-  k.q = (x >> 9) & ((1ull << Q_BITS) - 1);
+  k.q = (u32)(x >> 9);
+  k.q_hi = (u32)(x >> 41) & 0x7Fu;
   k.tag = ((u32)(x >> 32) & 0xFFFF0000u) | ((u32)w.left << 12) | (w.gen << 2) | (u32)w.leader;
   return k;
 }
@@ -124,11 +143,15 @@ DDG_W WarpKey w_key(const WarpState& w, const WarpIds& id, u32 mask) {
 DDG_W u32 w_build_code(const WarpState& w, const WarpIds& id) {
   u32 h[4], code = 0;
   for (int q = 0; q < 4; q++) h[q] = w_shfl(w.m, 4 * q + id.s);
-  int at = 32;
-  for (int r = 12; r >= 0; r--)
-    for (u32 q = 0; q < 4; q++)
-      if (h[q] >> r & 1 && at > 0) code |= q << (at -= 2);
-  return code;
+  int n = 0;
+#pragma unroll
+  for (int r = 12; r >= 0; r--) {
+    const u32 on = (h[0] | h[1] | h[2] | h[3]) >> r & 1;
+    const u32 who = (h[1] >> r & 1) | (h[2] >> r & 1) << 1 | (h[3] >> r & 1) * 3;
+    code = on ? code << 2 | who : code;
+    n += (int)on;
+  }
+  return code << 1 << (31 - 2 * n);
 }
 // The owners of the highest n cards, lowest card in the low bits (n = 0: 0).
 DDG_W u32 w_pattern(u32 code, int n) { return (code >> 1) >> (31 - 2 * n); }
@@ -140,6 +163,30 @@ DDG_W u32 w_top_n(u32 all, int n) {
   for (int step = 8; step; step >>= 1)
     if (w_popc(all >> (r + step)) >= n) r += step;
   return (all >> r) << r;
+}
+
+// A searcher has its table to itself, so its entries are stored as they are (those of tables
+// that lanes may share are sealed against torn reads, ddg_tt.cuh).
+struct WarpEntry {
+  u32 q, w0;     // q: hash bits 9..40 | hash bits 41..47:7 | lb:4 | ub:4 | best:6 | owners 48..57:10, 1 bit free
+  u32 w1, own;   // counts:16 | owners 0..15; owners 16..47
+};
+DDG_W WarpEntry w_entry(const TTBucket* b, int way) {
+#ifdef __CUDA_ARCH__
+  const uint4 x = *reinterpret_cast<const uint4*>(b->e[way]);
+  return WarpEntry{x.x, x.y, x.z, x.w};
+#else
+  WarpEntry e;
+  memcpy(&e, b->e[way], 16);
+  return e;
+#endif
+}
+DDG_W void w_entry_put(TTBucket* b, int way, WarpEntry e) {
+#ifdef __CUDA_ARCH__
+  *reinterpret_cast<uint4*>(b->e[way]) = make_uint4(e.q, e.w0, e.w1, e.own);
+#else
+  memcpy(b->e[way], &e, 16);
+#endif
 }
 
 // ---- transposition table -------------------------------------------------------------------
@@ -160,9 +207,8 @@ DDG_W int w_probe(WarpState& w, const WarpIds& id, const TTBucket* b, u32 tagw, 
   int best = 63;
   u32 counts = 0;
   if (match) {
-    u64 w0, w1;
-    entry_load(b, (int)((tagw >> 8) & 15), w0, w1);
-    counts = (u32)w1 & 0xFFFFu;
+    const WarpEntry e = w_entry(b, (int)((tagw >> 8) & 15));
+    counts = e.w1 & 0xFFFFu;
     // Tag, bucket and q are the whole hash of the suit lengths, a bijection, so an entry
     // with this q has these lengths: its counts are no longer than the suits.
     const int n0 = (int)(counts & 15), n1 = (int)(counts >> 4 & 15), n2 = (int)(counts >> 8 & 15);
@@ -170,9 +216,10 @@ DDG_W int w_probe(WarpState& w, const WarpIds& id, const TTBucket* b, u32 tagw, 
     mine = mine << (2 * n2) | w_pattern(codes[2], n2);
     mine = mine << (2 * n1) | w_pattern(codes[1], n1);
     mine = mine << (2 * n0) | w_pattern(codes[0], n0);
-    same = (w0 & ((1ull << Q_BITS) - 1)) == k.q && mine == ((w1 >> 16) | ((w0 >> 53) << 48));
-    const int lb = (int)((w0 >> Q_BITS) & 15), ub = (int)((w0 >> (Q_BITS + 4)) & 15);
-    best = (int)((w0 >> (Q_BITS + 8)) & 63);
+    same = ((e.q ^ k.q) | ((e.w0 ^ k.q_hi) & 0x7Fu) | ((u32)mine ^ (e.w1 >> 16 | e.own << 16)) |
+            ((u32)(mine >> 32) ^ (e.own >> 16 | (e.w0 >> 21 & 0x3FFu) << 16))) == 0;
+    const int lb = (int)(e.w0 >> 7 & 15), ub = (int)(e.w0 >> 11 & 15);
+    best = (int)(e.w0 >> 15 & 63);
     holds = lb >= need;
     decides = same && (holds || ub < need);
   }
@@ -202,19 +249,17 @@ DDG_W void w_store(WarpState& w, const WarpIds& id, TTBucket* b, u32 tagw, const
   if (n0 + n1 + n2 + (int)(counts >> 12) > MAX_REL) return;
   const int off = (id.s > 0 ? n0 : 0) + (id.s > 1 ? n1 : 0) + (id.s > 2 ? n2 : 0);
   const u64 mine = (u64)w_pattern(code, above) << (2 * off);
-  const u64 owners = (u64)w_or((u32)(mine >> 32)) << 32 | w_or((u32)mine);
-  const u64 w1 = (u64)counts | owners << 16;
-  const u32 hi = (u32)(owners >> 48);
+  const u32 own_lo = w_or((u32)mine), own_hi = w_or((u32)(mine >> 32));
+  WarpEntry e = {k.q, k.q_hi | own_hi >> 16 << 21, counts | own_lo << 16, own_lo >> 16 | own_hi << 16};
   const bool match = id.t < TT_WAYS && (tagw & ~0xF00u) == k.tag;
   const u32 mm = w_ballot(match);
   w_count(w, id, WCNT_STORES, 1);
   bool same = false;
   u32 old = 0;
   if (match) {
-    u64 e0, e1;
-    entry_load(b, (int)((tagw >> 8) & 15), e0, e1);
-    same = (e0 & ((1ull << Q_BITS) - 1)) == k.q && e1 == w1 && (u32)(e0 >> 53) == hi;
-    old = (u32)(e0 >> Q_BITS) & 0x3FFFu;  // lb:4 | ub:4 | best:6
+    const WarpEntry o = w_entry(b, (int)((tagw >> 8) & 15));
+    same = ((o.q ^ e.q) | (o.w1 ^ e.w1) | (o.own ^ e.own) | ((o.w0 ^ e.w0) & ~(0x3FFFu << 7))) == 0;
+    old = o.w0 >> 7 & 0x3FFFu;  // lb:4 | ub:4 | best:6
   }
   const u32 sm = w_ballot(same);
   int way;
@@ -239,8 +284,8 @@ DDG_W void w_store(WarpState& w, const WarpIds& id, TTBucket* b, u32 tagw, const
     const u32 prev = w_shfl_up1(tagw);
     if (id.t <= pos) b->tag[id.t] = id.t == 0 ? (k.tag | (u32)way << 8) : prev;
   }
-  if (id.t == TT_WAYS)
-    entry_store(b, way, k.q | (u64)((u32)lb | (u32)ub << 4 | (u32)(best < 0 ? 63 : best) << 8 | hi << 14) << Q_BITS, w1);
+  e.w0 |= ((u32)lb | (u32)ub << 4 | (u32)(best < 0 ? 63 : best) << 8) << 7;
+  if (id.t == TT_WAYS) w_entry_put(b, way, e);
   w_sync();
 }
 
@@ -265,6 +310,11 @@ DDG_W WarpTop w_make_top(const WarpState& w, const WarpIds& id, const WarpKey& k
                 ((k.lens_lo >> sh) & 15) << 12;
   WarpTop t;
   t.a = ((l | l << 16) >> (4 * w.leader)) & 0xFFFFu;
+  // bit 28: of the cards the leader does not hold, partner's is the highest
+  const u32 len = (u32)w_popc(w.all);
+  const u32 others = (w.code ^ (u32)w.leader * 0x55555555u) & ~(0xFFFFFFFFu >> (2 * len));
+  const int pos = (31 - w_top(others)) & 30;
+  t.a |= others && ((w.code >> (30 - pos) ^ (u32)w.leader) & 3) == 2 ? 1u << 28 : 0;
   t.ranks = 0;
   u32 a = w.all;
 #pragma unroll
@@ -353,6 +403,25 @@ DDG_W int w_qt_suit(const QtIn& c, const WarpIds& id, int suit, bool lead, bool 
   return qt;
 }
 
+// Can QuickTricks decide? Every suit's thread bounds its suit's quick tricks from above, as
+// if the opponents were out of trumps and partner could be reached; the walk over the
+// suits (w_quick_tricks) decides one call in eight, and is left out where the bounds do
+// not add up to the cutoff and none of its other answers can come: a suit neither opponent
+// holds, a ruff for the one trick needed, no quick trick when the opponents need one.
+DDG_W bool w_quick_possible(const WarpState& w, const WarpIds& id, const WarpTop& top, int cutoff, int cutoff_other) {
+  const int own = rt_len(top.a, 0), lho = rt_len(top.a, REL_L), part = rt_len(top.a, REL_P), rho = rt_len(top.a, REL_R);
+  const int win = rt_win(top.a), sec = rt_sec(top.a), longest = own > part ? own : part;
+  const int other = win == 0 ? part : own, most = lho > rho ? lho : rho;
+  const bool ours = !(win & 1) && win != REL_NONE;
+  // two top cards, or the third behind the left hand's second
+  const bool two = (!(sec & 1) && sec != REL_NONE) || (sec == REL_L && rt_thr(top.a) == REL_P);
+  const bool lone = (lho | rho) == 0 && longest != 0;
+  const int bound = lone || (most <= 1 && other <= 1) ? longest : !two ? 1 : most <= 2 ? longest : 2;
+  const u32 sum = w_add(id.t < 4 && (ours || lone) ? (u32)bound : 0u);
+  const bool no_trumps = w.trump < 0 || (w_shfl(top.a, w.trump & 3) & 0xFFFFu) == 0;
+  return (int)sum >= cutoff || w_any(lone && longest + 1 >= cutoff) || cutoff <= 1 || (cutoff_other <= 1 && no_trumps);
+}
+
 // QuickTricks (quick_tricks_impl): the leading side's sure tricks against `cutoff`;
 // decided = the answer is known (a count > 0: the leading side makes it).
 DDG_W int w_quick_tricks(const WarpState& w, const WarpIds& id, const WarpTop& top, int cutoff, int cutoff_other, u32& wr,
@@ -374,83 +443,70 @@ DDG_W int w_quick_tricks(const WarpState& w, const WarpIds& id, const WarpTop& t
   u32 entry = 0;  // [s] the entry card
   if (id.s == comm_suit) entry = 1u << rt_rank(top.ranks, by_win ? 0 : 1);
   // in the trump suit the entry is partner's top card, which by_win says as well
-  int qt = 0, suit = has_t ? trump : 0, lhoT = tl, rhoT = tr;
-  bool ruffed = false;
-  for (; suit <= 3; suit = qt_next_suit(suit, trump)) {
+  // The loop's state in one word: suit:3 | ruffed:1 | the opponents' trumps:4, 4 | count.
+  u32 state = (u32)(has_t ? trump : 0) | (u32)tl << 4 | (u32)tr << 8;
+  for (;;) {
+    state = w_uni(state);
+    const int suit = (int)(state & 7);
+    if (suit > 3) break;
+    u32 ruffed = state & 8;
+    int lhoT = (int)(state >> 4 & 15), rhoT = (int)(state >> 8 & 15), qt = (int)(state >> 12);
     const QtIn c = w_qt_in(w_shfl(top.a, suit), w_shfl(top.ranks, suit));
     const bool side = has_t && trump != suit;
-    const bool opps = (c.lho | c.rho) != 0;
     const bool no_ruff = !side || (lhoT == 0 && rhoT == 0);
-    if (!opps) {
-      if (c.part == 0) {  // only the leader holds the suit
-        if (c.own != 0 && no_ruff) {
-          qt += c.own;
-          if (qt >= cutoff) return qt;
+    bool one_hand = false;
+    if ((c.lho | c.rho) == 0) {
+      const bool only_lead = c.part == 0, only_part = comm && c.own == 0 && !only_lead;
+      one_hand = only_lead || only_part;
+      if (!only_lead) {
+        // The sure length of the partnership's suit may decide at once (qt_blocked_sum, from
+        // the leader's side and, with an entry, from partner's).
+        const bool in_t = has_t && suit == trump;
+        const int more = c.own > c.part ? c.own : c.part, less = c.own < c.part ? c.own : c.part;
+        const bool l0 = rt_len(top.a, 0) != 0, l2 = rt_len(top.a, REL_P) != 0;
+        const bool by_lead = w_any(id.s != trump && l0 && !l2) && c.own >= c.part;
+        const bool by_part = w_any(id.s != trump && !l0 && l2) && c.own <= c.part;
+        const int sum1 = in_t ? more + by_lead : less, sum2 = in_t ? more + by_part : less;
+        if (no_ruff && sum1 >= cutoff) return sum1;
+        if (comm && !only_part && no_ruff && sum2 >= cutoff) {
+          if (in_t) wr |= entry;
+          return sum2;
         }
-        continue;
       }
-      // The sure length of the partnership's suit may decide at once (qt_blocked_sum).
-      const bool only_part = comm && c.own == 0;
-#pragma unroll
-      for (int pass = 0; pass < 2; pass++) {
-        const bool by_lead = pass == 0;
-        if (!by_lead && (!comm || only_part)) continue;
-        int sum;
-        bool hit = false;
-        if (has_t && suit == trump) {
-          sum = c.own > c.part ? c.own : c.part;
-          const bool longer = by_lead ? c.own >= c.part : c.own <= c.part;
-          const int l0 = rt_len(top.a, 0), l2 = rt_len(top.a, REL_P);
-          const bool shortness = by_lead ? (l0 > 0 && l2 == 0) : (l2 > 0 && l0 == 0);
-          const u32 any = w_ballot(id.s != trump && shortness);
-          if (sum > 0 && longer && any) sum++;
-          hit = sum >= cutoff;
+      if (one_hand && no_ruff) {  // its cards (partner's over the entry)
+        qt += only_lead ? c.own : c.part;
+        if (only_part) wr |= entry;
+        if (qt >= cutoff) return qt;
+      }
+    }
+    if (!one_hand && c.win != REL_NONE) {
+      int res = QT_STAY;
+      if (c.win == 0 || (c.win == REL_P && comm)) {
+        const bool lead = c.win == 0, draws = lead && has_t && trump == suit && suit != comm_suit;
+        qt = w_qt_suit(c, id, suit, lead, side, draws, cutoff, lhoT, rhoT, comm_suit, lead ? 0u : entry, qt, wr, res);
+        if (res == QT_STOP) return qt;
+      }
+      // A ruff by partner.
+      if (res == QT_STAY && side && c.own > 0 && !ruffed && c.part == 0 && rt_len(ta, REL_P) > 0 &&
+          (qt == 0 || (c.win != 0 && c.win != REL_P && rt_win(ta) != 0 && rt_win(ta) != REL_P))) {
+        if ((c.rho > 0 || tr == 0) && (c.lho > 0 || tl == 0)) {
+          ruffed = 8;  // nobody can overruff
+          if (1 >= cutoff) return 1;
         } else {
-          sum = c.own < c.part ? c.own : c.part;
-          if (no_ruff) hit = sum >= cutoff;
+          const u32 pt = w_shfl(w.m, 4 * ((w.leader + 2) & 3) + trump);
+          const u32 lt = w_shfl(w.m, 4 * ((w.leader + 1) & 3) + trump);
+          const u32 rt = w_shfl(w.m, 4 * ((w.leader + 3) & 3) + trump);
+          if (((c.lho == 0 ? lt : 0) | (c.rho == 0 ? rt : 0)) < pt) {
+            ruffed = 8;
+            if (id.s == trump) wr |= 1u << w_top(pt);
+            if (1 >= cutoff) return 1;
+          }
         }
-        if (hit) {
-          if (!by_lead && has_t && suit == trump) wr |= entry;
-          return sum;
-        }
-      }
-      if (only_part) {  // only partner holds it: cashed over the entry
-        if (no_ruff) {
-          qt += c.part;
-          wr |= entry;
-          if (qt >= cutoff) return qt;
-        }
-        continue;
       }
     }
-    if (c.win == REL_NONE) continue;
-    int res = QT_STAY;
-    if (c.win == 0 || (c.win == REL_P && comm)) {
-      const bool lead = c.win == 0, draws = lead && has_t && trump == suit && suit != comm_suit;
-      qt = w_qt_suit(c, id, suit, lead, side, draws, cutoff, lhoT, rhoT, comm_suit, lead ? 0u : entry, qt, wr, res);
-    }
-    if (res == QT_STOP) return qt;
-    if (res == QT_NEXT) continue;
-    // A ruff by partner.
-    if (side && c.own > 0 && !ruffed && c.part == 0 && rt_len(ta, REL_P) > 0 &&
-        (qt == 0 || (c.win != 0 && c.win != REL_P && rt_win(ta) != 0 && rt_win(ta) != REL_P))) {
-      if ((c.rho > 0 || tr == 0) && (c.lho > 0 || tl == 0)) {
-        ruffed = true;  // nobody can overruff
-        if (1 >= cutoff) return 1;
-        continue;
-      }
-      const u32 pt = w_shfl(w.m, 4 * ((w.leader + 2) & 3) + trump);
-      const u32 lt = w_shfl(w.m, 4 * ((w.leader + 1) & 3) + trump), rt = w_shfl(w.m, 4 * ((w.leader + 3) & 3) + trump);
-      const u32 over = (c.lho == 0 ? lt : 0) | (c.rho == 0 ? rt : 0);
-      if (over < pt) {
-        ruffed = true;
-        if (id.s == trump) wr |= 1u << w_top(pt);
-        if (1 >= cutoff) return 1;
-      }
-      continue;
-    }
-    if (qt >= cutoff) return qt;
+    state = (u32)qt_next_suit(suit, trump) | ruffed | (u32)lhoT << 4 | (u32)rhoT << 8 | (u32)qt << 12;
   }
+  const int qt = (int)(state >> 12);
   if (qt == 0 && (!has_t || rt_win(ta) == REL_NONE)) {
     // No quick trick: the opponents win the first trick with a top card.
     if (rt_win(top.a) != REL_NONE && rt_len(top.a, 0) > 0) wr = 1u << rt_rank(top.ranks, 0);
@@ -598,8 +654,7 @@ DDG_W u32 w_run_tops(u32 own, u32 all) {
 DDG_W int w_lead_weight(const WarpState& w, const WarpTop& top, int card, int hint) {
   const int s = card_suit(card), r = card & 15, lead = w.leader, trump = w.trump;
   const u32 a = w_shfl(top.a, s), tk = w_shfl(top.ranks, s), all = w_shfl(w.all, s);
-  const u32 own = w_shfl(w.m, 4 * lead + s), risL = w_shfl(w.m, 4 * lho_of(lead) + s);
-  const u32 risP = w_shfl(w.m, 4 * partner_of(lead) + s), risR = w_shfl(w.m, 4 * rho_of(lead) + s);
+  const u32 own = w_shfl(w.m, 4 * lead + s);
   u32 ta = 0, hLT = 0, hPT = 0, hRT = 0;
   if (trump >= 0) {
     ta = w_shfl(top.a, trump);
@@ -625,7 +680,7 @@ DDG_W int w_lead_weight(const WarpState& w, const WarpTop& top, int card, int hi
   const bool p_long = (w2 == 0 && w3 == REL_P && lenP > 1) || (w2 == REL_P && w3 == 0 && lenP > 1);
   const bool pp = w2 == REL_P && w3 == REL_P;
   const bool w1_0 = w1 == 0, w1_p = w1 == REL_P, w2_p = w2 == REL_P;
-  const bool tops = risP > (risL | risR), lead_sec = seq & is_sec;
+  const bool tops = (a >> 28 & 1) != 0, lead_sec = seq & is_sec;
   int delta, base;
   bool with_rank;  // weight = delta + base (+ r_rank)
   if (trump >= 0 && rt_win(ta) != REL_NONE) {
@@ -712,47 +767,65 @@ DDG_W int w_follow_weight(const WarpState& w, int n, int seat, bool is_void, int
     }
     return base + (by_rank ? -rank : r_rank);
   }
-  // Void in the led suit: the discard's length and its top two cards at the trick's start.
-  const u32 sc = (u32)w_popc(me) << 6;
+  // Void in the led suit: weight = base - rank (or + r_rank) + the length's share (64 * length
+  // / D, by a multiplication) - a penalty for a bare top card or a guarded second one.
+  enum : u32 { K23 = 182361, K24 = 174763, K27 = 155344, K33 = 127100, K36 = 116509, K40 = 104858, K44 = 95326, K50 = 83886 };
+  const u32 length = (u32)w_popc(me);
   const int t1 = w_top(all) & 31, t2 = w_top(all & ~(1u << t1));
-  const bool one = sc == 64 && (me >> t1 & 1), two = sc == 128 && (t2 >= 0) & (me >> (t2 & 31) & 1);
+  const bool one = (length == 1) & (me >> t1 & 1), two = (length == 2) & (t2 >= 0) & (me >> (t2 & 31) & 1);
   const bool ruff = s == trump;
+  int base = 0, pen2 = 0, pen1 = 0;
+  u32 K;
+  bool with_rank = false;
   if (n == 1) {
     const u32 hPL = w_shfl(w.m, 4 * P + ls), hPT0 = w_shfl(w.m, 4 * P + (trump & 3)), hPT = has_t ? hPT0 : 0;
     const bool r_over = hRL > (hPL | lead_bit);  // 4th hand beats the trick
+    K = r_over ? K23 : K33;
+    pen2 = r_over ? 2 : 6;
+    pen1 = r_over ? 3 : 8;
     if (has_t) {
-      const int low_add = (int)(sc / 36) - (two ? 4 : 0), high_add = (int)(sc / 44);
       const bool p_in = hPL != 0, r_ruffs = !hRL && hRT;
       const bool pd_wins = p_in ? r_over || r_ruffs : (!hRL && hRT > hPT) || (!hPT && hRL > lead_bit);
       const bool safe = p_in || (r_ruffs && hRT > hPT);
       const bool high = ls == trump ? r_over : ruff ? safe | (bit > hPT) : pd_wins;
-      const int base = ls == trump ? 0 : ruff ? (high ? 24 : 15) : (high ? 60 : -2);
-      return base - rank + (high ? high_add : low_add);
+      base = ls == trump ? 0 : ruff ? (high ? 24 : 15) : (high ? 60 : -2);
+      K = high ? K44 : K36;
+      pen2 = high ? 0 : 4;
+      pen1 = 0;
     }
-    return -rank + (r_over ? (int)(sc / 23) - (two ? 2 : one ? 3 : 0) : (int)(sc / 33) - (two ? 6 : one ? 8 : 0));
+  } else if (n == 2) {
+    K = K24;
+    pen2 = pen1 = 4;
+    if (has_t) {
+      const int max4th = w_hi(hRL), m1r = rank2(move1);
+      const u32 hLL = w_shfl(w.m, 4 * lead + ls), allL = w_shfl(w.all, ls);
+      // the second card of the led suit was the leader's at the trick's start
+      const int l2 = w_top(allL & ~(1u << (w_top(allL) & 31)));
+      const bool sec_lead = l2 >= 0 && ((hLL | lead_bit) >> (l2 & 31) & 1);
+      const bool covered = high1 == 0 && lead0 > max4th && (max4th != 0 || !hRT);
+      const int follows = high1 == 0 ? (sec_lead ? 36 : 48) : 72, ruffed = high1 == 0 ? -12 : 36;
+      const bool ruffing = ruff & (ls != trump), under = (card_suit(move1) == trump) & (rank < m1r);
+      base = !ruffing ? 0 : covered ? -50 : under ? -32 : max4th != 0 ? follows : bit > hRT ? 48 : ruffed;
+      K = ruffing ? (covered ? 0 : under ? K40 : K50) : K40;
+      with_rank = ruffing & !covered & under;
+      pen2 = pen1 = 0;
+    }
+  } else {
+    const bool h2 = beats(c2, move1, trump);
+    const int move2 = h2 ? c2 : move1;
+    K = has_t ? K24 : K27;
+    pen2 = has_t ? 2 : 6;
+    pen1 = has_t ? 0 : 8;
+    if (has_t && ls != trump) {
+      const bool ours = !h2 && high1;  // partner is winning
+      const bool under = (card_suit(move2) == trump) & (rank <= rank2(move2));
+      base = ours ? (ruff ? 2 : 25) : ruff ? (under ? -13 : 33) : 14;
+      with_rank = ruff & !ours;
+      K = with_rank ? 0 : K;
+      pen2 = with_rank ? 0 : pen2;
+    }
   }
-  if (n == 2) {
-    const int max4th = w_hi(hRL), m1r = rank2(move1), m1s = card_suit(move1);
-    const u32 hLL = w_shfl(w.m, 4 * lead + ls), allL = w_shfl(w.all, ls);
-    if (!has_t) return -rank + (int)(sc / 24) - (two ? 4 : 0) - (one ? 4 : 0);
-    // the second card of the led suit was the leader's at the trick's start
-    const int l2 = w_top(allL & ~(1u << (w_top(allL) & 31)));
-    const bool sec_lead = l2 >= 0 && ((hLL | lead_bit) >> (l2 & 31) & 1);
-    const bool covered = high1 == 0 && lead0 > max4th && (max4th != 0 || !hRT);
-    const bool tops = bit > hRT;
-    const int base = high1 == 0 ? (max4th != 0 ? (sec_lead ? 36 : 48) : tops ? 48 : -12) : max4th != 0 ? 72 : tops ? 48 : 36;
-    const int plain = -rank + (int)(sc / 40);
-    const int ruffing = covered ? -rank - 50 : (m1s == trump) & (rank < m1r) ? -32 + r_rank + (int)(sc / 40) : base - rank + (int)(sc / 50);
-    return (ls == trump) | !ruff ? plain : ruffing;
-  }
-  const bool h2 = beats(c2, move1, trump);
-  const int move2 = h2 ? c2 : move1, m2r = rank2(move2);
-  const bool m2t = card_suit(move2) == trump;
-  if (!has_t) return -rank + (int)(sc / 27) - (two ? 6 : one ? 8 : 0);
-  const int val = (int)(sc / 24) - (two ? 2 : 0);
-  if (ls == trump) return -rank + val;
-  if (!h2 && high1) return (ruff ? 2 : 25) - rank + val;
-  return ruff ? (m2t & (rank <= m2r) ? -13 : 33) + r_rank : 14 - rank + val;
+  return base + (with_rank ? r_rank : -rank) + (int)(length * K >> 16) - (two ? pen2 : one ? pen1 : 0);
 }
 
 // Orders the candidates by weight (ties: highest card first, as insert_move keeps them)
@@ -762,8 +835,8 @@ DDG_W int w_order(const WarpIds& id, WarpFrame& f, u32 who, int card, int weight
   const u32 key = (u32)(weight + 1024) << 6 | (u32)card;
   int ahead = 0;
 #pragma unroll 1
-  for (u32 rest = who; rest; rest &= rest - 1) ahead += w_shfl(key, w_low(rest)) > key;
-  if (mine) f.mv[ahead] = (uint8_t)card;
+  for (u32 rest = who; (rest = w_uni(rest)) != 0; rest &= rest - 1) ahead += w_shfl(key, w_low(rest)) > key;
+  if (mine && ahead) f.mv[ahead - 1] = (uint8_t)card;
   return (int)w_shfl((u32)card, w_low(w_ballot(mine && ahead == 0)));
 }
 
@@ -812,58 +885,64 @@ DDG_W int w_compact(const WarpIds& id, WarpMem& sm, u32 cm, int seat, int& card)
 }
 
 // The frame's info word: value when no child cuts:1 | seat:2 | candidates:4 | the one being
-// searched:4 | undo leader:2 | its card:6 | win card:7 (64 = none).
+// searched:4 | -:2 | its card:6 | win card:7 (64 = none; set when it completed a trick).
 DDG_W u32 w_open_info(int seat, int n) { return (u32)(!ns_side(seat)) | (u32)seat << 1 | (u32)n << 3; }
 DDG_W int wi_result(u32 info) { return (int)(info & 1); }
 DDG_W int wi_seat(u32 info) { return (int)(info >> 1) & 3; }
 DDG_W int wi_n(u32 info) { return (int)(info >> 3) & 15; }
 DDG_W int wi_i(u32 info) { return (int)(info >> 7) & 15; }
-DDG_W int wi_undo_leader(u32 info) { return (int)(info >> 11) & 3; }
 DDG_W int wi_card(u32 info) { return (int)(info >> 13) & 63; }
 DDG_W int wi_win_card(u32 info) { return (int)(info >> 19) & 127; }
 enum : u32 { WI_NEXT = 1u << 7, WI_KEEP = (1u << 11) - 1 };  // one candidate on; what a play leaves
 
 DDG_W u32 w_tags(const TTBucket* b, const WarpIds& id) { return b->tag[id.t & 15]; }
 
-// A trick start. Entering it (enter_lead): cutoffs, the last trick, the TT probe, the
-// bounds; a bound's result is stored. Finishing it (`fin`, with its value v and relevant
-// cards w.rel, and the cutting card `best` or -1): the result is stored. Both need the
-// position's key and owner codes and end in the same store, so they share the code.
-// Returns the value, or -1 when the node expands (top and hint set).
+// ENTER at a trick start (enter_lead): cutoffs, the last trick, the TT probe, the bounds. The
+// value (w.rel set; `store`: a bound's, to be stored), or -1 when the node expands.
 template <class Env>
-DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool fin, int v, int best, WarpTop& top, int& hint) {
-  const int need = w.need;
-  if (!fin) {
-    w.rel = 0;
-    if (need <= 0) return 1;
-    if (w.left < need) return 0;
-    if (w.left == 1) {
-      const u32 bt = w_ballot(id.s == w.trump && w.all != 0);
-      const int su = bt ? w.trump : w_low(w_ballot(id.p == w.leader && w.m != 0)) & 3;
-      const u32 in = w_shfl(w.all, su);
-      if (id.s == su && w_popc(in) >= 2) w.rel = 1u << w_top(in);
-      return (int)(~w_shfl(w.code, su) >> 30 & 1);  // the top card's holder is N or S
-    }
+DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool& store, WarpTop& top, int& hint) {
+  w.rel = 0;
+  if (w.need <= 0) return 1;
+  if (w.left < w.need) return 0;
+  if (w.left == 1) {
+    const u32 bt = w_ballot(id.s == w.trump && w.all != 0);
+    const int su = bt ? w.trump : w_low(w_ballot(id.p == w.leader && w.m != 0)) & 3;
+    const u32 in = w_shfl(w.all, su);
+    if (id.s == su && w_popc(in) >= 2) w.rel = 1u << w_top(in);
+    return (int)(~w_shfl(w.code, su) >> 30 & 1);  // the top card's holder is N or S
   }
   const WarpKey k = w_key(w, id, env.mask());
-  TTBucket* b = env.table() + k.bucket;
-  const u32 tagw = w_tags(b, id);
-  if (!fin) {
-    const int hit = w_probe(w, id, b, tagw, k, w.code, need, hint);
-    if (hit >= 0) return hit;
-    top = w_make_top(w, id, k);
-    const bool ns_lead = ns_side(w.leader);
-    const int cut_ns = need, cut_ew = w.left - need + 1;
-    bool decided;
-    u32 wr;
-    const int q = w_quick_tricks(w, id, top, ns_lead ? cut_ns : cut_ew, ns_lead ? cut_ew : cut_ns, wr, decided);
-    if (decided) v = ns_lead ? q != 0 : q == 0;
-    else if (w_later_tricks(w, id, top, wr)) v = !ns_lead;
-    else return -1;
-    w.rel = wr;
-  }
-  w_store(w, id, b, tagw, k, w.code, w.rel, v ? need : 0, v ? w.left : need - 1, best);
+  const TTBucket* b = env.table() + k.bucket;
+  const int hit = w_probe(w, id, b, w_tags(b, id), k, w.code, w.need, hint);
+  if (hit >= 0) return hit;
+  top = w_make_top(w, id, k);
+  const bool ns_lead = ns_side(w.leader);
+  const int cut_ns = w.need, cut_ew = w.left - w.need + 1;
+  bool decided;
+  u32 wr;
+  int q = 0, v;
+  const int cut = ns_lead ? cut_ns : cut_ew, cut_other = ns_lead ? cut_ew : cut_ns;
+  decided = w_quick_possible(w, id, top, cut, cut_other);
+  if (decided) q = w_quick_tricks(w, id, top, cut, cut_other, wr, decided);
+  if (decided) v = ns_lead ? q != 0 : q == 0;
+  else if (w_later_tricks(w, id, top, wr)) v = !ns_lead;
+  else return -1;
+  w.rel = wr;
+  store = true;
   return v;
+}
+
+// A trick start's result goes to the table (a bound's, or a finished node's with its
+// cutting card `best` or -1).
+template <class Env>
+DDG_W void w_put(WarpState& w, const WarpIds& id, Env& env, int v, int best) {
+  const WarpKey k = w_key(w, id, env.mask());
+  TTBucket* b = env.table() + k.bucket;
+  w_store(w, id, b, w_tags(b, id), k, w.code, w.rel, v ? w.need : 0, v ? w.left : w.need - 1, best);
+}
+
+DDG_W WarpFrame& w_frame(WarpMem& sm, u32 st) {
+  return *reinterpret_cast<WarpFrame*>(reinterpret_cast<char*>(sm.fr) + (st & SW_OFF));
 }
 
 // A node expands (gen_moves_lead, gen_moves_follow): its candidates, one per run of alike
@@ -874,7 +953,7 @@ DDG_W int w_expand(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, const
   const u32 cm = w_run_tops(w.m, w.all);
   const u32 in_led = w_shfl(cm, 4 * seat + ls);
   const u32 led = w.nplayed ? in_led : 0;
-  WarpFrame& f = sm.fr[w.sp];
+  WarpFrame& f = w_frame(sm, w.st);
   u32 who = led;  // the threads that stand for a candidate
   int n = w_popc(led), card = ls * 16 + (id.t & 15);  // following suit: thread r for rank r
   if (!led) {
@@ -884,20 +963,18 @@ DDG_W int w_expand(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, const
   w.at = 0;
   w.info = w_open_info(seat, n);
   if (n == 1) {
-    card = (int)w_shfl((u32)card, w_low(who));
-    if (id.t == 0) f.mv[0] = (uint8_t)card;
-    return card;
+    return (int)w_shfl((u32)card, w_low(who));
   }
   if (led && w.nplayed > 1) {
     const u32 win = led & (0xFFFFFFFFu << w_follow_floor(w, w.nplayed, seat, led)), lose = led & ~win;
     const u32 below = (1u << id.t) - 1;
     const int ahead = win >> id.t & 1 ? w_popc(win & below) : w_popc(win) + w_popc(lose & below);
-    if (led >> id.t & 1) f.mv[ahead] = (uint8_t)card;
+    if ((led >> id.t & 1) && ahead) f.mv[ahead - 1] = (uint8_t)card;
     return ls * 16 + w_low(win ? win : led);
   }
   int weight;
   if (w.nplayed == 0) {
-    if (hint < 0 && w.sp == 0) {  // the root, no TT move: an outside hint, when the leader holds it
+    if (hint < 0 && (w.st & SW_OFF) == 0) {  // the root, no TT move: an outside hint, when the leader holds it
       const int h = env.root_hint(sm.job);
       if (h >= 0 && h < 64 && (w_shfl(w.m, 4 * seat + (h >> 4)) >> (h & 15) & 1)) hint = h;
     }
@@ -920,9 +997,9 @@ DDG_W int w_enter_follow(WarpState& w, const WarpIds& id) {
 // Plays `card` from the top frame and pushes the frame (play): at the fourth card the
 // trick is settled and the frame keeps what taking it back needs.
 DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, int card) {
-  WarpFrame& f = sm.fr[w.sp];
-  const int seat = wi_seat(w.info), su = card_suit(card), r = card & 15;
-  const u32 bit = 1u << r, code = w.code, trick = w.trick;
+  WarpFrame& f = w_frame(sm, w.st);
+  const int seat = wi_seat(w.info), su = card_suit(card), r = card & 15, np8 = (int)(w.st & SW_NP8);
+  const u32 bit = 1u << r, code = w.code, st = w.st, trick = w.trick;
   u32 info = (w.info & WI_KEEP) | (u32)card << 13;
   if (id.s == su) {
     // The card's owner leaves the code: the owners of the cards below move up.
@@ -932,53 +1009,49 @@ DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, int card) {
     w.now ^= bit;
   }
   if ((id.t & 15) == seat * 4 + su) w.m ^= bit;
-  w.trick |= (u32)card << (8 * w.nplayed);
-  w.nplayed++;
-  if (w.nplayed == 4) {
+  w.trick |= (u32)card << np8;
+  if (np8 == 24) {
     const int c = (int)(w.trick >> (8 * (id.t & 3))) & 0xFF, cs = card_suit(c);
     const u32 key = (cs == w.trump ? 512u : cs == card_suit((int)(w.trick & 0xFF)) ? 256u : 0u) | (u32)c << 2 | (u32)(id.t & 3);
     const u32 best = w_max(key);
-    const int wc = (int)(best >> 2) & 63;
+    const int wc = (int)(best >> 2) & 63, leader = (int)((st + best) & 3);
     const int same = w_popc(w_ballot(cs == card_suit(wc)) & 15);  // at least two: won by rank
-    info |= (u32)w.leader << 11 | (u32)(same >= 2 ? wc : 64) << 19;
+    info |= (u32)(same >= 2 ? wc : 64) << 19;
     if (id.t < 4) f.all[id.t] = (uint16_t)w.all;
     w.all = w.now;
-    w.leader = (w.leader + (int)(best & 3)) & 3;
     w.trick = 0;
-    w.nplayed = 0;
-    w.left--;
-    w.need -= ns_side(w.leader);
+    w.st = ((st & ~(SW_LEADER | SW_NP8)) | (u32)leader) + SW_FRAME - SW_LEFT - (ns_side(leader) ? SW_NEED : 0);
+  } else {
+    w.st = st + SW_CARD + SW_FRAME;
   }
   if (id.t < 4) {
     f.suit[id.t].at = w.at;
     f.suit[id.t].code = code;
   }
   if (id.t == 4) {
-    f.trick = trick;
+    f.st = st;
     f.info = info;
+    f.trick = trick;
   }
-  w.sp++;
   w_sync();
 }
 
 // Pops the top frame and takes its card back (node_done, unplay); returns the card.
 DDG_W int w_unplay(WarpState& w, const WarpIds& id, WarpMem& sm) {
-  w.sp--;
-  const WarpFrame& f = sm.fr[w.sp];
+  const bool completed = (w.st & SW_NP8) == 0;  // this ply completed a trick
+  const WarpFrame& f = w_frame(sm, w.st - SW_FRAME);
+  w.st = f.st;
+  w.info = f.info;
+  w.trick = f.trick;
   w.at = f.suit[id.s].at;
   w.code = f.suit[id.s].code;
-  w.trick = f.trick;
-  w.info = f.info;
+  w_unpack(w);
   const int card = wi_card(w.info), su = card_suit(card);
-  if (w.nplayed == 0) {  // this ply completed a trick
+  if (completed) {
     w.all = f.all[id.s];
-    w.need += ns_side(w.leader);
-    w.left++;
-    w.leader = wi_undo_leader(w.info);
     const int wc = wi_win_card(w.info);
     if (id.s == card_suit(wc)) w.rel |= 1u << (wc & 15);  // (none: suit 4)
   }
-  w.nplayed = (w.nplayed - 1) & 3;
   const u32 bit = 1u << (card & 15);
   if (id.s == su) w.now ^= bit;
   if ((id.t & 15) == wi_seat(w.info) * 4 + su) w.m ^= bit;
@@ -987,10 +1060,10 @@ DDG_W int w_unplay(WarpState& w, const WarpIds& id, WarpMem& sm) {
 
 // The frame's next candidate that is not a small card like one tried before (step_next):
 // every candidate is tested by its thread. -1: none left.
-DDG_W int w_next(WarpState& w, const WarpIds& id, const WarpMem& sm) {
+DDG_W int w_next(WarpState& w, const WarpIds& id, WarpMem& sm) {
   const int n = wi_n(w.info), i = wi_i(w.info);
   if (i >= n) return -1;
-  const int c = sm.fr[w.sp].mv[id.t & 15];
+  const int c = w_frame(sm, w.st).mv[(id.t - 1) & 15];  // (the first one is not asked for again)
   const u32 at = w_shfl(w.at, card_suit(c));
   const u32 acc = at & 0xFFFFu, tried = at >> 16, bit = 1u << (c & 15);
   const u32 small = (acc & (0u - acc)) - 1;  // below the lowest relevant card (all, when there is none)
@@ -1013,27 +1086,24 @@ DDG_W u32 w_widen(const WarpState& w, const WarpIds& id) {
 
 // ---- root searches (start_search, start_lead, root_result) -----------------------------------
 
-DDG_W void w_start_search(WarpState& w, const WarpJob& j) {
-  w.leader = (j.decl + 1) & 3;
-  w.nplayed = 0;
-  w.left = j.cards;
+DDG_W void w_start_search(WarpState& w, const WarpJob& j, int target) {
+  w.st = (u32)((j.decl + 1) & 3) | (u32)j.cards * SW_LEFT | (u32)target * SW_NEED;
   w.trick = 0;
-  w.sp = 0;
 }
 
 // Starts the trick count of the current declarer: the binary search at `first`, or the
 // stepping search from the seed `first`. (A deal has at least one card each, so every
 // lead needs a search.)
 DDG_W void w_start_lead(WarpState& w, const WarpIds& id, WarpJob& j, int first) {
-  int lo = 0, hi = 13;
+  int lo = 0, hi = 13, target;
   if (j.mode == MODE_BISECT) {
-    w.need = first < 1 ? 1 : first > 13 ? 13 : first;
+    target = first < 1 ? 1 : first > 13 ? 13 : first;
   } else {
     lo = first < 0 ? 0 : first > j.cards ? j.cards : first;
     hi = lo == 0 ? PH_UP : PH_FIRST;
-    w.need = lo == 0 ? 1 : lo;
+    target = lo == 0 ? 1 : lo;
   }
-  w_start_search(w, j);
+  w_start_search(w, j, target);
   w_sync();
   if (id.t == 0) {
     j.lo = (int8_t)lo;
@@ -1082,20 +1152,19 @@ DDG_W bool w_end_root(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, in
   int lo = j.lo, hi = j.hi;
   const int next = w_root_result(j.mode, j.cards, w.need, v, lo, hi);
   w_sync();
-  if (next >= 0) {
-    w.need = next;
+  if (w_any(next >= 0)) {
     if (id.t == 0) {
       j.lo = (int8_t)lo;
       j.hi = (int8_t)hi;
     }
     w_sync();
-    w_start_search(w, j);
+    w_start_search(w, j, next);
     return true;
   }
   env.answer(j, lo);
   const int decl = j.decl + 1;
   w_sync();
-  if (decl > j.last_decl) {
+  if (w_any(decl > j.last_decl)) {
     w_flush(w, id, sm);
     env.job_done(j);
     return false;
@@ -1111,42 +1180,46 @@ DDG_W bool w_end_root(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, in
 // start with a job, ST_ENTER to go on inside one (w and the frames as they were saved); on
 // return ST_IDLE (nothing left), ST_TAKE or ST_ENTER (stopped). An Env offers
 //   bool take(w, id, sm)   the next job: position, job record (else stage is set)
-//   bool stop(w, id, sm)   asked every 64 nodes: true ends the warp
+//   bool stop(w, id, sm)   asked every 256 nodes: true ends the warp
 //   int seed(job), root_hint(job); void answer(job, ns), root_best(job, card), job_done(sm)
 //   TTBucket* table(); u32 mask()
 template <class Env>
 DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
-  bool in_job = sm.job.stage == ST_ENTER;
+  bool in_job = sm.job.stage == ST_ENTER, stopped = false;
   for (;;) {
-    if (!in_job) {
-      if (!env.take(w, id, sm)) return;
+    if (w_any(!in_job)) {
+      if (!w_any(env.take(w, id, sm))) return;
       WarpJob& j = sm.job;
       w_start_lead(w, id, j, env.seed(j));
       in_job = true;
     }
+    w.trump = (int)w_uni((u32)w.trump);
     // One node per turn: entered, then the frames it closes, up to the next card played.
     for (;;) {
-      if ((w.nodes & 63u) == 63u && env.stop(w, id, sm)) return;
-      w.nodes++;
-      int v = -1, card = -1, best = -1, hint = -1;
-      bool fin = false, done = false;
-      WarpTop top = {0, 0};
-      for (;;) {
-        if (w.nplayed == 0) v = w_lead(w, id, env, fin, v, best, top, hint);
-        else v = w_enter_follow(w, id);
-        if (v < 0) {
-          card = w_expand(w, id, sm, env, top, hint);
+      w.st = w_uni(w.st);
+      w.trick = w_uni(w.trick);
+      w_unpack(w);
+      if (w_any((w.nodes & 255u) == 255u)) {
+        if (env.stop(w, id, sm)) {
+          stopped = true;
           break;
         }
+      }
+      w.nodes++;
+      int card = -1, best = -1, hint = -1;
+      bool store = false;
+      WarpTop top = {0, 0};
+      int v = w.nplayed == 0 ? w_lead(w, id, env, store, top, hint) : w_enter_follow(w, id);
+      if (v < 0) {
+        card = w_expand(w, id, sm, env, top, hint);
+      } else {
         // The node is decided: its card is taken back, and the frames it completes with it.
         for (;;) {
-          if (w.sp == 0) {
-            done = true;  // the root search
-            break;
-          }
+          if (w_any(store)) w_put(w, id, env, v, best);
+          if ((w.st & SW_OFF) == 0) break;  // the root search is done
           const int c = w_unplay(w, id, sm);
           best = -1;
-          if (v == (int)ns_side(wi_seat(w.info))) {  // the child cuts
+          if (w_any(v == (int)ns_side(wi_seat(w.info)))) {  // the child cuts
             w.at = (w.at & 0xFFFF0000u) | w.rel;
             best = c;
           } else {
@@ -1157,18 +1230,16 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
             v = wi_result(w.info);
           }
           w.rel = w_widen(w, id);
-          if (w.nplayed == 0) break;
+          store = w.nplayed == 0;
         }
-        if (done || card >= 0) break;
-        fin = true;  // a trick start: its result is stored
       }
-      if (done) {
+      if (w_any(card < 0)) {
         in_job = w_end_root(w, id, sm, env, v, best);
-        if (!in_job) break;
+        if (w_any(!in_job)) break;
         continue;
       }
 #ifdef DDG_BOUNDS_CHECK
-      if (w.sp >= STACK_DEPTH) {  // counted, skipped: the warp stops, its results stay unsolved
+      if ((w.st & SW_OFF) >= STACK_DEPTH * SW_FRAME) {  // counted, skipped: the warp stops, its results stay unsolved
         w_count(w, id, WCNT_BOUNDS, 1);
         w_flush(w, id, sm);
         if (id.t == 0) sm.job.stage = ST_IDLE;
@@ -1177,6 +1248,7 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
 #endif
       w_play(w, id, sm, card);
     }
+    if (w_any(stopped)) return;  // (a return out of both loops would cost ptxas the proof)
   }
 }
 

@@ -6,15 +6,15 @@
 // Searcher w of block b owns the TT slice, the stack area and the save slot of lane
 // b * warps + w.
 //
-// What bounds it: instruction fetch and issue. A node takes about 434 warp instructions (a
-// lane of batch_kernel took ~3,030 thread instructions on one thread of a warp that was
-// 35 % full), and 16 warps on an SM issue as much as 32 (1.8 a cycle), since warps that
-// stand at different places of the code share few fetches. Measured against batch_kernel
-// (block phases, 512 lanes to an SM): random 13-card deals with every SM full 1.18 against
-// 0.70 G nodes/s; one job alone on an SM about 1 M against 0.15 M nodes/s; 240 quick
-// 13-card deals 109 against 1,405 ms; 65,536 six-card endings 158 against 376 ms; 1,200
-// nine-card endings 135 against 1,117 ms; the 20 leads of a five-card ending asked one by
-// one 3.2 against 19.2 ms. batch_kernel stays for helping and for its own options.
+// What bounds it: on a full SM instruction fetch (the code a node may run is some 36 KB, the
+// SM's instruction cache holds 32 KB, and the misses fill the cache that the SMs of a GPC
+// share: 4.0 lines a cycle, all of it); alone on an SM one warp's chain of about 390
+// instructions a node, 1,760 cycles. Measured against batch_kernel (block phases, 512 lanes
+// to an SM): random 13-card deals with every SM full 1.82 against 0.70 G nodes/s; one job
+// alone on an SM 1.1 M against 0.15 M nodes/s; 240 quick 13-card deals 94 against 1,453 ms;
+// 65,536 six-card endings 150 against 377 ms; 1,200 nine-card endings (a job per lead) 135
+// against 1,117 ms; the 20 leads of a five-card ending asked one by one 3.5 against 23 ms.
+// batch_kernel stays for helping and for its own options.
 #pragma once
 #include "ddg_kernel.cuh"
 #include "ddg_warp.cuh"
@@ -29,9 +29,9 @@ enum { WARP_MAX = 32 };
 // below the top go to the lane's stack area.)
 struct WarpSave {
   uint16_t m[16], all[4], now[4];
-  u32 trick;
   u32 code[4];
-  int8_t trump, leader, nplayed, left, need, sp;
+  u32 st, trick;
+  int trump;
   WarpJob job;
 };
 static_assert(sizeof(WarpSave) <= sizeof(LaneSave), "a searcher's state fits its lane's save slot");
@@ -43,12 +43,104 @@ struct WarpBlock {
   int busy;        // stream: searchers with a job
   int idle_exit;   // stream: waiting searchers end (1: nothing will come, 2: stopped by the host)
   unsigned polls;  // stream: looks at the ring
+  int halt;        // stopped by the host
+  unsigned asks;   // questions whether to stop
   int running;     // searchers that did not end idle
   unsigned long long nodes, jobs_done, total[WCNT_COUNT];
   WarpMem warp[1];  // as many as the block has warps
 };
 inline size_t warp_smem(int warps) { return sizeof(WarpBlock) + sizeof(WarpMem) * (size_t)(warps - 1); }
 
+// Is the slice over, or the solve stopped by the host? In one thread. The host's flag is a
+// read over the bus, and the GPU does about 1.15 M of those a second however many SMs ask: a
+// read by every searcher every 1,024 nodes held the whole GPU at 1.18 G nodes/s. So one
+// question of a block in 64 reads it, and the others see what that one found.
+__device__ __forceinline__ int warp_ask(WarpBlock* sh, u64 t_end) {
+  const BatchArgs& a = sh->args;
+  volatile int* halt = &sh->halt;
+  if ((atomicAdd(&sh->asks, 1u) & 63u) == 63u && a.stop && *a.stop) *halt = 1;
+  return *halt | (int)(t_end && global_ns() > t_end);
+}
+
+// One look at the stream's ring, in one thread: 1 a job taken, 0 nothing will come, -1 stopped
+// by the host, -2 nothing now. One searcher of a block looks at a time.
+__device__ __forceinline__ int warp_stream_look(WarpBlock* sh, unsigned long long& job) {
+  const BatchArgs& a = sh->args;
+  volatile int* vexit = &sh->idle_exit;
+  volatile u64* vsince = &sh->idle_since;
+  int got = -2;
+  if (*vexit) return *vexit == 1 ? 0 : -1;
+  if (atomicCAS(&sh->polling, 0, 1) != 0) return got;
+  DevEnv q;
+  q.a = &a;
+  const bool closing = *reinterpret_cast<const volatile int*>(a.closing) != 0;
+  // The host's flag costs a read over the bus: looked at in every 256th look, here only (a
+  // read by every waiting searcher held up the whole kernel: 400 deals took 1.76 s).
+  if ((sh->polls++ & 255u) == 255u && stop_requested(a, 0)) {
+    *vexit = 2;
+    got = -1;
+  } else if (closing && !q.stream_more()) {
+    *vexit = 1;  // nothing more will come for any searcher
+    got = 0;
+  } else if (q.stream_take(job)) {
+    atomicAdd(&sh->busy, 1);
+    *vsince = 0;
+    got = 1;
+  } else if (*reinterpret_cast<volatile int*>(&sh->busy) == 0) {
+    const u64 now = global_ns();
+    if (!*vsince) *vsince = now;
+    else if (now - *vsince > a.idle_ns) *vexit = 1;
+  } else {
+    *vsince = 0;
+  }
+  __threadfence_block();
+  atomicExch(&sh->polling, 0);
+  return got;
+}
+
+// The next job of a batch, in one thread: 1 taken, 0 none left, -1 stopped.
+__device__ __forceinline__ int warp_next_job(WarpBlock* sh, const WarpJob& j, int wid, u64 t_end, unsigned long long& job) {
+  const BatchArgs& a = sh->args;
+  if (warp_ask(sh, t_end)) return -1;
+  // The first job of the launch is dealt round-robin over the blocks, so that a small batch
+  // spreads over every SM; later ones come from the shared counter.
+  const long long rr = (long long)wid * gridDim.x + blockIdx.x;
+  if (j.job < 0 && rr < a.rr_jobs) job = (unsigned long long)rr;
+  else job = atomicAdd(a.next_job, 1ull) + (unsigned long long)a.rr_jobs;
+  return (long long)job < a.n_jobs;
+}
+
+// The job's record.
+__device__ __forceinline__ void warp_set_job(const BatchArgs& a, WarpJob& j, unsigned long long job, int t) {
+  const unsigned long long deal = a.jpd == 5 ? job / 5 : job / 20;
+  const int sub = (int)(job - deal * a.jpd);
+  const bool all = a.jpd == 5;
+  j.job = (long long)job;
+  j.deal = (long long)deal;
+  j.strain = (int8_t)(a.one_job ? a.one_strain : all ? sub : sub >> 2);
+  j.decl = (int8_t)(a.one_job ? (a.one_decl >= 0 ? a.one_decl : 0) : all ? 0 : sub & 3);
+  j.last_decl = (int8_t)(a.one_job ? (a.one_decl >= 0 ? a.one_decl : 3) : all ? 3 : sub & 3);
+  j.mode = (int8_t)a.mode;
+  j.start_nodes = j.nodes;
+  if (a.job_start_ns && t == 0) a.job_start_ns[job] = global_ns();
+}
+
+// A job's end, in one thread.
+template <bool STREAM>
+__device__ __forceinline__ void warp_job_done(WarpBlock* sh, WarpJob* j) {
+  const BatchArgs& a = sh->args;
+  if (a.job_nodes) a.job_nodes[j->job] = j->nodes - j->start_nodes;
+  if (a.job_end_ns) a.job_end_ns[j->job] = global_ns();
+  j->jobs_done++;
+  if (STREAM) {
+    stream_deal_done(a, j->deal);
+    atomicSub(&sh->busy, 1);
+  }
+}
+
+// STREAM: the jobs come from a stream's ring. (A kernel of its own: what it takes to wait for
+// deals would cost every other launch the compiler's proof that warps stay together.)
+template <bool STREAM>
 struct WarpEnv {
   WarpBlock* sh;
   TTBucket* tt;
@@ -59,7 +151,7 @@ struct WarpEnv {
   __device__ __forceinline__ TTBucket* table() { return tt; }
   __device__ __forceinline__ u32 mask() const { return (1u << sh->args.tt_log2) - 1; }
   __device__ __forceinline__ long long out_row(const WarpJob& j) const {
-    return sh->args.ring ? (j.deal & sh->args.ring_mask) : j.deal;
+    return STREAM ? (j.deal & sh->args.ring_mask) : j.deal;
   }
   __device__ __forceinline__ long long entry(const WarpJob& j) const { return out_row(j) * 20 + j.strain * 4 + j.decl; }
   // Ring slots are rewritten while the kernel runs: their values come from L2.
@@ -79,113 +171,44 @@ struct WarpEnv {
     if ((threadIdx.x & 31) == 0) sh->args.out20[entry(j)] = (uint8_t)((j.decl & 1) == 0 ? ns : 13 - ns);
   }
   __device__ __forceinline__ void job_done(WarpJob& j) {
-    const BatchArgs& a = sh->args;
-    if ((threadIdx.x & 31) == 0) {
-      if (a.job_nodes) a.job_nodes[j.job] = j.nodes - j.start_nodes;
-      if (a.job_end_ns) a.job_end_ns[j.job] = global_ns();
-      j.jobs_done++;
-      if (a.ring) {
-        stream_deal_done(a, j.deal);
-        atomicSub(&sh->busy, 1);
-      }
-    }
+    if ((threadIdx.x & 31) == 0) warp_job_done<STREAM>(sh, &j);
     __syncwarp();
-  }
-
-  // The stream's next job, in thread 0: 1 taken, 0 nothing will come, -1 stopped. One
-  // searcher of a block looks at the ring at a time; the others wait longer the more of
-  // the block's searchers are busy, so that deals spread over the SMs.
-  __device__ __noinline__ int stream_next(unsigned long long& job) {
-    const BatchArgs& a = sh->args;
-    volatile int* vbusy = &sh->busy;
-    volatile int* vexit = &sh->idle_exit;
-    volatile u64* vsince = &sh->idle_since;
-    DevEnv q;
-    q.a = &a;
-    for (;;) {
-      if (*vexit) return *vexit == 1 ? 0 : -1;
-      if (atomicCAS(&sh->polling, 0, 1) == 0) {
-        int got = -2;
-        const bool closing = *reinterpret_cast<const volatile int*>(a.closing) != 0;
-        // The host's flag costs a read over the bus: looked at in every 256th look, here
-        // only (a read by every waiting searcher held up the whole kernel: 400 deals took
-        // 1.76 s).
-        if ((sh->polls++ & 255u) == 255u && stop_requested(a, 0)) {
-          *vexit = 2;
-          got = -1;
-        } else if (closing && !q.stream_more()) {
-          *vexit = 1;  // nothing more will come for any searcher
-          got = 0;
-        } else if (q.stream_take(job)) {
-          atomicAdd(&sh->busy, 1);
-          *vsince = 0;
-          got = 1;
-        } else if (*vbusy == 0) {
-          const u64 now = global_ns();
-          if (!*vsince) *vsince = now;
-          else if (now - *vsince > a.idle_ns) *vexit = 1;
-        } else {
-          *vsince = 0;
-        }
-        __threadfence_block();
-        atomicExch(&sh->polling, 0);
-        if (got != -2) return got;
-      }
-      __nanosleep(1000u + 500u * (unsigned)*vbusy);
-    }
   }
 
   __device__ __forceinline__ bool take(WarpState& w, const WarpIds& id, WarpMem& sm) {
     const BatchArgs& a = sh->args;
     WarpJob& j = sm.job;
     __syncwarp();
-    int got = 1;
     unsigned long long job = 0;
-    if (id.t == 0) {
-      if (a.ring) {
-        got = stream_next(job);
-      } else if ((t_end && global_ns() > t_end) || ((j.jobs_done & 15u) == 15u && stop_requested(a, 0))) {
-        got = -1;  // (the host's flag costs a read over the bus: looked at for every 16th job)
-      } else {
-        // The first job of the launch is dealt round-robin over the blocks, so that a small
-        // batch spreads over every SM; later ones come from the shared counter.
-        const long long rr = (long long)wid * gridDim.x + blockIdx.x;
-        if (j.job < 0 && rr < a.rr_jobs) job = (unsigned long long)rr;
-        else job = atomicAdd(a.next_job, 1ull) + (unsigned long long)a.rr_jobs;
-        if ((long long)job >= a.n_jobs) got = 0;
+    int got = -2;
+    if (STREAM) {
+      for (;;) {
+        if (id.t == 0) got = warp_stream_look(sh, job);
+        got = (int)w_uni((u32)got);
+        if (got != -2) break;
+        // the busier the block, the longer the wait: deals spread over the SMs
+        __nanosleep(1000u + 500u * (unsigned)*reinterpret_cast<volatile int*>(&sh->busy));
       }
-      if (got != 1) {
-        j.stage = got == 0 ? ST_IDLE : ST_TAKE;
-      } else {
-        j.job = (long long)job;
-        j.deal = j.job / a.jpd;
-        const int sub = (int)(j.job - j.deal * a.jpd);
-        j.strain = (int8_t)(a.jpd == 5 ? sub : sub >> 2);
-        j.decl = (int8_t)(a.jpd == 5 ? 0 : sub & 3);
-        j.last_decl = (int8_t)(a.jpd == 5 ? 3 : sub & 3);
-        if (a.one_job) {
-          j.strain = (int8_t)a.one_strain;
-          j.decl = (int8_t)(a.one_decl >= 0 ? a.one_decl : 0);
-          j.last_decl = (int8_t)(a.one_decl >= 0 ? a.one_decl : 3);
-        }
-        j.mode = (int8_t)a.mode;
-        j.start_nodes = j.nodes;
-        if (a.job_start_ns) a.job_start_ns[j.job] = global_ns();
-      }
+    } else {
+      if (id.t == 0) got = warp_next_job(sh, j, wid, t_end, job);
+      got = (int)w_uni((u32)got);
     }
-    got = __shfl_sync(0xFFFFFFFFu, got, 0);
+    if (id.t == 0) j.stage = got == 0 ? ST_IDLE : ST_TAKE;
     if (got != 1) return false;
+    // By all threads, which write the same values: nested branches in a one-thread region
+    // would cost the compiler its proof that the warp is together afterwards.
+    warp_set_job(a, j, (unsigned long long)w_uni((u32)(job >> 32)) << 32 | w_uni((u32)job), id.t);
     __syncwarp();
-    const long long row = a.ring ? (j.deal & a.ring_mask) : j.deal;
-    const unsigned short* h = reinterpret_cast<const unsigned short*>((a.ring ? a.ring : a.hands) + row * 4);
-    w.m = (a.ring ? __ldcg(h + 4 * id.p + id.s) : h[4 * id.p + id.s]) & 0x1FFFu;
+    const long long row = STREAM ? (j.deal & a.ring_mask) : j.deal;
+    const unsigned short* h = reinterpret_cast<const unsigned short*>((STREAM ? a.ring : a.hands) + row * 4);
+    w.m = (STREAM ? __ldcg(h + 4 * id.p + id.s) : h[4 * id.p + id.s]) & 0x1FFFu;
     w.all = w.now = w_shfl(w.m, id.s) | w_shfl(w.m, 4 + id.s) | w_shfl(w.m, 8 + id.s) | w_shfl(w.m, 12 + id.s);
     w.code = w_build_code(w, id);
     const int cards = (int)w_add(id.t < 4 ? (u32)w_popc(w.m) : 0u);
     w.trump = strain_trump(j.strain);
     // A new TT generation; at the wrap all tags are cleared, by the whole warp.
     w.gen++;
-    if (w.gen >= (1u << GEN_BITS)) {
+    if (w_any(w.gen >= (1u << GEN_BITS))) {
       const u32 n = (mask() + 1) * 4;
       for (u32 k = id.t; k < n; k += 32) reinterpret_cast<uint4*>(tt[k >> 2].tag)[k & 3] = make_uint4(0, 0, 0, 0);
       w.gen = 1;
@@ -196,31 +219,28 @@ struct WarpEnv {
   }
 
   __device__ __forceinline__ bool stop(WarpState& w, const WarpIds& id, WarpMem& sm) {
-    const bool look = (w.nodes & 1023u) == 1023u;  // the host's flag costs a read over the bus
-    if (!look && !t_end) return false;
     int end = 0;
-    if (id.t == 0) {
-      if (look) end = stop_requested(sh->args, t_end);
-      else end = global_ns() > t_end;
-    }
-    end = __shfl_sync(0xFFFFFFFFu, end, 0);
-    if (end || (w.nodes & 0xFFFFu) == 0xFFFFu) w_flush(w, id, sm);
-    if (end && id.t == 0) sm.job.stage = ST_ENTER;
-    return end != 0;
+    if (id.t == 0) end = warp_ask(sh, t_end);
+    const bool over = w_any(end != 0);
+    if (w_any(over || (w.nodes & 0xFFFFu) == 0xFFFFu)) w_flush(w, id, sm);
+    if (over && id.t == 0) sm.job.stage = ST_ENTER;
+    return over;
   }
 };
 
+template <bool STREAM>
 __global__ void __launch_bounds__(WARP_MAX * 32, 1) warp_kernel(BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpBlock& sh = *reinterpret_cast<WarpBlock*>(smem_raw);
-  const int wid = threadIdx.x >> 5, t = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int wid = (int)w_uni(threadIdx.x >> 5), t = threadIdx.x & 31, warps = blockDim.x >> 5;
   const long long lane = (long long)blockIdx.x * warps + wid;
   const u64 t_end = a.slice_ns ? global_ns() + a.slice_ns : 0;
   if (threadIdx.x == 0) {
     sh.args = a;
     sh.idle_since = 0;
     sh.polling = sh.busy = sh.idle_exit = sh.running = 0;
-    sh.polls = 0;
+    sh.polls = sh.asks = 0;
+    sh.halt = 0;
     sh.nodes = sh.jobs_done = 0;
     for (int k = 0; k < WCNT_COUNT; k++) sh.total[k] = 0;
   }
@@ -236,15 +256,12 @@ __global__ void __launch_bounds__(WARP_MAX * 32, 1) warp_kernel(BatchArgs a) {
     w.m = sv->m[t & 15];
     w.all = sv->all[id.s];
     w.now = sv->now[id.s];
+    w.code = sv->code[id.s];
+    w.st = sv->st;
     w.trick = sv->trick;
     w.trump = sv->trump;
-    w.leader = sv->leader;
-    w.nplayed = sv->nplayed;
-    w.left = sv->left;
-    w.need = sv->need;
-    w.code = sv->code[id.s];
-    w.sp = sv->sp;
-    for (int k = t; k < w.sp * 4; k += 32) reinterpret_cast<uint4*>(sm.fr)[k] = reinterpret_cast<const uint4*>(stack)[k];
+    const int words = (int)(w.st & SW_OFF) / 16;
+    for (int k = t; k < words; k += 32) reinterpret_cast<uint4*>(sm.fr)[k] = reinterpret_cast<const uint4*>(stack)[k];
     if (t == 0) {
       sm.job = sv->job;
       sm.job.start_nodes = 0ull - (sm.job.nodes - sm.job.start_nodes);
@@ -261,7 +278,7 @@ __global__ void __launch_bounds__(WARP_MAX * 32, 1) warp_kernel(BatchArgs a) {
     for (int k = 0; k < WCNT_COUNT; k++) sm.job.total[k] = 0;
   }
   __syncwarp();
-  WarpEnv env;
+  WarpEnv<STREAM> env;
   env.sh = &sh;
   env.tt = a.tt + (lane << a.tt_log2);
   env.t_end = t_end;
@@ -284,15 +301,12 @@ __global__ void __launch_bounds__(WARP_MAX * 32, 1) warp_kernel(BatchArgs a) {
       sv->now[t] = (uint16_t)w.now;
       sv->code[t] = w.code;
     }
-    for (int k = t; k < w.sp * 4; k += 32) reinterpret_cast<uint4*>(stack)[k] = reinterpret_cast<const uint4*>(sm.fr)[k];
+    const int words = (int)(w.st & SW_OFF) / 16;
+    for (int k = t; k < words; k += 32) reinterpret_cast<uint4*>(stack)[k] = reinterpret_cast<const uint4*>(sm.fr)[k];
     if (t == 0) {
+      sv->st = w.st;
       sv->trick = w.trick;
-      sv->trump = (int8_t)w.trump;
-      sv->leader = (int8_t)w.leader;
-      sv->nplayed = (int8_t)w.nplayed;
-      sv->left = (int8_t)w.left;
-      sv->need = (int8_t)w.need;
-      sv->sp = (int8_t)w.sp;
+      sv->trump = w.trump;
       sv->job = sm.job;
     }
   }
