@@ -12,95 +12,40 @@ struct ddg_guide {
   float* adam_m = nullptr;
   float* adam_v = nullptr;
   float* grad = nullptr;
-  guide_nn::bf16 *w1 = nullptr, *w2 = nullptr, *w2t = nullptr, *w3 = nullptr, *w3t = nullptr;
-  // workspace for max_rows rows
-  guide_nn::bf16 *X = nullptr, *Xt = nullptr, *H1 = nullptr, *H1t = nullptr, *H2 = nullptr, *H2t = nullptr;
-  guide_nn::bf16 *dO = nullptr, *dOt = nullptr, *dZ1 = nullptr, *dZ1t = nullptr, *dZ2 = nullptr, *dZ2t = nullptr;
-  float *Z1 = nullptr, *Z2 = nullptr, *L = nullptr, *dW3full = nullptr;
-  float* acc = nullptr;  // loss, hits, rows
+  unsigned char* packed = nullptr;  // bf16 weights in the tensor cores' layout (guide_nn::PK_*)
+  // a training step's workspace for max_rows rows, [column][row]
+  guide_nn::bf16 *Xt = nullptr, *H1t = nullptr, *H2t = nullptr, *dOt = nullptr, *dZ1t = nullptr, *dZ2t = nullptr;
+  float *Z1t = nullptr, *Z2t = nullptr;
+  float* part = nullptr;  // weight-gradient parts: splits x 5 x 128 x 256
+  float* acc = nullptr;   // loss, hits, rows, and the error flag behind them
   int64_t* rows_buf = nullptr;
-  int* err = nullptr;
+  int* err = nullptr;  // = acc + 3
+  int sms = 0;
 };
 
 namespace guide_nn {
 
 static bool g_attr_done[64];
 
-static int set_gemm_attrs() {
+static int set_kernel_attrs() {
   int dev = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && g_attr_done[dev]) return DDG_OK;
-  CUDA_TRY(cudaFuncSetAttribute((const void*)gemm_tc<EPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)gemm_tc<EPI_BIAS_GELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)gemm_tc<EPI_BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)gemm_tc<EPI_GELU_BACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM));
+  CUDA_TRY(cudaFuncSetAttribute((const void*)mlp_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MLP_SMEM));
+  CUDA_TRY(cudaFuncSetAttribute((const void*)mlp_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MLP_SMEM));
+  CUDA_TRY(cudaFuncSetAttribute((const void*)gemm_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, DW_SMEM));
   if (dev >= 0 && dev < 64) g_attr_done[dev] = true;
   return DDG_OK;
 }
 
-// C = A . B^T with the fused epilogue; M % 128 == 0, N % 16 == 0, N <= 256, K % 64 == 0.
-template <int EPI>
-static int gemm(const GemmArgs& g, cudaStream_t st) {
-  if (g.M % TILE_M || g.N % 16 || g.N > 256 || g.N < 16 || g.K % KCHUNK || g.lda % 8 || g.ldb % 8)
-    return fail(DDG_E_ARG, "gemm shape %d x %d x %d", g.M, g.N, g.K);
-  gemm_tc<EPI><<<g.M / TILE_M, 128, GEMM_SMEM, st>>>(g);
+// Batch rows to a split of the weight gradients (a multiple of 128), at most 32 splits.
+static int dw_rows(int R) { return (R / DW_K + 31) / 32 * DW_K; }
+static int dw_splits(int R) { return (R + dw_rows(R) - 1) / dw_rows(R); }
+
+static int refresh_packed(ddg_guide* g, cudaStream_t st) {
+  pack_params<<<((int)N_PARAMS + 255) / 256, 256, 0, st>>>(g->master, g->packed);
   CUDA_TRY(cudaGetLastError());
   return DDG_OK;
-}
-
-static GemmArgs gargs(const bf16* A, int lda, const bf16* B, int ldb, int M, int N, int K, int* err) {
-  GemmArgs g;
-  memset(&g, 0, sizeof(g));
-  g.A = A;
-  g.lda = lda;
-  g.B = B;
-  g.ldb = ldb;
-  g.M = M;
-  g.N = N;
-  g.K = K;
-  g.err = err;
-  return g;
-}
-
-static int tr(const bf16* in, int ldi, int R, int C, bf16* out, int ldo, cudaStream_t st) {
-  dim3 grid((C + 31) / 32, (R + 31) / 32), block(32, 8);
-  transpose<<<grid, block, 0, st>>>(in, ldi, R, C, out, ldo);
-  CUDA_TRY(cudaGetLastError());
-  return DDG_OK;
-}
-
-static int refresh_bf16(ddg_guide* g, cudaStream_t st) {
-  const int t = 256;
-  to_bf16<<<(HID * IN_PAD + t - 1) / t, t, 0, st>>>(g->master + OFF_W1, HID, IN_PAD, g->w1, nullptr, 0);
-  to_bf16<<<(HID * HID + t - 1) / t, t, 0, st>>>(g->master + OFF_W2, HID, HID, g->w2, g->w2t, HID);
-  to_bf16<<<(OUT_PAD * HID + t - 1) / t, t, 0, st>>>(g->master + OFF_W3, OUT_PAD, HID, g->w3, g->w3t, DO_LD);
-  CUDA_TRY(cudaGetLastError());
-  return DDG_OK;
-}
-
-// Forward pass of rows 0..R-1 of X (R % 128 == 0): Z1/H1, Z2/H2, logits L.
-static int forward(ddg_guide* g, int R, cudaStream_t st) {
-  GemmArgs a = gargs(g->X, IN_PAD, g->w1, IN_PAD, R, HID, IN_PAD, g->err);
-  a.C = g->Z1;
-  a.ldc = HID;
-  a.bias = g->master + OFF_B1;
-  a.H = g->H1;
-  a.ldh = HID;
-  int rc = gemm<EPI_BIAS_GELU>(a, st);
-  if (rc) return rc;
-  GemmArgs b = gargs(g->H1, HID, g->w2, HID, R, HID, HID, g->err);
-  b.C = g->Z2;
-  b.ldc = HID;
-  b.bias = g->master + OFF_B2;
-  b.H = g->H2;
-  b.ldh = HID;
-  rc = gemm<EPI_BIAS_GELU>(b, st);
-  if (rc) return rc;
-  GemmArgs c = gargs(g->H2, HID, g->w3, HID, R, OUT_PAD, HID, g->err);
-  c.C = g->L;
-  c.ldc = OUT_PAD;
-  c.bias = g->master + OFF_B3;
-  return gemm<EPI_BIAS>(c, st);
 }
 
 static int check_err(ddg_guide* g) {
@@ -119,9 +64,8 @@ int64_t ddg_guide_param_count(void) { return guide_nn::N_PARAMS; }
 void ddg_guide_destroy(ddg_guide* g) {
   if (!g) return;
   cudaSetDevice(g->device);
-  void* bufs[] = {g->master, g->adam_m, g->adam_v, g->grad, g->w1, g->w2, g->w2t, g->w3, g->w3t, g->X, g->Xt,
-                  g->H1, g->H1t, g->H2, g->H2t, g->dO, g->dOt, g->dZ1, g->dZ1t, g->dZ2, g->dZ2t, g->Z1, g->Z2,
-                  g->L, g->dW3full, g->acc, g->rows_buf, g->err};
+  void* bufs[] = {g->master, g->adam_m, g->adam_v, g->grad, g->packed, g->Xt, g->H1t, g->H2t, g->dOt, g->dZ1t, g->dZ2t,
+                  g->Z1t, g->Z2t, g->part, g->acc, g->rows_buf};
   for (void* b : bufs) cudaFree(b);
   delete g;
 }
@@ -133,7 +77,7 @@ int ddg_guide_create(int device, int max_rows, const float* params, ddg_guide** 
   if (max_rows <= 0 || max_rows % TILE_M || max_rows > (1 << 20))
     return fail(DDG_E_ARG, "max_rows %d is not a positive multiple of 128 (<= 1M)", max_rows);
   CUDA_TRY(cudaSetDevice(device));
-  int rc = set_gemm_attrs();
+  int rc = set_kernel_attrs();
   if (rc) return rc;
   ddg_guide* g = new ddg_guide();
   g->device = device;
@@ -148,37 +92,28 @@ int ddg_guide_create(int device, int max_rows, const float* params, ddg_guide** 
   A((void**)&g->adam_m, P * 4);
   A((void**)&g->adam_v, P * 4);
   A((void**)&g->grad, P * 4);
-  A((void**)&g->w1, (size_t)HID * IN_PAD * 2);
-  A((void**)&g->w2, (size_t)HID * HID * 2);
-  A((void**)&g->w2t, (size_t)HID * HID * 2);
-  A((void**)&g->w3, (size_t)OUT_PAD * HID * 2);
-  A((void**)&g->w3t, (size_t)HID * DO_LD * 2);
-  A((void**)&g->X, R * IN_PAD * 2);
+  A((void**)&g->packed, PK_BYTES);
   A((void**)&g->Xt, R * IN_PAD * 2);
-  A((void**)&g->H1, R * HID * 2);
   A((void**)&g->H1t, R * HID * 2);
-  A((void**)&g->H2, R * HID * 2);
   A((void**)&g->H2t, R * HID * 2);
-  A((void**)&g->dO, R * DO_LD * 2);
   A((void**)&g->dOt, R * DO_LD * 2);
-  A((void**)&g->dZ1, R * HID * 2);
   A((void**)&g->dZ1t, R * HID * 2);
-  A((void**)&g->dZ2, R * HID * 2);
   A((void**)&g->dZ2t, R * HID * 2);
-  A((void**)&g->Z1, R * HID * 4);
-  A((void**)&g->Z2, R * HID * 4);
-  A((void**)&g->L, R * OUT_PAD * 4);
-  A((void**)&g->dW3full, (size_t)DO_LD * HID * 4);
+  A((void**)&g->Z1t, R * HID * 4);
+  A((void**)&g->Z2t, R * HID * 4);
+  // (the splits of any step's rows: at most 32, and a step of fewer rows may have more than the largest)
+  A((void**)&g->part, (size_t)std::min(32, max_rows / DW_K) * DW_TILES * TILE_M * HID * 4);
   A((void**)&g->acc, 4 * 4);
   A((void**)&g->rows_buf, R * 8);
-  A((void**)&g->err, 4);
+  g->err = reinterpret_cast<int*>(g->acc + 3);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess && params) e = cudaMemcpy(g->master, params, P * 4, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     ddg_guide_destroy(g);
     return fail(e == cudaErrorMemoryAllocation ? DDG_E_MEMORY : DDG_E_CUDA, "guide buffers: %s",
                 cudaGetErrorString(e));
   }
-  rc = refresh_bf16(g, nullptr);
+  rc = refresh_packed(g, nullptr);
   if (rc == DDG_OK && cudaDeviceSynchronize() != cudaSuccess) rc = fail(DDG_E_CUDA, "guide init");
   if (rc) {
     ddg_guide_destroy(g);
@@ -199,7 +134,7 @@ int ddg_guide_set_params(ddg_guide* g, const float* params) {
   if (!g || !params) return fail(DDG_E_ARG, "null argument");
   CUDA_TRY(cudaSetDevice(g->device));
   CUDA_TRY(cudaMemcpy(g->master, params, guide_nn::N_PARAMS * 4, cudaMemcpyHostToDevice));
-  int rc = guide_nn::refresh_bf16(g, nullptr);
+  int rc = guide_nn::refresh_packed(g, nullptr);
   if (rc) return rc;
   CUDA_TRY(cudaDeviceSynchronize());
   return DDG_OK;
@@ -216,59 +151,42 @@ int ddg_guide_train_step(ddg_guide* g, const uint64_t* d_hands, const uint8_t* d
   for (int i = 0; i < n_rows; i++) rows[i] = rows_host[i];
   cudaStream_t st = nullptr;
   CUDA_TRY(cudaMemcpy(g->rows_buf, rows.data(), (size_t)R * 8, cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemsetAsync(g->acc, 0, 16, st));
-  CUDA_TRY(cudaMemsetAsync(g->err, 0, 4, st));
-  features<<<R, 64, 0, st>>>(d_hands, g->rows_buf, R, g->X);
-  int rc = forward(g, R, st);
-  if (rc) return rc;
-  loss_grad<<<(R + 127) / 128, 128, 0, st>>>(g->L, d_hands, d_tricks20, d_best20, g->rows_buf, R, g->dO, g->acc);
-  // Backward. Weight gradients: dW = dYᵀ . X as products over the batch (K = R).
-  if ((rc = tr(g->dO, DO_LD, R, DO_LD, g->dOt, R, st)) || (rc = tr(g->H2, HID, R, HID, g->H2t, R, st)) ||
-      (rc = tr(g->H1, HID, R, HID, g->H1t, R, st)) || (rc = tr(g->X, IN_PAD, R, IN_PAD, g->Xt, R, st)))
-    return rc;
-  GemmArgs w3 = gargs(g->dOt, R, g->H2t, R, DO_LD, HID, R, g->err);
-  w3.C = g->dW3full;
-  w3.ldc = HID;
-  if ((rc = gemm<EPI_STORE>(w3, st))) return rc;
-  CUDA_TRY(cudaMemcpyAsync(g->grad + OFF_W3, g->dW3full, (size_t)OUT_PAD * HID * 4, cudaMemcpyDeviceToDevice, st));
-  colsum<<<1, 128, 0, st>>>(g->dO, DO_LD, R, OUT_PAD, g->grad + OFF_B3);
-  GemmArgs h2 = gargs(g->dO, DO_LD, g->w3t, DO_LD, R, HID, DO_LD, g->err);  // dH2 = dO . W3
-  h2.H = g->dZ2;
-  h2.ldh = HID;
-  h2.Z = g->Z2;
-  h2.ldz = HID;
-  if ((rc = gemm<EPI_GELU_BACK>(h2, st))) return rc;
-  if ((rc = tr(g->dZ2, HID, R, HID, g->dZ2t, R, st))) return rc;
-  GemmArgs w2 = gargs(g->dZ2t, R, g->H1t, R, HID, HID, R, g->err);
-  w2.C = g->grad + OFF_W2;
-  w2.ldc = HID;
-  if ((rc = gemm<EPI_STORE>(w2, st))) return rc;
-  colsum<<<2, 128, 0, st>>>(g->dZ2, HID, R, HID, g->grad + OFF_B2);
-  GemmArgs h1 = gargs(g->dZ2, HID, g->w2t, HID, R, HID, HID, g->err);  // dH1 = dZ2 . W2
-  h1.H = g->dZ1;
-  h1.ldh = HID;
-  h1.Z = g->Z1;
-  h1.ldz = HID;
-  if ((rc = gemm<EPI_GELU_BACK>(h1, st))) return rc;
-  if ((rc = tr(g->dZ1, HID, R, HID, g->dZ1t, R, st))) return rc;
-  GemmArgs w1 = gargs(g->dZ1t, R, g->Xt, R, HID, IN_PAD, R, g->err);
-  w1.C = g->grad + OFF_W1;
-  w1.ldc = IN_PAD;
-  if ((rc = gemm<EPI_STORE>(w1, st))) return rc;
-  colsum<<<2, 128, 0, st>>>(g->dZ1, HID, R, HID, g->grad + OFF_B1);
+  CUDA_TRY(cudaMemsetAsync(g->acc, 0, 16, st));  // the sums and the error flag
+  MlpArgs a;
+  memset(&a, 0, sizeof(a));
+  a.hands = d_hands;
+  a.rows = g->rows_buf;
+  a.n = a.R = R;
+  a.tiles = R / TILE_M;
+  a.packed = g->packed;
+  a.master = g->master;
+  a.tricks20 = d_tricks20;
+  a.best20 = d_best20;
+  a.Xt = g->Xt;
+  a.H1t = g->H1t;
+  a.H2t = g->H2t;
+  a.dOt = g->dOt;
+  a.dZ2t = g->dZ2t;
+  a.dZ1t = g->dZ1t;
+  a.Z1t = g->Z1t;
+  a.Z2t = g->Z2t;
+  a.acc = g->acc;
+  a.err = g->err;
+  mlp_rows<true><<<std::min(a.tiles, g->sms), MLP_THREADS, MLP_SMEM, st>>>(a);
+  const DwArgs dw = {g->dZ1t, g->Xt, g->dZ2t, g->H1t, g->dOt, g->H2t, R, dw_rows(R), g->part, g->err};
+  gemm_dw<<<dim3(DW_TILES, dw_splits(R)), DW_THREADS, DW_SMEM, st>>>(dw);
+  if (lr > 0) g->step++;
+  const FinishArgs f = {g->part, dw_splits(R), R, g->dZ1t, g->dZ2t, g->dOt, g->grad, g->master, g->adam_m, g->adam_v, g->packed,
+                        lr, 1.f - powf(0.9f, (float)g->step), 1.f - powf(0.999f, (float)g->step)};
+  dw_finish<<<FIN_BLOCKS, FIN_THREADS, 0, st>>>(f);
   CUDA_TRY(cudaGetLastError());
   if (grad_host) CUDA_TRY(cudaMemcpy(grad_host, g->grad, N_PARAMS * 4, cudaMemcpyDeviceToHost));
-  if (lr > 0) {
-    g->step++;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - powf(b1, (float)g->step), c2 = 1.f - powf(b2, (float)g->step);
-    adam<<<(N_PARAMS + 255) / 256, 256, 0, st>>>(g->master, g->adam_m, g->adam_v, g->grad, N_PARAMS, lr, b1, b2,
-                                                 1e-8f, c1, c2);
-    if ((rc = refresh_bf16(g, st))) return rc;
-  }
-  CUDA_TRY(cudaDeviceSynchronize());
-  if ((rc = check_err(g))) return rc;
-  if (stats3) CUDA_TRY(cudaMemcpy(stats3, g->acc, 12, cudaMemcpyDeviceToHost));
+  float sums[4];  // waits for the step
+  CUDA_TRY(cudaMemcpy(sums, g->acc, 16, cudaMemcpyDeviceToHost));
+  int err = 0;
+  memcpy(&err, sums + 3, 4);
+  if (err) return fail(DDG_E_TIMEOUT, "guide: a tensor-core product did not complete (bounded wait)");
+  if (stats3) memcpy(stats3, sums, 12);
   return DDG_OK;
 }
 
@@ -292,17 +210,18 @@ static int guide_predict_on(ddg_guide* g, const uint64_t* d_hands, int64_t n, in
   using namespace guide_nn;
   CUDA_TRY(cudaMemsetAsync(g->err, 0, 4, stream));
   const int64_t total = n * 20;
-  for (int64_t first = 0; first < total; first += g->max_rows) {
-    const int rows = (int)std::min<int64_t>(g->max_rows, total - first);
-    const int R = (rows + TILE_M - 1) / TILE_M * TILE_M;
-    std::vector<int64_t> idx(R, -1);
-    for (int i = 0; i < rows; i++) idx[i] = first + i;
-    // from pageable memory: the call returns once the rows are staged, so idx may go
-    CUDA_TRY(cudaMemcpyAsync(g->rows_buf, idx.data(), (size_t)R * 8, cudaMemcpyHostToDevice, stream));
-    features<<<R, 64, 0, stream>>>(d_hands, g->rows_buf, R, g->X);
-    int rc = forward(g, R, stream);
-    if (rc) return rc;
-    predict_out<<<(rows + 127) / 128, 128, 0, stream>>>(g->L, d_hands, first, rows, d_seed20, d_hint20);
+  if (total > 0) {
+    MlpArgs a;
+    memset(&a, 0, sizeof(a));
+    a.hands = d_hands;
+    a.n = total;
+    a.tiles = (int)((total + TILE_M - 1) / TILE_M);
+    a.packed = g->packed;
+    a.master = g->master;
+    a.seed20 = d_seed20;
+    a.hint20 = d_hint20;
+    a.err = g->err;
+    mlp_rows<false><<<std::min(a.tiles, g->sms), MLP_THREADS, MLP_SMEM, stream>>>(a);
     CUDA_TRY(cudaGetLastError());
   }
   if (stream) {
