@@ -59,6 +59,7 @@ struct ddg_solver {
   uint8_t* d_out = nullptr;
   int8_t* d_seeds = nullptr;
   int64_t cap = 0;
+  unsigned char* h_io = nullptr;  // pinned staging of the host-memory calls on few deals (HostIo)
   uint64_t total_nodes = 0;  // search nodes over all calls
   uint64_t* d_job_end_ns = nullptr;  // caller's buffer for job completion times, or null
   uint64_t* d_job_start_ns = nullptr;  // caller's buffer for the times jobs were taken, or null
@@ -76,6 +77,18 @@ struct ddg_solver {
   const void* graph_key[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   int64_t graph_n = -1;
   int graph_grid = 0, graph_block = 0;
+};
+
+// Pinned staging for a host-memory call on at most IO_DEALS deals: its copies and its launch
+// are queued together and waited for once. Pageable copies wait one by one, some 10 us each
+// (the call for one lead of a five-card ending: 173 us with four waits). Larger calls copy
+// straight from and to the caller's memory.
+enum { IO_DEALS = 1024 };
+struct HostIo {
+  unsigned long long counters[CNT_WORDS];
+  uint64_t hands[IO_DEALS * 4];
+  int8_t seeds[IO_DEALS * 20];
+  uint8_t out[IO_DEALS * 20];
 };
 
 extern "C" {
@@ -178,6 +191,7 @@ void ddg_solver_destroy(ddg_solver* s) {
   cudaFree(s->d_out);
   cudaFree(s->d_seeds);
   if (s->h_stop) cudaFreeHost(s->h_stop);
+  if (s->h_io) cudaFreeHost(s->h_io);
   if (s->ev0) cudaEventDestroy(s->ev0);
   if (s->ev1) cudaEventDestroy(s->ev1);
   delete s;
@@ -388,8 +402,12 @@ static BatchArgs make_args(ddg_solver* s, const uint64_t* d_hands, int64_t n, co
 }
 
 // Counters of the last launch into `st` (and the solver's node total). Returns the words.
+static int take_stats(ddg_solver* s, int grid, int block, ddg_stats* st, const unsigned long long* c);
 static int read_stats(ddg_solver* s, int grid, int block, ddg_stats* st, unsigned long long* c) {
   CUDA_TRY(cudaMemcpy(c, s->counters, CNT_WORDS * 8, cudaMemcpyDeviceToHost));
+  return take_stats(s, grid, block, st, c);
+}
+static int take_stats(ddg_solver* s, int grid, int block, ddg_stats* st, const unsigned long long* c) {
   s->total_nodes += c[CNT_NODES];
   if (c[CNT_FAULTS])
     return fail(DDG_E_TIMEOUT, "%llu blocks gave up a bounded queue wait; results incomplete", c[CNT_FAULTS]);
@@ -921,6 +939,58 @@ static int ensure_staging(ddg_solver* s, int64_t n) {
   return DDG_OK;
 }
 
+// One host-memory call: deals (and seeds) to the device, the solve `a` describes (its buffers
+// are the staging ones, filled in here), tables and counters back.
+static int staged_solve(ddg_solver* s, const uint64_t* hands, int64_t n, const int8_t* seeds, BatchArgs a, uint8_t* out20,
+                        ddg_stats* st) {
+  const bool few = n <= IO_DEALS;
+  if (few && !s->h_io) CUDA_TRY(cudaHostAlloc((void**)&s->h_io, sizeof(HostIo), cudaHostAllocDefault));
+  HostIo* io = reinterpret_cast<HostIo*>(s->h_io);
+  if (few) {
+    memcpy(io->hands, hands, (size_t)n * 32);
+    CUDA_TRY(cudaMemcpyAsync(s->d_hands, io->hands, (size_t)n * 32, cudaMemcpyHostToDevice, nullptr));
+    if (seeds) {
+      memcpy(io->seeds, seeds, (size_t)n * 20);
+      CUDA_TRY(cudaMemcpyAsync(s->d_seeds, io->seeds, (size_t)n * 20, cudaMemcpyHostToDevice, nullptr));
+    }
+  } else {
+    CUDA_TRY(cudaMemcpy(s->d_hands, hands, (size_t)n * 32, cudaMemcpyHostToDevice));
+    if (seeds) CUDA_TRY(cudaMemcpy(s->d_seeds, seeds, (size_t)n * 20, cudaMemcpyHostToDevice));
+  }
+  s->sliced = false;  // a plain solve ends any resumable one
+  CUDA_TRY(cudaMemsetAsync(s->counters, 0, CNT_WORDS * 8, nullptr));
+  CUDA_TRY(cudaMemsetAsync(s->d_out, 0xFF, (size_t)n * 20, nullptr));
+  if (s->tasks) CUDA_TRY(cudaMemsetAsync(s->tasks, 0, s->tasks_bytes, nullptr));
+  if (a.job_end_ns) CUDA_TRY(cudaMemsetAsync(a.job_end_ns, 0, (size_t)a.n_jobs * 8, nullptr));
+  if (a.job_start_ns) CUDA_TRY(cudaMemsetAsync(a.job_start_ns, 0, (size_t)a.n_jobs * 8, nullptr));
+  *(volatile int*)s->h_stop = 0;
+  CUDA_TRY(cudaEventRecord(s->ev0, nullptr));
+  int grid = 0, block = 0;
+  int rc = launch_batch(s, a, nullptr, s->sms, &grid, &block);
+  if (rc) return rc;
+  CUDA_TRY(cudaEventRecord(s->ev1, nullptr));
+  if (few) {
+    CUDA_TRY(cudaMemcpyAsync(io->out, s->d_out, (size_t)n * 20, cudaMemcpyDeviceToHost, nullptr));
+    CUDA_TRY(cudaMemcpyAsync(io->counters, s->counters, sizeof(io->counters), cudaMemcpyDeviceToHost, nullptr));
+  }
+  if (!few || s->cfg.time_limit_s > 0) {
+    rc = wait_launch(s);
+    if (rc) return rc;
+  }
+  if (!few) {
+    unsigned long long c[CNT_WORDS];
+    rc = read_stats(s, grid, block, st, c);
+    if (rc) return rc;
+    CUDA_TRY(cudaMemcpy(out20, s->d_out, (size_t)n * 20, cudaMemcpyDeviceToHost));
+    return DDG_OK;
+  }
+  CUDA_TRY(cudaStreamSynchronize(nullptr));
+  rc = take_stats(s, grid, block, st, io->counters);
+  if (rc) return rc;
+  memcpy(out20, io->out, (size_t)n * 20);
+  return DDG_OK;
+}
+
 static int solve_host(ddg_solver* s, const uint64_t* hands, int64_t n, const int8_t* seeds,
                       uint8_t* out20, ddg_stats* st) {
   if (!s) return fail(DDG_E_ARG, "null solver");
@@ -931,15 +1001,12 @@ static int solve_host(ddg_solver* s, const uint64_t* hands, int64_t n, const int
     int rc = ddg_check_deal(hands + i * 4);
     if (rc) return fail(rc, "deal %lld: %s", (long long)i, g_err);
   }
+  if (s->streaming) return fail(DDG_E_STATE, "a stream is open on this solver");
   CUDA_TRY(cudaSetDevice(s->device));
   int rc = ensure_staging(s, n);
   if (rc) return rc;
-  CUDA_TRY(cudaMemcpy(s->d_hands, hands, (size_t)n * 32, cudaMemcpyHostToDevice));
-  if (seeds) CUDA_TRY(cudaMemcpy(s->d_seeds, seeds, (size_t)n * 20, cudaMemcpyHostToDevice));
-  rc = ddg_solve_device(s, s->d_hands, n, seeds ? s->d_seeds : nullptr, s->d_out, nullptr, nullptr, st);
-  if (rc) return rc;
-  CUDA_TRY(cudaMemcpy(out20, s->d_out, (size_t)n * 20, cudaMemcpyDeviceToHost));
-  return DDG_OK;
+  return staged_solve(s, hands, n, seeds, make_args(s, s->d_hands, n, seeds ? s->d_seeds : nullptr, s->d_out, nullptr),
+                      out20, st);
 }
 
 int ddg_solve_batch(ddg_solver* s, const uint64_t* hands, int64_t n, uint8_t* out20, ddg_stats* st) {
@@ -966,31 +1033,13 @@ static int solve_one(ddg_solver* s, const uint64_t* hands4, int strain, int decl
   CUDA_TRY(cudaSetDevice(s->device));
   rc = ensure_staging(s, 1);
   if (rc) return rc;
-  s->sliced = false;
-  CUDA_TRY(cudaMemcpy(s->d_hands, hands4, 32, cudaMemcpyHostToDevice));
-  if (seeds20) CUDA_TRY(cudaMemcpy(s->d_seeds, seeds20, 20, cudaMemcpyHostToDevice));
   BatchArgs a = make_args(s, s->d_hands, 1, seeds20 ? s->d_seeds : nullptr, s->d_out, nullptr);
   a.n_jobs = 1;
   a.one_job = 1;
   a.one_strain = strain;
   a.one_decl = decl;
   a.first_target = first_target;
-  CUDA_TRY(cudaMemset(s->counters, 0, CNT_WORDS * 8));
-  CUDA_TRY(cudaMemset(s->d_out, 0xFF, 20));
-  if (s->tasks) CUDA_TRY(cudaMemset(s->tasks, 0, s->tasks_bytes));
-  *(volatile int*)s->h_stop = 0;
-  CUDA_TRY(cudaEventRecord(s->ev0, nullptr));
-  int grid = 0, block = 0;
-  rc = launch_batch(s, a, nullptr, s->sms, &grid, &block);
-  if (rc) return rc;
-  CUDA_TRY(cudaEventRecord(s->ev1, nullptr));
-  rc = wait_launch(s);
-  if (rc) return rc;
-  unsigned long long c[CNT_WORDS];
-  rc = read_stats(s, grid, block, nullptr, c);
-  if (rc) return rc;
-  CUDA_TRY(cudaMemcpy(out20, s->d_out, 20, cudaMemcpyDeviceToHost));
-  return DDG_OK;
+  return staged_solve(s, hands4, 1, seeds20, a, out20, nullptr);
 }
 
 int ddg_solve_strain(ddg_solver* s, const uint64_t* hands4, int strain, const int* ns4, int* out4) {
