@@ -40,6 +40,8 @@ DDG_W void w_sync() { __syncwarp(); }
 DDG_W int w_top(u32 x) { return 31 - __clz((int)x); }   // highest set bit, -1 for 0
 DDG_W int w_low(u32 x) { return __ffs((int)x) - 1; }    // lowest set bit, -1 for 0
 DDG_W int w_popc(u32 x) { return __popc(x); }
+DDG_W u32 w_rev(u32 x) { return __brev(x); }
+DDG_W u32 w_shl_hi(u32 hi, u32 lo, int k) { return __funnelshift_l(lo, hi, k); }  // high word of hi:lo << k, k < 32
 #else  // the host emulation provides the collectives (warp_emu.hpp)
 #define DDG_W static inline
 DDG_W bool w_any(bool p) { return w_ballot(p) != 0; }
@@ -47,23 +49,36 @@ DDG_W u32 w_uni(u32 v) { return v; }
 DDG_W int w_top(u32 x) { return x ? 31 - __builtin_clz(x) : -1; }
 DDG_W int w_low(u32 x) { return x ? __builtin_ctz(x) : -1; }
 DDG_W int w_popc(u32 x) { return __builtin_popcount(x); }
+DDG_W u32 w_shl_hi(u32 hi, u32 lo, int k) { return (u32)(((u64)hi << 32 | lo) << k >> 32); }
+DDG_W u32 w_rev(u32 x) {
+  u32 r = 0;
+  for (int k = 0; k < 32; k++) r |= (x >> k & 1) << (31 - k);
+  return r;
+}
 #endif
 
-// One level of the search in shared memory: what taking its move back needs.
+// One level of the search in shared memory: what taking its move back needs, and its
+// candidates' keys, unordered: the next one is the greatest key below the last one's
+// (a key is unique), one reduction over the warp, so the list is never sorted.
 struct alignas(16) WarpFrame {
   struct {
-    u32 at;    // relevant cards gathered so far | cards tried << 16
-    u32 code;  // owner code before this frame's card was played
+    u32 at;     // relevant cards gathered so far | cards tried << 16
+    u32 code;   // the rest as it was before this frame's card was played: taking the card back
+    u32 cards;  // is loading them. In play at the start of the trick | in a hand << 16
+    u32 word;   // of suits 0, 1, 2: state word, w_open_info(), trick
   } suit[4];
-  u32 st, info, trick;  // state word and trick before this frame's card; w_open_info()
-  uint8_t mv[12];       // candidates 1.., best first (the first is played at once)
-  uint16_t all[4];      // a frame that completed a trick: the cards in play at its start
+  uint16_t m[16];     // cards of every (suit, seat)
+  uint16_t keys[16];  // (weight + KEY_BIAS) << 6 | card; 0: no candidate
 };
-static_assert(sizeof(WarpFrame) == 64, "a frame is two 32-byte halves");
+static_assert(sizeof(WarpFrame) == 128, "frames are copied as 16-byte words");
+enum { KEY_BIAS = 352 };  // the weights lie within -300 .. 140
 
-// The state word: leader:2 | -:1 | cards played to the trick * 8:2 | -:1 | frame offset
-// (depth * 64):6 | tricks left:4 | tricks NS still need:4.
-enum : u32 { SW_LEADER = 3, SW_CARD = 8, SW_NP8 = 0x18, SW_FRAME = 64, SW_OFF = 0xFC0, SW_LEFT = 1u << 12, SW_NEED = 1u << 16 };
+// The state word: leader:2 | -:1 | cards played to the trick * 8:2 | -:3 | offset of the
+// node's frame:13 | tricks left:4 | tricks NS still need:4.
+enum : u32 {
+  SW_LEADER = 3, SW_CARD = 8, SW_NP8 = 0x18, SW_FRAME = (u32)sizeof(WarpFrame) << 8, SW_OFF = 0x1FFF00, SW_LEFT = 1u << 21,
+  SW_NEED = 1u << 25
+};
 
 // Counters, one to a thread.
 enum { WCNT_PROBES = 0, WCNT_HITS = 1, WCNT_STORES = 2, WCNT_READS = 3, WCNT_BYTES = 4, WCNT_BOUNDS = 5, WCNT_COUNT = 6 };
@@ -79,7 +94,7 @@ struct WarpJob {
 
 struct WarpMem {
   WarpFrame fr[STACK_DEPTH];
-  uint8_t scratch[16];  // candidates before they are ordered
+  uint8_t scratch[16];  // candidates, handed to threads 0, 1, 2, ...
   WarpJob job;
 };
 
@@ -104,9 +119,13 @@ struct WarpState {
 DDG_W void w_unpack(WarpState& w) {
   w.leader = (int)(w.st & SW_LEADER);
   w.nplayed = (int)(w.st >> 3 & 3);
-  w.left = (int)(w.st >> 12 & 15);
-  w.need = (int)(w.st >> 16 & 15);
+  w.left = (int)(w.st >> 21 & 15);
+  w.need = (int)(w.st >> 25 & 15);
 }
+
+// Branch weights: what few nodes run is kept out of the line of what most run.
+#define W_RARE(x) (__builtin_expect(!!(x), 0))
+#define W_OFTEN(x) (__builtin_expect(!!(x), 1))
 
 struct WarpIds {  // what a thread stands for
   int t, s, p;
@@ -153,8 +172,8 @@ DDG_W u32 w_build_code(const WarpState& w, const WarpIds& id) {
   }
   return code << 1 << (31 - 2 * n);
 }
-// The owners of the highest n cards, lowest card in the low bits (n = 0: 0).
-DDG_W u32 w_pattern(u32 code, int n) { return (code >> 1) >> (31 - 2 * n); }
+// The owners of the highest n cards, lowest card in the low bits (n = 0: 0; at most 13).
+DDG_W u32 w_pattern(u32 code, int twice_n) { return w_shl_hi(0, code, twice_n); }
 
 // The top n cards of a suit.
 DDG_W u32 w_top_n(u32 all, int n) {
@@ -211,13 +230,16 @@ DDG_W int w_probe(WarpState& w, const WarpIds& id, const TTBucket* b, u32 tagw, 
     counts = e.w1 & 0xFFFFu;
     // Tag, bucket and q are the whole hash of the suit lengths, a bijection, so an entry
     // with this q has these lengths: its counts are no longer than the suits.
-    const int n0 = (int)(counts & 15), n1 = (int)(counts >> 4 & 15), n2 = (int)(counts >> 8 & 15);
-    u64 mine = w_pattern(codes[3], (int)(counts >> 12));
-    mine = mine << (2 * n2) | w_pattern(codes[2], n2);
-    mine = mine << (2 * n1) | w_pattern(codes[1], n1);
-    mine = mine << (2 * n0) | w_pattern(codes[0], n0);
-    same = ((e.q ^ k.q) | ((e.w0 ^ k.q_hi) & 0x7Fu) | ((u32)mine ^ (e.w1 >> 16 | e.own << 16)) |
-            ((u32)(mine >> 32) ^ (e.own >> 16 | (e.w0 >> 21 & 0x3FFu) << 16))) == 0;
+    const int b0 = (int)(counts << 1 & 30), b1 = (int)(counts >> 3 & 30), b2 = (int)(counts >> 7 & 30);
+    u32 lo = w_pattern(codes[3], (int)(counts >> 11 & 30)), hi = 0;
+    hi = w_shl_hi(hi, lo, b2);
+    lo = lo << b2 | w_pattern(codes[2], b2);
+    hi = w_shl_hi(hi, lo, b1);
+    lo = lo << b1 | w_pattern(codes[1], b1);
+    hi = w_shl_hi(hi, lo, b0);
+    lo = lo << b0 | w_pattern(codes[0], b0);
+    same = ((e.q ^ k.q) | ((e.w0 ^ k.q_hi) & 0x7Fu) | (lo ^ (e.w1 >> 16 | e.own << 16)) |
+            (hi ^ (e.own >> 16 | (e.w0 >> 21 & 0x3FFu) << 16))) == 0;
     const int lb = (int)(e.w0 >> 7 & 15), ub = (int)(e.w0 >> 11 & 15);
     best = (int)(e.w0 >> 15 & 63);
     holds = lb >= need;
@@ -234,7 +256,7 @@ DDG_W int w_probe(WarpState& w, const WarpIds& id, const TTBucket* b, u32 tagw, 
     w_count(w, id, WCNT_HITS, 1);
     return (int)((up >> at) & 1);
   }
-  if (hints) hint = (int)w_shfl((u32)best, w_top(hints));
+  if (W_RARE(hints)) hint = (int)w_shfl((u32)best, w_top(hints));
   return -1;
 }
 
@@ -248,7 +270,7 @@ DDG_W void w_store(WarpState& w, const WarpIds& id, TTBucket* b, u32 tagw, const
   const int n0 = (int)(counts & 15), n1 = (int)(counts >> 4 & 15), n2 = (int)(counts >> 8 & 15);
   if (n0 + n1 + n2 + (int)(counts >> 12) > MAX_REL) return;
   const int off = (id.s > 0 ? n0 : 0) + (id.s > 1 ? n1 : 0) + (id.s > 2 ? n2 : 0);
-  const u64 mine = (u64)w_pattern(code, above) << (2 * off);
+  const u64 mine = (u64)w_pattern(code, 2 * above) << (2 * off);
   const u32 own_lo = w_or((u32)mine), own_hi = w_or((u32)(mine >> 32));
   WarpEntry e = {k.q, k.q_hi | own_hi >> 16 << 21, counts | own_lo << 16, own_lo >> 16 | own_hi << 16};
   const bool match = id.t < TT_WAYS && (tagw & ~0xF00u) == k.tag;
@@ -416,10 +438,16 @@ DDG_W bool w_quick_possible(const WarpState& w, const WarpIds& id, const WarpTop
   // two top cards, or the third behind the left hand's second
   const bool two = (!(sec & 1) && sec != REL_NONE) || (sec == REL_L && rt_thr(top.a) == REL_P);
   const bool lone = (lho | rho) == 0 && longest != 0;
-  const int bound = lone || (most <= 1 && other <= 1) ? longest : !two ? 1 : most <= 2 ? longest : 2;
+  // Side suits run on only when the opponents' trumps are gone: the leader draws two at most.
+  const u32 ta0 = w_shfl(top.a, w.trump & 3), ta = w.trump >= 0 ? ta0 : 0;
+  const int drawn = rt_win(ta) == 0 ? 2 : 0;
+  const bool clear = w.trump < 0 || id.s == w.trump || (rt_len(ta, REL_L) <= drawn && rt_len(ta, REL_R) <= drawn);
+  const bool third = sec == REL_L && rt_thr(top.a) == REL_P;
+  const int bound = !clear ? (lone ? 0 : third ? 2 : 1)
+                           : lone || (most <= 1 && other <= 1) ? longest : !two ? 1 : most <= 2 ? longest : 2;
   const u32 sum = w_add(id.t < 4 && (ours || lone) ? (u32)bound : 0u);
-  const bool no_trumps = w.trump < 0 || (w_shfl(top.a, w.trump & 3) & 0xFFFFu) == 0;
-  return (int)sum >= cutoff || w_any(lone && longest + 1 >= cutoff) || cutoff <= 1 || (cutoff_other <= 1 && no_trumps);
+  return (int)sum >= cutoff || w_any(lone && clear && longest + 1 >= cutoff) || cutoff <= 1 ||
+         (cutoff_other <= 1 && (ta & 0xFFFFu) == 0);
 }
 
 // QuickTricks (quick_tricks_impl): the leading side's sure tricks against `cutoff`;
@@ -543,6 +571,9 @@ DDG_W bool w_later_tricks(const WarpState& w, const WarpIds& id, const WarpTop& 
     if (theirs && others) wr = 1u << rt_rank(top.ranks, 0);
     return true;
   }
+  // With trumps about, all but one answer needs the bound within two tricks of an end.
+  const bool near = ns ? need >= w.left - 1 : need <= 2;
+  if (!near && (rt_len(ta, 0) | rt_len(ta, REL_P)) != 0) return false;
   const u32 tk = w_shfl(top.ranks, w.trump);
   const int win = rt_win(ta), sec = rt_sec(ta), thr = rt_thr(ta);
   const bool win_ours = win == 0 || win == REL_P;
@@ -593,6 +624,7 @@ DDG_W bool w_quick_2nd(const WarpState& w, const WarpIds& id, u32& wr) {
   const int hand = lho_of(w.leader), P = partner_of(hand), third = lho_of(hand);
   const int cutoff = ns_side(hand) ? w.need : w.left - w.need + 1;
   wr = 0;
+  if (trump >= 0 && cutoff > 1) return false;  // with trumps it counts this trick only
   const u32 me = w_shfl(w.m, 4 * hand + ls), pd = w_shfl(w.m, 4 * P + ls), th = w_shfl(w.m, 4 * third + ls);
   const u32 ranks = me | pd, bit = 1u << (lead & 15);
   const bool wins = ranks > (bit | th);
@@ -607,7 +639,6 @@ DDG_W bool w_quick_2nd(const WarpState& w, const WarpIds& id, u32& wr) {
   if (by_rank && !wins) return false;
   if (by_rank && id.s == ls) wr = 1u << w_top(ranks);
   if (1 >= cutoff) return true;
-  if (trump >= 0) return false;
   const int hh = me > pd ? hand : P;
   const u32 mine = w_shfl(w.m, 4 * hh + id.s);
   const int c1 = w_top(w.all);
@@ -635,19 +666,16 @@ DDG_W bool w_quick_2nd(const WarpState& w, const WarpIds& id, u32& wr) {
 
 // ---- move generation -----------------------------------------------------------------------
 
-// Cards of a holding that are the top of their run (run_tops for one suit).
+// Cards of a holding that are the top of their run (run_tops for one suit). With the highest
+// rank in the lowest bit, a run is a stretch of ones in (own or not in play); adding own
+// sends a carry from its first own card through the rest, which leaves there a zero at the
+// first own card and a one at every later one.
 DDG_W u32 w_run_tops(u32 own, u32 all) {
-  u32 open = ~(all & ~own) & 0x1FFFu;
-  u32 fill = own;
-  fill |= open & (fill >> 1);
-  open &= open >> 1;
-  fill |= open & (fill >> 2);
-  open &= open >> 2;
-  fill |= open & (fill >> 4);
-  open &= open >> 4;
-  fill |= open & (fill >> 8);
-  return own & ~(fill >> 1);
+  const u32 o = w_rev(own);
+  return w_rev(o & ~(w_rev(own | ~all) + o));
 }
+// Is the highest card of `cards` one of `mine`? (Sets compare like their highest cards.)
+DDG_W bool w_top_is(u32 cards, u32 mine) { return (cards & mine) > (cards & ~mine); }
 
 // The DDS lead weight (lead_weight) of `card` in this thread; top, hands and lengths of the
 // card's suit come from its threads.
@@ -670,8 +698,7 @@ DDG_W int w_lead_weight(const WarpState& w, const WarpTop& top, int card, int hi
     tt = (all & ~own & between) == 0;
   }
   const int r_rank = w_popc(all >> r);
-  const u32 below = all & (bit - 1);
-  const bool seq = below && (own >> w_top(below) & 1);
+  const bool seq = w_top_is(all & (bit - 1), own);  // the next card down is the leader's too
   const int lenL = rt_len(a, REL_L), lenR = rt_len(a, REL_R), lenP = rt_len(a, REL_P);
   const u32 cnt = (u32)((lenL == 0 ? w.left : lenL) + (lenR == 0 ? w.left : lenR)) << 2;
   const int w1 = rt_win(a), w2 = rt_sec(a), w3 = rt_thr(a);
@@ -720,16 +747,13 @@ DDG_W int w_lead_weight(const WarpState& w, const WarpTop& top, int card, int hi
   return delta + base + by + (tt ? 19 : 0);
 }
 
-DDG_W int w_hi(u32 m) { return w_top(m) + 2 - (m == 0); }  // DDS rank of the highest / lowest card, 0 = none
-DDG_W int w_lo(u32 m) { return m ? w_low(m) + 2 : 0; }
-
 // The DDS follow weights (follow_weight) of `card` in this thread; n = cards played. What
 // is the same for all candidates of a node is decided once (the branches); what differs
 // from card to card is chosen by selects, so the warp does not diverge.
 DDG_W int w_follow_weight(const WarpState& w, int n, int seat, bool is_void, int card) {
   const int lead = w.leader, trump = w.trump;
   const bool has_t = trump >= 0;
-  const int c0 = (int)(w.trick & 0xFF), ls = card_suit(c0), lead0 = rank2(c0);
+  const int c0 = (int)(w.trick & 0xFF), ls = card_suit(c0);
   const int s = card_suit(card), r = card & 15, rank = r + 2;
   const int P = partner_of(lead), R = rho_of(lead);
   const u32 hRL = w_shfl(w.m, 4 * R + ls), hRT0 = w_shfl(w.m, 4 * R + (trump & 3)), hRT = has_t ? hRT0 : 0;
@@ -738,32 +762,33 @@ DDG_W int w_follow_weight(const WarpState& w, int n, int seat, bool is_void, int
   const u32 bit = 1u << r, lead_bit = 1u << (c0 & 15);
   const int c1 = (int)(w.trick >> 8 & 0xFF), c2 = (int)(w.trick >> 16 & 0xFF);
   const int high1 = n > 1 && beats(c1, c0, trump) ? 1 : 0, move1 = high1 ? c1 : c0;
+  // Cards of one suit compare as their bits do, and a card with a hand's highest as its bit
+  // with the hand's set.
   if (!is_void) {  // the 2nd hand (the others' order: w_follow_floor)
     const u32 hPL = w_shfl(w.m, 4 * P + ls), hPT0 = w_shfl(w.m, 4 * P + (trump & 3)), hPT = has_t ? hPT0 : 0;
     const u32 hLL = w_shfl(w.m, 4 * lead + ls);
-    const int max3rd = w_hi(hPL), maxpd = w_hi(hRL), min3rd = w_lo(hPL), minpd = w_lo(hRL);
-    const u32 below = all & (bit - 1);
-    const bool seq = (below != 0) & (me >> (w_top(below) & 31) & 1);
-    const bool over = (rank > lead0) & (rank > max3rd), pd_over = maxpd > lead0 && maxpd > max3rd;
-    const bool under = (rank < min3rd) | (rank < minpd);
+    const bool seq = w_top_is(all & (bit - 1), me);
+    const bool over = bit > (hPL | lead_bit), pd_over = hRL > (hPL | lead_bit), above = bit > lead_bit;
+    const bool under3 = (hPL != 0) & ((hPL & (bit - 1)) == 0);  // below all of the third hand's
+    const bool under = under3 | ((hRL != 0) & ((hRL & (bit - 1)) == 0));
     int base;
     bool by_rank;  // weight = base - rank, else base + r_rank
     if (has_t) {
-      const bool side = ls != trump, pd_ruffs = maxpd == 0 && hRT;
-      const bool p_follows = max3rd != 0 || !hPT, pd_over_ruffs = hRT > hPT;
+      const bool side = ls != trump, pd_ruffs = !hRL && hRT;
+      const bool p_follows = hPL || !hPT, pd_over_ruffs = hRT > hPT;
       const bool u1 = !side || p_follows || (pd_ruffs && pd_over_ruffs), u2 = !side || p_follows;
       const bool u3 = side && pd_ruffs && (p_follows || pd_over_ruffs), u4 = side && pd_ruffs;
-      const bool lead_high = lead0 > maxpd && lead0 > max3rd;
-      const bool win = over ? u1 : pd_over ? u2 : (lead_high & (lead0 > rank)) ? u3 : u4;
-      const bool keep = maxpd > lead0 && hLL > hRL;
-      const int high = rank < maxpd ? 78 : rank > max3rd ? 73 : seq ? 62 : 49;
-      const int on_win = min3rd > rank ? 40 : keep ? 41 : rank > lead0 ? high : maxpd > 0 ? 47 : 40;
-      const int on_loss = under ? -9 : rank < lead0 ? -16 : seq ? 22 : 10;
+      const bool lead_high = lead_bit > (hPL | hRL);
+      const bool win = over ? u1 : pd_over ? u2 : lead_high & !above ? u3 : u4;
+      const bool keep = hRL > lead_bit && hLL > hRL;
+      const int high = bit < hRL ? 78 : bit > hPL ? 73 : seq ? 62 : 49;
+      const int on_win = under3 ? 40 : keep ? 41 : above ? high : hRL ? 47 : 40;
+      const int on_loss = under ? -9 : !above ? -16 : seq ? 22 : 10;
       base = win ? on_win : on_loss;
-      by_rank = win ? !((min3rd > rank) | keep) : !(under | (rank < lead0));
+      by_rank = win ? !(under3 | keep) : !(under | !above);
     } else {
-      base = pd_over ? 0 : over ? 81 : under ? -3 : rank < lead0 ? -11 : seq ? 10 : 13;
-      by_rank = pd_over | over | !(under | (rank < lead0) | seq);
+      base = pd_over ? 0 : over ? 81 : under ? -3 : !above ? -11 : seq ? 10 : 13;
+      by_rank = pd_over | over | !(under | !above | seq);
     }
     return base + (by_rank ? -rank : r_rank);
   }
@@ -797,15 +822,15 @@ DDG_W int w_follow_weight(const WarpState& w, int n, int seat, bool is_void, int
     K = K24;
     pen2 = pen1 = 4;
     if (has_t) {
-      const int max4th = w_hi(hRL), m1r = rank2(move1);
+      const int m1r = rank2(move1);
       const u32 hLL = w_shfl(w.m, 4 * lead + ls), allL = w_shfl(w.all, ls);
       // the second card of the led suit was the leader's at the trick's start
       const int l2 = w_top(allL & ~(1u << (w_top(allL) & 31)));
       const bool sec_lead = l2 >= 0 && ((hLL | lead_bit) >> (l2 & 31) & 1);
-      const bool covered = high1 == 0 && lead0 > max4th && (max4th != 0 || !hRT);
+      const bool covered = high1 == 0 && lead_bit > hRL && (hRL || !hRT);
       const int follows = high1 == 0 ? (sec_lead ? 36 : 48) : 72, ruffed = high1 == 0 ? -12 : 36;
       const bool ruffing = ruff & (ls != trump), under = (card_suit(move1) == trump) & (rank < m1r);
-      base = !ruffing ? 0 : covered ? -50 : under ? -32 : max4th != 0 ? follows : bit > hRT ? 48 : ruffed;
+      base = !ruffing ? 0 : covered ? -50 : under ? -32 : hRL ? follows : bit > hRT ? 48 : ruffed;
       K = ruffing ? (covered ? 0 : under ? K40 : K50) : K40;
       with_rank = ruffing & !covered & under;
       pen2 = pen1 = 0;
@@ -828,45 +853,30 @@ DDG_W int w_follow_weight(const WarpState& w, int n, int seat, bool is_void, int
   return base + (with_rank ? r_rank : -rank) + (int)(length * K >> 16) - (two ? pen2 : one ? pen1 : 0);
 }
 
-// Orders the candidates by weight (ties: highest card first, as insert_move keeps them)
-// into the frame; the thread of each one counts those ahead of it. Returns the first.
-DDG_W int w_order(const WarpIds& id, WarpFrame& f, u32 who, int card, int weight) {
-  const bool mine = who >> id.t & 1;
-  const u32 key = (u32)(weight + 1024) << 6 | (u32)card;
-  int ahead = 0;
-#pragma unroll 1
-  for (u32 rest = who; (rest = w_uni(rest)) != 0; rest &= rest - 1) ahead += w_shfl(key, w_low(rest)) > key;
-  if (mine && ahead) f.mv[ahead - 1] = (uint8_t)card;
-  return (int)w_shfl((u32)card, w_low(w_ballot(mine && ahead == 0)));
-}
-
-// The 3rd or 4th hand follows suit (`led`, its candidates of the led suit): the DDS weight is
-// up - rank for a card that wins and -rank for one that does not, with `up` above any rank
-// and "wins" a threshold, so the order is the winners from the lowest up, then the others
-// from the lowest up. Returns the threshold: the winners are the cards of at least that
-// rank (13: none).
-DDG_W int w_follow_floor(const WarpState& w, int n, int seat, u32 led) {
+// The 3rd or 4th hand follows suit: the DDS weight is up - rank for a card that wins and
+// -rank for one that does not, with `up` above any rank and "wins" a threshold, so the order
+// is the winners from the lowest up, then the others from the lowest up. Returns the set
+// that a winner's bit exceeds (all ones: no card wins).
+DDG_W u32 w_follow_floor(const WarpState& w, int n, int seat) {
   const int trump = w.trump, c0 = (int)(w.trick & 0xFF), c1 = (int)(w.trick >> 8 & 0xFF), ls = card_suit(c0);
   const bool high1 = beats(c1, c0, trump);
   const int move1 = high1 ? c1 : c0;
   const bool side = trump >= 0 && ls != trump;
+  const u32 none = 0xFFFFFFFFu;
   if (n == 3) {
     const int c2 = (int)(w.trick >> 16 & 0xFF);
     const bool h2 = beats(c2, move1, trump);
     const int move2 = h2 ? c2 : move1;
-    return (!h2 && high1) || (side && card_suit(move2) == trump) ? 13 : (move2 & 15) + 1;
+    return (!h2 && high1) || (side && card_suit(move2) == trump) ? none : 1u << (move2 & 15);
   }
-  const u32 fourth = w_shfl(w.m, 4 * rho_of(w.leader) + ls);
-  const int max4th = w_top(fourth), min4th = w_low(fourth), r1 = move1 & 15;  // -1: none
-  const int max3rd = w_top(w_shfl(w.m, 4 * seat + ls));
-  (void)led;
-  if (side && card_suit(move1) == trump) return 13;
-  if (side && high1 && max4th < 0) return r1 + 1;
-  if (!high1 && ((c0 & 15) > max4th || (side && max4th < 0))) return 13;
-  if (max3rd < min4th || max3rd < r1) return 13;
-  const int both = (max4th > r1 ? max4th : r1) + 1;
-  if (trump >= 0 && max3rd > max4th) return ls == trump || high1 ? both : max4th + 1;
-  return trump >= 0 && ls == trump ? 13 : both;
+  const u32 fourth = w_shfl(w.m, 4 * rho_of(w.leader) + ls), third = w_shfl(w.m, 4 * seat + ls);
+  const u32 b1 = 1u << (move1 & 15), lead_bit = 1u << (c0 & 15);
+  if (side && card_suit(move1) == trump) return none;
+  if (side && high1 && !fourth) return b1;
+  if (!high1 && (lead_bit > fourth || (side && !fourth))) return none;
+  if ((fourth && third < (fourth & (0u - fourth))) || third < b1) return none;
+  if (trump >= 0 && third > fourth) return ls == trump || high1 ? fourth | b1 : fourth;
+  return trump >= 0 && ls == trump ? none : fourth | b1;
 }
 
 // Hands the cards of `cm` ([sp], the threads of `seat`) to threads 0, 1, 2, ...: thread
@@ -884,16 +894,16 @@ DDG_W int w_compact(const WarpIds& id, WarpMem& sm, u32 cm, int seat, int& card)
   return n;
 }
 
-// The frame's info word: value when no child cuts:1 | seat:2 | candidates:4 | the one being
-// searched:4 | -:2 | its card:6 | win card:7 (64 = none; set when it completed a trick).
-DDG_W u32 w_open_info(int seat, int n) { return (u32)(!ns_side(seat)) | (u32)seat << 1 | (u32)n << 3; }
+// The frame's info word: value when no child cuts:1 | seat:2 | more than one candidate:1 | key
+// of the one being searched:15 | win card:7 (64 = none; set when it completed a trick).
+DDG_W u32 w_open_info(int seat, bool more) { return (u32)(!ns_side(seat)) | (u32)seat << 1 | (u32)more << 3; }
 DDG_W int wi_result(u32 info) { return (int)(info & 1); }
 DDG_W int wi_seat(u32 info) { return (int)(info >> 1) & 3; }
-DDG_W int wi_n(u32 info) { return (int)(info >> 3) & 15; }
-DDG_W int wi_i(u32 info) { return (int)(info >> 7) & 15; }
-DDG_W int wi_card(u32 info) { return (int)(info >> 13) & 63; }
+DDG_W bool wi_more(u32 info) { return info >> 3 & 1; }
+DDG_W u32 wi_key(u32 info) { return info >> 4 & 0x7FFFu; }
 DDG_W int wi_win_card(u32 info) { return (int)(info >> 19) & 127; }
-enum : u32 { WI_NEXT = 1u << 7, WI_KEEP = (1u << 11) - 1 };  // one candidate on; what a play leaves
+DDG_W int key_card(u32 key) { return (int)(key & 63); }
+enum : u32 { WI_KEEP = 15 };  // what a play leaves
 
 DDG_W u32 w_tags(const TTBucket* b, const WarpIds& id) { return b->tag[id.t & 15]; }
 
@@ -904,7 +914,7 @@ DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool& store, WarpTop
   w.rel = 0;
   if (w.need <= 0) return 1;
   if (w.left < w.need) return 0;
-  if (w.left == 1) {
+  if (W_RARE(w.left == 1)) {
     const u32 bt = w_ballot(id.s == w.trump && w.all != 0);
     const int su = bt ? w.trump : w_low(w_ballot(id.p == w.leader && w.m != 0)) & 3;
     const u32 in = w_shfl(w.all, su);
@@ -914,7 +924,7 @@ DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool& store, WarpTop
   const WarpKey k = w_key(w, id, env.mask());
   const TTBucket* b = env.table() + k.bucket;
   const int hit = w_probe(w, id, b, w_tags(b, id), k, w.code, w.need, hint);
-  if (hit >= 0) return hit;
+  if (W_OFTEN(hit >= 0)) return hit;
   top = w_make_top(w, id, k);
   const bool ns_lead = ns_side(w.leader);
   const int cut_ns = w.need, cut_ew = w.left - w.need + 1;
@@ -923,7 +933,7 @@ DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool& store, WarpTop
   int q = 0, v;
   const int cut = ns_lead ? cut_ns : cut_ew, cut_other = ns_lead ? cut_ew : cut_ns;
   decided = w_quick_possible(w, id, top, cut, cut_other);
-  if (decided) q = w_quick_tricks(w, id, top, cut, cut_other, wr, decided);
+  if (W_RARE(decided)) q = w_quick_tricks(w, id, top, cut, cut_other, wr, decided);
   if (decided) v = ns_lead ? q != 0 : q == 0;
   else if (w_later_tricks(w, id, top, wr)) v = !ns_lead;
   else return -1;
@@ -942,18 +952,17 @@ DDG_W void w_put(WarpState& w, const WarpIds& id, Env& env, int v, int best) {
 }
 
 DDG_W WarpFrame& w_frame(WarpMem& sm, u32 st) {
-  return *reinterpret_cast<WarpFrame*>(reinterpret_cast<char*>(sm.fr) + (st & SW_OFF));
+  return *reinterpret_cast<WarpFrame*>(reinterpret_cast<char*>(sm.fr) + (st >> 8 & 0x1FFF));
 }
 
 // A node expands (gen_moves_lead, gen_moves_follow): its candidates, one per run of alike
-// cards, ordered by the DDS weights into a fresh frame. Returns the first.
+// cards, with their DDS weights, into a fresh frame. Returns the first one's key.
 template <class Env>
-DDG_W int w_expand(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, const WarpTop& top, int hint) {
+DDG_W u32 w_expand(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, const WarpTop& top, int hint) {
   const int seat = (w.leader + w.nplayed) & 3, ls = (int)(w.trick >> 4) & 3;
   const u32 cm = w_run_tops(w.m, w.all);
   const u32 in_led = w_shfl(cm, 4 * seat + ls);
   const u32 led = w.nplayed ? in_led : 0;
-  WarpFrame& f = w_frame(sm, w.st);
   u32 who = led;  // the threads that stand for a candidate
   int n = w_popc(led), card = ls * 16 + (id.t & 15);  // following suit: thread r for rank r
   if (!led) {
@@ -961,28 +970,23 @@ DDG_W int w_expand(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, const
     who = (1u << n) - 1;
   }
   w.at = 0;
-  w.info = w_open_info(seat, n);
-  if (n == 1) {
-    return (int)w_shfl((u32)card, w_low(who));
-  }
-  if (led && w.nplayed > 1) {
-    const u32 win = led & (0xFFFFFFFFu << w_follow_floor(w, w.nplayed, seat, led)), lose = led & ~win;
-    const u32 below = (1u << id.t) - 1;
-    const int ahead = win >> id.t & 1 ? w_popc(win & below) : w_popc(win) + w_popc(lose & below);
-    if ((led >> id.t & 1) && ahead) f.mv[ahead - 1] = (uint8_t)card;
-    return ls * 16 + w_low(win ? win : led);
-  }
+  w.info = w_open_info(seat, n != 1);
+  if (n == 1) return 64 | w_shfl((u32)card, w_low(who));
   int weight;
-  if (w.nplayed == 0) {
+  if (W_RARE(w.nplayed == 0)) {
     if (hint < 0 && (w.st & SW_OFF) == 0) {  // the root, no TT move: an outside hint, when the leader holds it
       const int h = env.root_hint(sm.job);
       if (h >= 0 && h < 64 && (w_shfl(w.m, 4 * seat + (h >> 4)) >> (h & 15) & 1)) hint = h;
     }
     weight = w_lead_weight(w, top, card, hint);
+  } else if (led && w.nplayed > 1) {
+    weight = ((1u << (card & 15)) > w_follow_floor(w, w.nplayed, seat) ? 16 : 0) - (card & 15);
   } else {
     weight = w_follow_weight(w, w.nplayed, seat, !led, card);
   }
-  return w_order(id, f, who, card, weight);
+  const u32 key = who >> id.t & 1 ? (u32)(weight + KEY_BIAS) << 6 | (u32)card : 0;
+  if (id.t < 16) w_frame(sm, w.st).keys[id.t] = (uint16_t)key;
+  return w_max(key);
 }
 
 // ENTER inside a trick (enter_follow): the second hand's QuickTricks.
@@ -994,13 +998,14 @@ DDG_W int w_enter_follow(WarpState& w, const WarpIds& id) {
   return ns_side(lho_of(w.leader)) ? 1 : 0;
 }
 
-// Plays `card` from the top frame and pushes the frame (play): at the fourth card the
+// Plays the card of `key` from the top frame and pushes the frame (play): at the fourth card the
 // trick is settled and the frame keeps what taking it back needs.
-DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, int card) {
+DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, u32 key) {
   WarpFrame& f = w_frame(sm, w.st);
-  const int seat = wi_seat(w.info), su = card_suit(card), r = card & 15, np8 = (int)(w.st & SW_NP8);
-  const u32 bit = 1u << r, code = w.code, st = w.st, trick = w.trick;
-  u32 info = (w.info & WI_KEEP) | (u32)card << 13;
+  const int card = key_card(key), su = card_suit(card), r = card & 15, np8 = (int)(w.st & SW_NP8);
+  const u32 bit = 1u << r, code = w.code, st = w.st, trick = w.trick, cards = w.all | w.now << 16;
+  u32 info = (w.info & WI_KEEP) | key << 4;
+  if (id.t < 16) f.m[id.t] = (uint16_t)w.m;
   if (id.s == su) {
     // The card's owner leaves the code: the owners of the cards below move up.
     const u32 low = 0xFFFFFFFFu >> (2 * w_popc(w.now >> r) - 2);
@@ -1008,16 +1013,15 @@ DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, int card) {
     w.at |= bit << 16;
     w.now ^= bit;
   }
-  if ((id.t & 15) == seat * 4 + su) w.m ^= bit;
+  if ((id.t & 15) == wi_seat(w.info) * 4 + su) w.m ^= bit;
   w.trick |= (u32)card << np8;
   if (np8 == 24) {
     const int c = (int)(w.trick >> (8 * (id.t & 3))) & 0xFF, cs = card_suit(c);
-    const u32 key = (cs == w.trump ? 512u : cs == card_suit((int)(w.trick & 0xFF)) ? 256u : 0u) | (u32)c << 2 | (u32)(id.t & 3);
-    const u32 best = w_max(key);
+    const u32 rank = (cs == w.trump ? 512u : cs == card_suit((int)(w.trick & 0xFF)) ? 256u : 0u) | (u32)c << 2 | (u32)(id.t & 3);
+    const u32 best = w_max(rank);
     const int wc = (int)(best >> 2) & 63, leader = (int)((st + best) & 3);
     const int same = w_popc(w_ballot(cs == card_suit(wc)) & 15);  // at least two: won by rank
     info |= (u32)(same >= 2 ? wc : 64) << 19;
-    if (id.t < 4) f.all[id.t] = (uint16_t)w.all;
     w.all = w.now;
     w.trick = 0;
     w.st = ((st & ~(SW_LEADER | SW_NP8)) | (u32)leader) + SW_FRAME - SW_LEFT - (ns_side(leader) ? SW_NEED : 0);
@@ -1027,11 +1031,8 @@ DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, int card) {
   if (id.t < 4) {
     f.suit[id.t].at = w.at;
     f.suit[id.t].code = code;
-  }
-  if (id.t == 4) {
-    f.st = st;
-    f.info = info;
-    f.trick = trick;
+    f.suit[id.t].cards = cards;
+    f.suit[id.t].word = id.t == 0 ? st : id.t == 1 ? info : trick;
   }
   w_sync();
 }
@@ -1040,39 +1041,35 @@ DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, int card) {
 DDG_W int w_unplay(WarpState& w, const WarpIds& id, WarpMem& sm) {
   const bool completed = (w.st & SW_NP8) == 0;  // this ply completed a trick
   const WarpFrame& f = w_frame(sm, w.st - SW_FRAME);
-  w.st = f.st;
-  w.info = f.info;
-  w.trick = f.trick;
+  w.st = f.suit[0].word;
+  w.info = f.suit[1].word;
+  w.trick = f.suit[2].word;
   w.at = f.suit[id.s].at;
   w.code = f.suit[id.s].code;
+  const u32 cards = f.suit[id.s].cards;
+  w.all = cards & 0xFFFFu;
+  w.now = cards >> 16;
+  w.m = f.m[id.t & 15];
   w_unpack(w);
-  const int card = wi_card(w.info), su = card_suit(card);
   if (completed) {
-    w.all = f.all[id.s];
     const int wc = wi_win_card(w.info);
     if (id.s == card_suit(wc)) w.rel |= 1u << (wc & 15);  // (none: suit 4)
   }
-  const u32 bit = 1u << (card & 15);
-  if (id.s == su) w.now ^= bit;
-  if ((id.t & 15) == wi_seat(w.info) * 4 + su) w.m ^= bit;
-  return card;
+  return key_card(wi_key(w.info));
 }
 
-// The frame's next candidate that is not a small card like one tried before (step_next):
-// every candidate is tested by its thread. -1: none left.
-DDG_W int w_next(WarpState& w, const WarpIds& id, WarpMem& sm) {
-  const int n = wi_n(w.info), i = wi_i(w.info);
-  if (i >= n) return -1;
-  const int c = w_frame(sm, w.st).mv[(id.t - 1) & 15];  // (the first one is not asked for again)
+// The frame's next candidate (step_next): of those behind the last one, the first that is
+// not a small card like one tried before; every candidate is tested by its thread. Returns
+// its key, 0 when none is left.
+DDG_W u32 w_next(WarpState& w, const WarpIds& id, WarpMem& sm) {
+  if (!wi_more(w.info)) return 0;
+  const u32 key = w_frame(sm, w.st).keys[id.t & 15];
+  const int c = key_card(key);
   const u32 at = w_shfl(w.at, card_suit(c));
   const u32 acc = at & 0xFFFFu, tried = at >> 16, bit = 1u << (c & 15);
   const u32 small = (acc & (0u - acc)) - 1;  // below the lowest relevant card (all, when there is none)
   const bool skip = (small & bit) != 0 && (small & tried) != 0;
-  const u32 open = w_ballot(id.t < n && !skip) >> i << i;
-  if (!open) return -1;
-  const int next = w_low(open);
-  w.info = (w.info & ~(15u << 7)) | (u32)next << 7;
-  return (int)w_shfl((u32)c, next);
+  return w_max(key < wi_key(w.info) && !skip ? key : 0);
 }
 
 // The top frame is done (finish): the relevant cards widen through runs of the hand's own
@@ -1180,7 +1177,7 @@ DDG_W bool w_end_root(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, in
 // start with a job, ST_ENTER to go on inside one (w and the frames as they were saved); on
 // return ST_IDLE (nothing left), ST_TAKE or ST_ENTER (stopped). An Env offers
 //   bool take(w, id, sm)   the next job: position, job record (else stage is set)
-//   bool stop(w, id, sm)   asked every 256 nodes: true ends the warp
+//   bool stop(w, id, sm)   asked at a trick start after 256 nodes or more: true ends the warp
 //   int seed(job), root_hint(job); void answer(job, ns), root_best(job, card), job_done(sm)
 //   TTBucket* table(); u32 mask()
 template <class Env>
@@ -1191,7 +1188,6 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
       if (!w_any(env.take(w, id, sm))) return;
       WarpJob& j = sm.job;
       w_start_lead(w, id, j, env.seed(j));
-      in_job = true;
     }
     w.trump = (int)w_uni((u32)w.trump);
     // One node per turn: entered, then the frames it closes, up to the next card played.
@@ -1199,24 +1195,27 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
       w.st = w_uni(w.st);
       w.trick = w_uni(w.trick);
       w_unpack(w);
-      if (w_any((w.nodes & 255u) == 255u)) {
+      if (w.nplayed == 0 && W_RARE(w_any(w.nodes > 255u))) {
+        w_flush(w, id, sm);
         if (env.stop(w, id, sm)) {
           stopped = true;
           break;
         }
       }
       w.nodes++;
-      int card = -1, best = -1, hint = -1;
+      int hint = -1;
       bool store = false;
       WarpTop top = {0, 0};
       int v = w.nplayed == 0 ? w_lead(w, id, env, store, top, hint) : w_enter_follow(w, id);
+      u32 key;  // the next card to play
       if (v < 0) {
-        card = w_expand(w, id, sm, env, top, hint);
+        key = w_expand(w, id, sm, env, top, hint);
       } else {
         // The node is decided: its card is taken back, and the frames it completes with it.
+        int best = -1;
         for (;;) {
-          if (w_any(store)) w_put(w, id, env, v, best);
-          if ((w.st & SW_OFF) == 0) break;  // the root search is done
+          if (W_RARE(w_any(store))) w_put(w, id, env, v, best);
+          if (W_RARE((w.st & SW_OFF) == 0)) goto root_done;
           const int c = w_unplay(w, id, sm);
           best = -1;
           if (w_any(v == (int)ns_side(wi_seat(w.info)))) {  // the child cuts
@@ -1224,19 +1223,19 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
             best = c;
           } else {
             w.at |= w.rel;
-            w.info += WI_NEXT;
-            card = w_next(w, id, sm);
-            if (card >= 0) break;
+            key = w_next(w, id, sm);
+            if (key) break;
             v = wi_result(w.info);
           }
           w.rel = w_widen(w, id);
           store = w.nplayed == 0;
         }
-      }
-      if (w_any(card < 0)) {
-        in_job = w_end_root(w, id, sm, env, v, best);
-        if (w_any(!in_job)) break;
-        continue;
+        if (false) {
+        root_done:
+          in_job = w_end_root(w, id, sm, env, v, best);
+          if (w_any(!in_job)) break;
+          continue;
+        }
       }
 #ifdef DDG_BOUNDS_CHECK
       if ((w.st & SW_OFF) >= STACK_DEPTH * SW_FRAME) {  // counted, skipped: the warp stops, its results stay unsolved
@@ -1246,7 +1245,7 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
         return;
       }
 #endif
-      w_play(w, id, sm, card);
+      w_play(w, id, sm, key);
     }
     if (w_any(stopped)) return;  // (a return out of both loops would cost ptxas the proof)
   }

@@ -74,7 +74,6 @@ struct Env {
     if (id.t == 0) x->asked++;
     w_sync();
     const bool end = x->b->stop_every && x->asked % x->b->stop_every == 0;
-    w_flush(w, id, sm);
     if (end && id.t == 0) sm.job.stage = ST_ENTER;
     w_sync();
     return end;
@@ -101,7 +100,7 @@ void fiber(void* arg, int t) {
 
 extern "C" {
 // n deals; stats[0..5] = nodes, probes, hits, stores, entry reads, TT bytes. `stop_every`:
-// every so many stop questions (256 nodes each) the warp's registers are kept, it ends and
+// every so many stop questions (256 nodes or a few more each) the warp's registers are kept, it ends and
 // is started again. `backwards`: the fibers run ahead of one another in the other order.
 int warp_replay(const uint64_t* hands, long long n, int tt_log2, int jpd, int mode, const int8_t* seeds,
                 const int8_t* hints, int threads, int stop_every, int backwards, int* out20, int8_t* best20,
