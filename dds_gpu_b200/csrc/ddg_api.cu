@@ -274,11 +274,11 @@ int ddg_solver_create(const ddg_config* cfg_in, ddg_solver** out) {
   s->by_warp = warp_route(cfg);
 #ifndef DDG_TT_SIG
   if (s->by_warp) {
-    e = cudaFuncSetAttribute((const void*)warp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)warp_smem(WARP_MAX));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute((const void*)warp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)warp_smem(WARP_MAX));
+    const void* kernels[] = {(const void*)warp_kernel<WARP_MAX, false>, (const void*)warp_kernel<WARP_FEW, false>,
+                             (const void*)warp_kernel<WARP_MAX, true>};
+    for (int k = 0; k < 3 && e == cudaSuccess; k++)
+      e = cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)warp_smem(k == 1 ? WARP_FEW : WARP_MAX));
     if (e != cudaSuccess) {
       delete s;
       return fail(DDG_E_CUDA, "warp kernel: %s", cudaGetErrorString(e));
@@ -348,7 +348,9 @@ static int launch_batch(ddg_solver* s, const BatchArgs& a, cudaStream_t stream, 
     args.rr_jobs = a.ring ? 0 : std::min<long long>(a.n_jobs, (long long)grid * use);
     *grid_out = grid;
     *block_out = use * 32;
-    const void* fn = a.ring ? (const void*)warp_kernel<true> : (const void*)warp_kernel<false>;
+    const void* fn = a.ring ? (const void*)warp_kernel<WARP_MAX, true>
+                     : use <= WARP_FEW ? (const void*)warp_kernel<WARP_FEW, false>
+                                       : (const void*)warp_kernel<WARP_MAX, false>;
     CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(use * 32), params, warp_smem(use), stream));
     return DDG_OK;
   }

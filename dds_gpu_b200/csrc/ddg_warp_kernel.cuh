@@ -23,7 +23,11 @@
 
 namespace ddg {
 
-enum { WARP_MAX = 32 };
+// Searchers to an SM at most; and at most WARP_FEW in a launch with no more jobs than that,
+// whose kernel may use 104 registers a thread instead of 64. One
+// search alone on an SM 1.31 M against 1.25 M nodes/s; but 16 searchers an SM reach 2.02 G
+// nodes/s where 32 reach 2.30 G, so a launch with more jobs takes 32.
+enum { WARP_MAX = 32, WARP_FEW = 16 };
 
 // A searcher between two slices of a resumable solve, in its lane's save slot. (The frames
 // below the top go to the lane's stack area.)
@@ -227,8 +231,8 @@ struct WarpEnv {
   }
 };
 
-template <bool STREAM>
-__global__ void __launch_bounds__(WARP_MAX * 32, 1) warp_kernel(BatchArgs a) {
+template <int WARPS, bool STREAM>
+__global__ void __launch_bounds__(WARPS * 32, 1) warp_kernel(BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpBlock& sh = *reinterpret_cast<WarpBlock*>(smem_raw);
   const int wid = (int)w_uni(threadIdx.x >> 5), t = threadIdx.x & 31, warps = blockDim.x >> 5;
