@@ -578,13 +578,17 @@ int ddg_solve_begin_ex(ddg_solver* s, const uint64_t* d_hands, int64_t n, const 
   if (s->streaming) return fail(DDG_E_STATE, "a stream is open on this solver");
   CUDA_TRY(cudaSetDevice(s->device));
   if (!s->save) {
-    cudaError_t e = cudaMalloc(&s->save, (size_t)s->lanes * sizeof(LaneSave));
+    size_t bytes = (size_t)s->lanes * sizeof(LaneSave);
+#ifndef DDG_TT_SIG
+    if (s->by_warp) bytes = (size_t)std::min(s->lanes, s->sms * WARP_MAX) * sizeof(WarpSave);
+#endif
+    cudaError_t e = cudaMalloc(&s->save, bytes);
     if (e != cudaSuccess) {
       s->save = nullptr;
       return fail(e == cudaErrorMemoryAllocation ? DDG_E_MEMORY : DDG_E_CUDA, "lane save area: %s",
                   cudaGetErrorString(e));
     }
-    s->bytes += (size_t)s->lanes * sizeof(LaneSave);
+    s->bytes += bytes;
   }
   cudaStream_t stream = (cudaStream_t)stream_v;
   s->slice_args = make_args(s, d_hands, n, d_seed20, d_out20, nullptr);

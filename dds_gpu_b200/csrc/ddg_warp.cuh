@@ -94,6 +94,7 @@ struct WarpJob {
 
 struct WarpMem {
   WarpFrame fr[STACK_DEPTH];
+  u64 hash[14];         // of the trick starts being searched, by tricks left
   uint8_t scratch[16];  // candidates, handed to threads 0, 1, 2, ...
   WarpJob job;
 };
@@ -137,20 +138,20 @@ DDG_W void w_count(WarpState& w, const WarpIds& id, int what, u32 k) {
 
 // ---- key and owner codes -------------------------------------------------------------------
 
+struct WarpLens {
+  u32 hi, lo;  // length_key()
+};
+// Suit lengths of all hands: one popcount for the 16 holdings, two OR reductions.
+DDG_W WarpLens w_lens(const WarpState& w, const WarpIds& id) {
+  const u32 part = (u32)w_popc(w.m) << (28 - 4 * (id.t & 7));
+  return WarpLens{w_or(id.t & 8 ? 0 : part), w_or(id.t & 8 ? part : 0)};
+}
 struct WarpKey {
   u32 q, q_hi;  // hash bits 9..40 and 41..47
-  u32 lens_hi, lens_lo;  // length_key()
   u32 bucket, tag;
 };
-
-// Suit lengths of all hands and their hash (make_key): one popcount for the 16 holdings,
-// two OR reductions for the 64-bit word.
-DDG_W WarpKey w_key(const WarpState& w, const WarpIds& id, u32 mask) {
+DDG_W WarpKey w_key(const WarpState& w, u64 x, u32 mask) {  // make_key
   WarpKey k;
-  const u32 part = (u32)w_popc(w.m) << (28 - 16 * (id.p & 1) - 4 * id.s);
-  k.lens_hi = w_or(id.p < 2 ? part : 0);
-  k.lens_lo = w_or(id.p >= 2 ? part : 0);
-  const u64 x = key_hash((u64)k.lens_hi << 32 | k.lens_lo, w.leader);
   k.bucket = (u32)x & mask;
   k.q = (u32)(x >> 9);
   k.q_hi = (u32)(x >> 41) & 0x7Fu;
@@ -175,13 +176,13 @@ DDG_W u32 w_build_code(const WarpState& w, const WarpIds& id) {
 // The owners of the highest n cards, lowest card in the low bits (n = 0: 0; at most 13).
 DDG_W u32 w_pattern(u32 code, int twice_n) { return w_shl_hi(0, code, twice_n); }
 
-// The top n cards of a suit.
-DDG_W u32 w_top_n(u32 all, int n) {
-  int r = 0;
-#pragma unroll
-  for (int step = 8; step; step >>= 1)
-    if (w_popc(all >> (r + step)) >= n) r += step;
-  return (all >> r) << r;
+// The top n cards of this thread's suit: the suit's eight threads each test two ranks for n
+// cards at or above them.
+DDG_W u32 w_top_n(const WarpIds& id, u32 all, int n) {
+  const int r = id.t >> 2;
+  const u32 a = w_ballot(w_popc(all >> r) >= n) >> id.s & 0x11111111u, b = w_ballot(w_popc(all >> (r + 8)) >= n) >> id.s & 0x11111111u;
+  const int low = w_popc(a) + w_popc(b) - 1;
+  return (all >> low) << low;
 }
 
 // A searcher has its table to itself, so its entries are stored as they are (those of tables
@@ -252,7 +253,7 @@ DDG_W int w_probe(WarpState& w, const WarpIds& id, const TTBucket* b, u32 tagw, 
   if (dec) {
     const int at = w_low(dec);
     const u32 c = w_shfl(counts, at);
-    w.rel = w_top_n(w.all, (int)(c >> (4 * id.s)) & 15);
+    w.rel = w_top_n(id, w.all, (int)(c >> (4 * id.s)) & 15);
     w_count(w, id, WCNT_HITS, 1);
     return (int)((up >> at) & 1);
   }
@@ -265,13 +266,13 @@ DDG_W int w_probe(WarpState& w, const WarpIds& id, const TTBucket* b, u32 tagw, 
 // checks its entry, and the tag line shifts by one shuffle.
 DDG_W void w_store(WarpState& w, const WarpIds& id, TTBucket* b, u32 tagw, const WarpKey& k, u32 code, u32 rel, int lb,
                    int ub, int best) {
-  const int above = rel ? w_popc(w.all >> w_low(rel)) : 0;  // cards at or above the lowest relevant one
-  const u32 counts = w_or((u32)above << (4 * id.s));
-  const int n0 = (int)(counts & 15), n1 = (int)(counts >> 4 & 15), n2 = (int)(counts >> 8 & 15);
-  if (n0 + n1 + n2 + (int)(counts >> 12) > MAX_REL) return;
-  const int off = (id.s > 0 ? n0 : 0) + (id.s > 1 ? n1 : 0) + (id.s > 2 ? n2 : 0);
-  const u64 mine = (u64)w_pattern(code, 2 * above) << (2 * off);
-  const u32 own_lo = w_or((u32)mine), own_hi = w_or((u32)(mine >> 32));
+  const u32 above = (u32)w_popc(w.all & (0u - (rel & (0u - rel))));  // cards at or above the lowest relevant one
+  const u32 each = w_or(above << (8 * id.s)), upto = each * 0x01010101u;  // a byte a suit; of the suits up to it
+  if ((upto >> 24) > MAX_REL) return;
+  const u32 n4 = (each | each >> 4) & 0x00FF00FFu, counts = (n4 | n4 >> 8) & 0xFFFFu;
+  const int off = 2 * (int)((upto >> (8 * id.s) & 0xFF) - above);
+  const u32 pat = w_pattern(code, 2 * (int)above);
+  const u32 own_lo = w_or(off < 32 ? pat << off : 0), own_hi = w_or(off < 32 ? w_shl_hi(0, pat, off) : pat << (off & 31));
   WarpEntry e = {k.q, k.q_hi | own_hi >> 16 << 21, counts | own_lo << 16, own_lo >> 16 | own_hi << 16};
   const bool match = id.t < TT_WAYS && (tagw & ~0xF00u) == k.tag;
   const u32 mm = w_ballot(match);
@@ -293,9 +294,7 @@ DDG_W void w_store(WarpState& w, const WarpIds& id, TTBucket* b, u32 tagw, const
     lb = olb > lb ? olb : lb;
     ub = oub < ub ? oub : ub;
     best = best < 0 ? obest : best;
-    w_count(w, id, WCNT_BYTES, 64 + 16 * (u32)w_popc(mm & ((sm & (0u - sm)) * 2 - 1)) + 8);
   } else {
-    w_count(w, id, WCNT_BYTES, 64 + 16 * (u32)w_popc(mm) + 64 + 16);
     // The way (take_way): the first empty one, else the least 2 * tricks left + age, other
     // generations first; of equal ones the oldest.
     const int age = TT_WAYS - 1 - (id.t & 15);
@@ -306,6 +305,8 @@ DDG_W void w_store(WarpState& w, const WarpIds& id, TTBucket* b, u32 tagw, const
     const u32 prev = w_shfl_up1(tagw);
     if (id.t <= pos) b->tag[id.t] = id.t == 0 ? (k.tag | (u32)way << 8) : prev;
   }
+  // (the entries read: up to the one that matches)
+  w_count(w, id, WCNT_BYTES, (sm ? 64 + 8 : 64 + 64 + 16) + 16 * (u32)w_popc(mm & ((sm & (0u - sm)) * 2 - 1)));
   e.w0 |= ((u32)lb | (u32)ub << 4 | (u32)(best < 0 ? 63 : best) << 8) << 7;
   if (id.t == TT_WAYS) w_entry_put(b, way, e);
   w_sync();
@@ -326,10 +327,10 @@ DDG_W int rt_sec(u32 a) { return (int)(a >> 20) & 15; }
 DDG_W int rt_thr(u32 a) { return (int)(a >> 24) & 15; }
 DDG_W int rt_rank(u32 r, int k) { return (int)(r >> (4 * k)) & 15; }
 
-DDG_W WarpTop w_make_top(const WarpState& w, const WarpIds& id, const WarpKey& k) {
+DDG_W WarpTop w_make_top(const WarpState& w, const WarpIds& id, const WarpLens& k) {
   const int sh = 12 - 4 * id.s;  // lengths of seats 0..3 in this suit, then rotated to the leader
-  const u32 l = ((k.lens_hi >> (sh + 16)) & 15) | ((k.lens_hi >> sh) & 15) << 4 | ((k.lens_lo >> (sh + 16)) & 15) << 8 |
-                ((k.lens_lo >> sh) & 15) << 12;
+  const u32 l = ((k.hi >> (sh + 16)) & 15) | ((k.hi >> sh) & 15) << 4 | ((k.lo >> (sh + 16)) & 15) << 8 |
+                ((k.lo >> sh) & 15) << 12;
   WarpTop t;
   t.a = ((l | l << 16) >> (4 * w.leader)) & 0xFFFFu;
   // bit 28: of the cards the leader does not hold, partner's is the highest
@@ -910,7 +911,7 @@ DDG_W u32 w_tags(const TTBucket* b, const WarpIds& id) { return b->tag[id.t & 15
 // ENTER at a trick start (enter_lead): cutoffs, the last trick, the TT probe, the bounds. The
 // value (w.rel set; `store`: a bound's, to be stored), or -1 when the node expands.
 template <class Env>
-DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool& store, WarpTop& top, int& hint) {
+DDG_W int w_lead(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, bool& store, WarpTop& top, int& hint) {
   w.rel = 0;
   if (w.need <= 0) return 1;
   if (w.left < w.need) return 0;
@@ -921,11 +922,15 @@ DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool& store, WarpTop
     if (id.s == su && w_popc(in) >= 2) w.rel = 1u << w_top(in);
     return (int)(~w_shfl(w.code, su) >> 30 & 1);  // the top card's holder is N or S
   }
-  const WarpKey k = w_key(w, id, env.mask());
+  const WarpLens lens = w_lens(w, id);
+  const u64 x = key_hash((u64)lens.hi << 32 | lens.lo, w.leader);
+  const WarpKey k = w_key(w, x, env.mask());
   const TTBucket* b = env.table() + k.bucket;
   const int hit = w_probe(w, id, b, w_tags(b, id), k, w.code, w.need, hint);
   if (W_OFTEN(hit >= 0)) return hit;
-  top = w_make_top(w, id, k);
+  if (id.t == 0) sm.hash[w.left] = x;  // for the store
+  w_sync();
+  top = w_make_top(w, id, lens);
   const bool ns_lead = ns_side(w.leader);
   const int cut_ns = w.need, cut_ew = w.left - w.need + 1;
   bool decided;
@@ -945,8 +950,8 @@ DDG_W int w_lead(WarpState& w, const WarpIds& id, Env& env, bool& store, WarpTop
 // A trick start's result goes to the table (a bound's, or a finished node's with its
 // cutting card `best` or -1).
 template <class Env>
-DDG_W void w_put(WarpState& w, const WarpIds& id, Env& env, int v, int best) {
-  const WarpKey k = w_key(w, id, env.mask());
+DDG_W void w_put(WarpState& w, const WarpIds& id, const WarpMem& sm, Env& env, int v, int best) {
+  const WarpKey k = w_key(w, sm.hash[w.left], env.mask());
   TTBucket* b = env.table() + k.bucket;
   w_store(w, id, b, w_tags(b, id), k, w.code, w.rel, v ? w.need : 0, v ? w.left : w.need - 1, best);
 }
@@ -1206,7 +1211,7 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
       int hint = -1;
       bool store = false;
       WarpTop top = {0, 0};
-      int v = w.nplayed == 0 ? w_lead(w, id, env, store, top, hint) : w_enter_follow(w, id);
+      int v = w.nplayed == 0 ? w_lead(w, id, sm, env, store, top, hint) : w_enter_follow(w, id);
       u32 key;  // the next card to play
       if (v < 0) {
         key = w_expand(w, id, sm, env, top, hint);
@@ -1214,7 +1219,7 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
         // The node is decided: its card is taken back, and the frames it completes with it.
         int best = -1;
         for (;;) {
-          if (W_RARE(w_any(store))) w_put(w, id, env, v, best);
+          if (w_any(store)) w_put(w, id, sm, env, v, best);
           if (W_RARE((w.st & SW_OFF) == 0)) goto root_done;
           const int c = w_unplay(w, id, sm);
           best = -1;

@@ -3,17 +3,16 @@
 // A block is up to WARP_MAX searchers on an SM of its own. A searcher takes a job, runs it to
 // its end and takes the next; searchers share nothing but the queue, so there is no
 // barrier in the loop and the SM's schedulers always have the other warps to issue from.
-// Searcher w of block b owns the TT slice, the stack area and the save slot of lane
-// b * warps + w.
+// Searcher w of block b owns the TT slice, stack area and save slot number b * warps + w.
 //
 // What bounds it: on a full SM the integer pipe and instruction fetch (about 2.6 instructions
 // a cycle; the code a node may run is some 36 KB, the SM's instruction cache holds 32 KB);
-// alone on an SM one warp's chain of instructions, 1,570 cycles a node, of which the
+// alone on an SM one warp's chain of instructions, 1,500 cycles a node, of which the
 // table's memory is a twentieth. Measured against batch_kernel (block phases, 512 lanes to
-// an SM): random 13-card deals with every SM full 2.30 against 0.70 G nodes/s; one job
-// alone on an SM 1.25 M against 0.15 M nodes/s; 240 quick 13-card deals 84 against 1,380 ms;
-// 65,536 six-card endings 125 against 370 ms; 1,200 nine-card endings (a job per lead) 110
-// against 1,160 ms; the 20 leads of a five-card ending asked one by one 2.0 against 17 ms.
+// an SM): random 13-card deals with every SM full 2.36 against 0.70 G nodes/s; one job
+// alone on an SM 1.3 M against 0.15 M nodes/s; 240 quick 13-card deals 78 against 1,367 ms;
+// 65,536 six-card endings 123 against 381 ms; 1,200 nine-card endings (a job per lead) 126
+// against 1,280 ms; the 20 leads of a five-card ending asked one by one 2.4 against 20 ms.
 // batch_kernel stays for helping and for its own options.
 #pragma once
 #include "ddg_kernel.cuh"
@@ -25,20 +24,20 @@ namespace ddg {
 
 // Searchers to an SM at most; and at most WARP_FEW in a launch with no more jobs than that,
 // whose kernel may use 104 registers a thread instead of 64. One
-// search alone on an SM 1.31 M against 1.25 M nodes/s; but 16 searchers an SM reach 2.02 G
-// nodes/s where 32 reach 2.30 G, so a launch with more jobs takes 32.
+// search alone on an SM 1.31 M against 1.25 M nodes/s; but 16 searchers an SM reached 2.02 G
+// nodes/s where 32 reached 2.30 G, so a launch with more jobs takes 32.
 enum { WARP_MAX = 32, WARP_FEW = 16 };
 
-// A searcher between two slices of a resumable solve, in its lane's save slot. (The frames
+// A searcher between two slices of a resumable solve (the solver's save area). (The frames
 // below the top go to the lane's stack area.)
 struct WarpSave {
   uint16_t m[16], all[4], now[4];
   u32 code[4];
   u32 st, trick;
   int trump;
+  u64 hash[14];
   WarpJob job;
 };
-static_assert(sizeof(WarpSave) <= sizeof(LaneSave), "a searcher's state fits its lane's save slot");
 
 struct WarpBlock {
   BatchArgs args;
@@ -254,7 +253,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) warp_kernel(BatchArgs a) {
   memset(&w, 0, sizeof(w));
   w.gen = a.lane_gen[lane];
   WarpFrame* stack = reinterpret_cast<WarpFrame*>(a.stacks) + lane * STACK_DEPTH;
-  WarpSave* sv = a.save ? reinterpret_cast<WarpSave*>(a.save + lane) : nullptr;
+  WarpSave* sv = a.save ? reinterpret_cast<WarpSave*>(a.save) + lane : nullptr;
   if (a.resume) {
     w.m = sv->m[t & 15];
     w.all = sv->all[id.s];
@@ -263,6 +262,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) warp_kernel(BatchArgs a) {
     w.st = sv->st;
     w.trick = sv->trick;
     w.trump = sv->trump;
+    if (t < 14) sm.hash[t] = sv->hash[t];
     const int words = (int)(w.st & SW_OFF) / (16 << 8);
     for (int k = t; k < words; k += 32) reinterpret_cast<uint4*>(sm.fr)[k] = reinterpret_cast<const uint4*>(stack)[k];
     if (t == 0) {
@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) warp_kernel(BatchArgs a) {
   }
   if (sv) {
     if (t < 16) sv->m[t] = (uint16_t)w.m;
+    if (t < 14) sv->hash[t] = sm.hash[t];
     if (t < 4) {
       sv->all[t] = (uint16_t)w.all;
       sv->now[t] = (uint16_t)w.now;
