@@ -113,7 +113,8 @@ struct MlpArgs {
 __device__ __forceinline__ int card_index(int bit) { return (bit >> 4) * 13 + (bit & 15); }
 __device__ __forceinline__ constexpr int card_bit(int idx) { return (idx / 13) * 16 + idx % 13; }
 
-constexpr int MLP_THREADS = 512;
+template <bool TRAIN>
+constexpr int MLP_THREADS = TRAIN ? 512 : 1024;
 constexpr int SM_A = 0, A_BYTES = TILE_M * HID * 2 + 1024;  // activations; training: logits in its upper half
 constexpr int SM_LOGITS = TILE_M * HID;                     // 66 x 128 fp32
 constexpr int SM_RING = A_BYTES, SM_BIAS = SM_RING + 4 * CHUNK, SM_BAR = SM_BIAS + (HID + HID + OUT_PAD) * 4;
@@ -216,14 +217,17 @@ __device__ __forceinline__ void tile_features(const MlpArgs& g, int m0, unsigned
 }
 
 // What bounds it: inference, the GELUs (512 erff a row; the products take a tenth of the
-// time), at 16 warps an SM; a training step's 32 tiles use 32 SMs and are bound by one
-// tile's chain. Measured, against one kernel per layer with its activations in HBM and its
-// weights loaded through registers, chunk by chunk: the 400,000 rows of 20,000 deals 0.55
+// time): 32 warps an SM, 0.53 ms for the rows below against 0.56 with 16. Two CTAs an SM
+// with a ring of their own each, 40 or 32 KB of it, were slower (0.90, 0.60 ms: the weights
+// come too late). A training step's 32 tiles use 32 SMs and are bound by one tile's chain;
+// 32 warps (64 registers, a few spilled) changed nothing there. Measured, against one kernel per layer with its activations in HBM and its
+// weights loaded through registers, chunk by chunk: the 400,000 rows of 20,000 deals 0.53
 // against 14.2 ms; a step of 4,096 rows with its gradients copied out 0.27 against 1.76 ms
 // (5 launches against 28; the three weight gradients 160 us each there, two CTAs walking
 // the whole batch).
 template <bool TRAIN>
-__global__ void __launch_bounds__(MLP_THREADS, 1) mlp_rows(MlpArgs g) {
+__global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
+  constexpr int THREADS = MLP_THREADS<TRAIN>, COLS = HID / (THREADS / TILE_M);  // a thread's columns
   extern __shared__ __align__(128) unsigned char sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* sA = sm + SM_A;
@@ -238,7 +242,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_rows(MlpArgs g) {
     for (int b = 0; b < 9; b++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + b * 8));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
-  for (int k = tid; k < HID + HID + OUT_PAD; k += MLP_THREADS)
+  for (int k = tid; k < HID + HID + OUT_PAD; k += THREADS)
     bias[k] = g.master[k < HID ? OFF_B1 + k : k < 2 * HID ? OFF_B2 + k - HID : OFF_B3 + k - 2 * HID];
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
@@ -250,12 +254,12 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_rows(MlpArgs g) {
   int q = 0;  // chunks used (thread 0)
   if (tid == 0)
     for (int c = 0; c < 4 && ring.issued < ring.total; c++) ring.load();
-  const int quarter = warp & 3, group = warp >> 2;  // tensor-memory lanes 32 * quarter.., columns 64 * group..
+  const int quarter = warp & 3, group = warp >> 2;  // tensor-memory lanes 32 * quarter.., columns COLS * group..
   const int row = quarter * 32 + lane;
   const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
   uint32_t phase = 0;
   bool ok = true;
-  if (mine) tile_features(g, (int)blockIdx.x * TILE_M, sA, tid, MLP_THREADS);
+  if (mine) tile_features(g, (int)blockIdx.x * TILE_M, sA, tid, THREADS);
   for (int t = 0; t < mine && ok; t++) {
     const int tile = (int)blockIdx.x + t * (int)gridDim.x, m0 = tile * TILE_M;
     const int64_t at = m0 + row;  // this thread's row
@@ -276,7 +280,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_rows(MlpArgs g) {
     };
     // A hidden layer's epilogue: bias and GELU to A; training keeps both, transposed.
     auto hidden = [&](int col, const float* b, float* Zt, bf16* Ht) {
-      for (int c0 = group * 64; c0 < group * 64 + 64; c0 += 16) {
+      for (int c0 = group * COLS; c0 < (group + 1) * COLS; c0 += 16) {
         uint32_t r[16];
         tmem_ld16(tmem + lanes + (uint32_t)(col + c0), r);
         uint32_t pk[8];
@@ -298,7 +302,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_rows(MlpArgs g) {
     };
     run(0, 4, HID);
     if (TRAIN) {  // the features, transposed, while the first product runs
-      for (int k = warp; k < HID; k += MLP_THREADS / 32)
+      for (int k = warp; k < HID; k += THREADS / 32)
         for (int rr = lane; rr < TILE_M; rr += 32)
           g.Xt[(size_t)k * g.R + m0 + rr] = *reinterpret_cast<const bf16*>(sA + core_at(rr, k, TILE_M));
     }
@@ -311,36 +315,39 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_rows(MlpArgs g) {
     if (!wait()) break;
     if (!TRAIN) {
       if (tid < TILE_M) {  // seeds and root leads: the best trick count, the leader's best-scored card
-        float l[OUT_PAD];
-#pragma unroll
-        for (int c0 = 0; c0 < OUT_PAD; c0 += 16) tmem_ld16(tmem + lanes + (uint32_t)c0, reinterpret_cast<uint32_t*>(l) + c0);
         const int64_t e = at;
-        if (e < g.n) {
-          const float* b = bias + 2 * HID;
-          int arg = 0;
-          float bv = l[0] + b[0];
+        const float* b = bias + 2 * HID;
+        const uint64_t own = e < g.n ? g.hands[e / 20 * 4 + (((int)(e % 4) + 1) & 3)] : 0;
+        int arg = 0, best = -1;
+        float bv = 0.f, bv2 = -1e30f;
 #pragma unroll
-          for (int c = 1; c < OUT_T; c++)
-            if (l[c] + b[c] > bv) {
-              bv = l[c] + b[c];
-              arg = c;
-            }
-          if (g.seed20) g.seed20[e] = (int8_t)arg;
-          if (g.hint20) {
-            const uint64_t own = g.hands[e / 20 * 4 + (((int)(e % 4) + 1) & 3)];
-            int best = -1;
-            bv = -1e30f;
+        for (int c0 = 0; c0 < OUT_PAD; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem + lanes + (uint32_t)c0, r);
 #pragma unroll
-            for (int c = 0; c < OUT_M; c++)
-              if ((own >> card_bit(c) & 1) && l[OUT_T + c] + b[OUT_T + c] > bv) {
-                bv = l[OUT_T + c] + b[OUT_T + c];
-                best = card_bit(c);
+          for (int k = 0; k < 16; k++) {
+            const int c = c0 + k;
+            if (c >= OUT) continue;
+            const float v = __uint_as_float(r[k]) + b[c];
+            if (c == 0) {
+              bv = v;
+            } else if (c < OUT_T) {
+              if (v > bv) {
+                bv = v;
+                arg = c;
               }
-            g.hint20[e] = (int8_t)best;
+            } else if ((own >> card_bit(c - OUT_T) & 1) && v > bv2) {
+              bv2 = v;
+              best = card_bit(c - OUT_T);
+            }
           }
         }
+        if (e < g.n) {
+          if (g.seed20) g.seed20[e] = (int8_t)arg;
+          if (g.hint20) g.hint20[e] = (int8_t)best;
+        }
       } else if (t + 1 < mine) {  // meanwhile the other warps make the next tile's features
-        tile_features(g, (tile + (int)gridDim.x) * TILE_M, sA, tid - TILE_M, MLP_THREADS - TILE_M);
+        tile_features(g, (tile + (int)gridDim.x) * TILE_M, sA, tid - TILE_M, THREADS - TILE_M);
       }
     } else {
       if (tid < TILE_M) {
@@ -421,7 +428,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_rows(MlpArgs g) {
         if (!wait()) break;
         const float* Zt = layer == 0 ? g.Z2t : g.Z1t;
         bf16* dZt = layer == 0 ? g.dZ2t : g.dZ1t;
-        for (int c0 = group * 64; c0 < group * 64 + 64; c0 += 16) {
+        for (int c0 = group * COLS; c0 < (group + 1) * COLS; c0 += 16) {
           uint32_t r[16], pk[8];
           tmem_ld16(tmem + lanes + (uint32_t)(col + c0), r);
 #pragma unroll
@@ -440,7 +447,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_rows(MlpArgs g) {
       if (!ok) break;
       if (t + 1 < mine) {
         __syncthreads();
-        tile_features(g, (tile + (int)gridDim.x) * TILE_M, sA, tid, MLP_THREADS);
+        tile_features(g, (tile + (int)gridDim.x) * TILE_M, sA, tid, THREADS);
       }
     }
   }

@@ -172,7 +172,7 @@ int ddg_guide_train_step(ddg_guide* g, const uint64_t* d_hands, const uint8_t* d
   a.Z2t = g->Z2t;
   a.acc = g->acc;
   a.err = g->err;
-  mlp_rows<true><<<std::min(a.tiles, g->sms), MLP_THREADS, MLP_SMEM, st>>>(a);
+  mlp_rows<true><<<std::min(a.tiles, g->sms), MLP_THREADS<true>, MLP_SMEM, st>>>(a);
   const DwArgs dw = {g->dZ1t, g->Xt, g->dZ2t, g->H1t, g->dOt, g->H2t, R, dw_rows(R), g->part, g->err};
   gemm_dw<<<dim3(DW_TILES, dw_splits(R)), DW_THREADS, DW_SMEM, st>>>(dw);
   if (lr > 0) g->step++;
@@ -221,7 +221,7 @@ static int guide_predict_on(ddg_guide* g, const uint64_t* d_hands, int64_t n, in
     a.seed20 = d_seed20;
     a.hint20 = d_hint20;
     a.err = g->err;
-    mlp_rows<false><<<std::min(a.tiles, g->sms), MLP_THREADS, MLP_SMEM, stream>>>(a);
+    mlp_rows<false><<<std::min(a.tiles, g->sms), MLP_THREADS<false>, MLP_SMEM, stream>>>(a);
     CUDA_TRY(cudaGetLastError());
   }
   if (stream) {
