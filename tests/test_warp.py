@@ -130,14 +130,15 @@ def device_solve(solver, hands, jpd=5):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("lanes", [512, 2048, 0])
+@pytest.mark.parametrize("lanes", [512, 2048, 2560, 0])
 def test_pool_sizes(ddg, lanes):
-    """From four searchers to an SM to the most one holds; jobs fewer and more than them,
-    and more than 63 to a searcher (its TT generation wraps)."""
+    """From three searchers to an SM to the most one holds, on both sides of the 16 up to which
+    a launch takes the build with more registers; jobs fewer and more than them, and more than
+    63 to a searcher of the smallest pool (its TT generation wraps)."""
     s = ddg.Solver(lanes=lanes)
     try:
-        for name, sel in (("k6_4096.npz", slice(0, 4096)), ("k9_120.npz", slice(0, 1)), ("k3_120.npz", slice(0, 120)),
-                          ("k5_120.npz", slice(0, 31))):
+        for name, sel in (("k6_4096.npz", slice(0, 4096)), ("k6_4096.npz", slice(0, 4096)), ("k9_120.npz", slice(0, 1)),
+                          ("k3_120.npz", slice(0, 120)), ("k5_120.npz", slice(0, 31))):
             g = load_golden(name)
             t, nodes, st = device_solve(s, g["hands"][sel])
             assert (t == g["tricks"][sel]).all()
