@@ -57,11 +57,11 @@ BENCH_SET = 20000
 JPD = 5
 SAMPLE = os.path.join(ROOT, "tests", "golden", "k13_bench_2000.npz")
 GUIDED_SAMPLE = os.path.join(ROOT, "tests", "golden", "k13_bench_2000_guided.npz")
-# DRAM bytes (read + write) per search node of one launch of this workload's own shape
-# (TT 2^10, 75,776 lanes, third 0.5 s slice), from `bench.py --profile-case --warmup 2
-# --slice-s 0.5` under ncu (dram__bytes_read.sum + dram__bytes_write.sum = 27.04 + 10.04
-# GB over 350.2 M nodes).
-DRAM_BYTES_PER_NODE = 105.9
+# DRAM bytes (read + write) per search node of one launch of this workload, from
+# `bench.py --profile-case` under ncu: warp_kernel 35.7 (4,588 searchers, third 0.2 s slice:
+# 83.1 GB/s over 200.4 ms and 467.4 M nodes), batch_kernel 105.9 (75,776 lanes, third 0.5 s
+# slice: 27.04 + 10.04 GB over 350.2 M nodes).
+DRAM_BYTES_PER_NODE = {"warp": 35.7, "batch": 105.9}
 WORKLOAD = ("13-card seeded random deals, all 5 strains x 4 declarers, exact TT 2^10 buckets per lane, "
             "one job per (deal, strain)")
 
@@ -529,6 +529,7 @@ def our_arm(a, rank, world, local_rank):
     peak, peak_kind = peaks()
     launches = len(stats)
     achieved = (alg_bytes / launches) / (kernel_ms / launches * 1e-3) / 1e9 if kernel_ms else 0.0
+    by_warp = a.schedule == 0 and not any(it)  # the block phases' counters stay zero: one warp to a search
     eff = {name: (ln[k] / (32.0 * it[k]) if it[k] else None)
            for k, name in enumerate(["cheap", "enter_lead", "enter_follow", "moves_lead", "moves_follow"])}
     s_head = summary[head]
@@ -554,8 +555,8 @@ def our_arm(a, rank, world, local_rank):
         "warp_efficiency": eff,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind,
-                     "traffic": (DRAM_BYTES_PER_NODE * nodes / launches) if DRAM_BYTES_PER_NODE else None,
-                     "kernel": f"ddg::batch_kernel<{solver.block_shape}>",
+                     "traffic": DRAM_BYTES_PER_NODE["warp" if by_warp else "batch"] * nodes / launches,
+                     "kernel": "ddg::warp_kernel" if by_warp else f"ddg::batch_kernel<{solver.block_shape}>",
                      "algorithmic_bytes": (f"64 B per TT probe + 16 B per entry read + 80 B per store: "
                                            f"{alg_bytes / max(1, nodes):.1f} B/node (the kernel's own count, which "
                                            f"also charges each store its tag-line read: "

@@ -10,9 +10,9 @@
 // alone on an SM one warp's chain of instructions, 1,500 cycles a node, of which the
 // table's memory is a twentieth. Measured against batch_kernel (block phases, 512 lanes to
 // an SM): random 13-card deals with every SM full 2.36 against 0.70 G nodes/s; one job
-// alone on an SM 1.3 M against 0.15 M nodes/s; 240 quick 13-card deals 78 against 1,367 ms;
-// 65,536 six-card endings 123 against 381 ms; 1,200 nine-card endings (a job per lead) 126
-// against 1,280 ms; the 20 leads of a five-card ending asked one by one 2.4 against 20 ms.
+// alone on an SM 1.3 M against 0.15 M nodes/s; 240 quick 13-card deals 75 against 1,381 ms;
+// 65,536 six-card endings 122 against 371 ms; 1,200 nine-card endings (a job per lead) 95
+// against 1,074 ms; the 20 leads of a five-card ending asked one by one 2.8 against 23 ms.
 // batch_kernel stays for helping and for its own options.
 #pragma once
 #include "ddg_kernel.cuh"

@@ -36,18 +36,27 @@ typedef struct ddg_guide ddg_guide; /* the learned guide (below) */
 
 /* Solver configuration. Zero fields take the defaults. Mirrors the reference's knobs:
  * TT_LOG2 (gpu/gpu_main.cu:192), THREADS (:202), PER_LEAD (gpu/stream_main.cu:167),
- * TIME_LIMIT (gpu/gpu_main.cu:247). */
+ * TIME_LIMIT (gpu/gpu_main.cu:247).
+ *
+ * Two kernels search. With the defaults it is the warp kernel: a warp to a search, at most 32
+ * searches on an SM (so of a full pool of lanes at most 32 * SMs are in use). Helping, another
+ * block shape or schedule, and any value given to free_below, free_steps, free_pack,
+ * phase_spread, cheap_limit or flat_moves ask for the lane-per-thread kernels, which
+ * these options belong to (a thread to a search, block lanes on an SM); so does
+ * libddg_sig.so. Tricks are the same, and with help = 0 so are the nodes of every job. */
 typedef struct ddg_config {
   int tt_log2;          /* TT buckets per lane = 2^tt_log2, 9..20; default 10 (320 KB per lane) */
-  int lanes;            /* solver lanes (GPU threads, one search each); default: fill the GPU */
-  int block;            /* threads per block (lanes per block): 64, 128, 256 or 512; default 512 */
+  int lanes;            /* solver lanes, one TT each: the most searches at once; default: fill the GPU */
+  int block;            /* threads per block (lanes per block): 64, 128, 256 or 512; default 512
+                           (64 to 256: the lane-per-thread kernels) */
   int jobs_per_deal;    /* 5 = one job per strain, the 4 leads share a TT; 20 = one per lead */
   int device;           /* CUDA device ordinal */
   int schedule;         /* 0: block-phase kernel (all warps of a block run each stage phase
                            in turn over the block's compacted lanes); 1: queue kernel (each
                            warp takes up to 32 lanes from the fullest per-stage queue of its
                            block, no block barriers); 2: block-phase kernel with ENTER
-                           inside a trick run in the cheap pass (four phases, not five) */
+                           inside a trick run in the cheap pass (four phases, not five);
+                           0 with everything else at its default: the warp kernel */
   int min_blocks;       /* resident blocks per SM the kernel is compiled for (register cap):
                            block 64: 1; block 128: 1, 4, 6; block 256: 1..3; block 512: 1;
                            0 = 2 for block 256, else 1 */
@@ -91,8 +100,8 @@ typedef struct ddg_stats {
   uint64_t tt_bytes;       /* TT bytes read + written (tag lines, entries) */
   uint64_t enter_exit[7];  /* ENTER outcomes: trivial, last trick, TT hit, quick tricks,
                               later tricks, 2nd-hand quick tricks, expanded; counted by
-                              libddg_check.so only (zero in libddg.so, whose per-lane
-                              counters are kept small to leave shared memory to L1) */
+                              libddg_check.so's lane-per-thread kernels only (zero elsewhere) */
+  /* The block loop's counters; all zero from the warp kernel, which has no phases. */
   uint64_t phase_warps[5]; /* warp passes per phase of the block loop: cheap stages, ENTER at
                               a trick start, ENTER inside a trick, lead moves, follow moves */
   uint64_t phase_items[5]; /* lanes served by those passes; items / (32 * warps) is the
@@ -104,7 +113,7 @@ typedef struct ddg_stats {
   uint64_t tasks;          /* sibling-move tasks handed to helping lanes */
   int64_t jobs_done;       /* finished jobs */
   double kernel_ms;        /* device time of the solve kernel (CUDA events) */
-  int lanes;               /* lanes launched */
+  int lanes;               /* lanes of the solver */
   int grid, block;         /* launch shape */
   uint64_t tt_entry_reads; /* tag-matched entries read by probes (16 bytes each): the TT's
                               algorithmic bytes are 64 * probes + 16 * entry reads + 80 * stores */
@@ -117,7 +126,8 @@ const char* ddg_last_error(void);
 void ddg_config_default(ddg_config* cfg);
 
 /* Creates a solver on cfg->device: allocates the per-lane TTs and search stacks once
- * (lanes * (320 << tt_log2 + 2.6 KB) bytes) and clears the TT tags. */
+ * (lanes * (320 << tt_log2) bytes, and stacks: 6.9 KB for each of the warp kernel's at
+ * most 32 * SMs searchers, or 2.6 KB a lane) and clears the TT tags. */
 int ddg_solver_create(const ddg_config* cfg, ddg_solver** out);
 void ddg_solver_destroy(ddg_solver* s);
 /* Lanes actually allocated, and the bytes of device memory the pool holds. */
@@ -199,7 +209,8 @@ int ddg_solve_begin_ex(ddg_solver* s, const uint64_t* d_hands, int64_t n, const 
  * for nothing but a free lane: requests that arrive while others are on the GPU start as
  * lanes free up. Lanes that find no deal for idle_timeout_s (0 = 30 s) end; the next
  * submit or poll launches the kernel again. While a stream is open the solver's other
- * calls return DDG_E_STATE. Runs on the block-phase kernel (schedule 0 or 2), helping off. */
+ * calls return DDG_E_STATE. Runs on the warp kernel or the block-phase kernel (schedule 0 or
+ * 2), helping off. */
 typedef struct ddg_stream ddg_stream;
 int ddg_stream_open(ddg_solver* s, int ring_slots, double idle_timeout_s, ddg_stream** out);
 /* A stream whose deals are searched with the learned guide (`guide`, on the solver's
