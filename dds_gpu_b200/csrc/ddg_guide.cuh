@@ -19,6 +19,8 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include "ddg_guide_rows.cuh"
+
 namespace guide_nn {
 
 typedef __nv_bfloat16 bf16;
@@ -33,7 +35,6 @@ enum : int {
   OUT_PAD = 80,  // N of the last layer (a multiple of 16)
   DO_LD = 128,   // row length of dO: K of the dH2 = dO . W3 product (a multiple of 64)
   KCHUNK = 64,
-  TILE_M = 128,
 };
 
 // Flat parameter layout (fp32): W1[256][256] b1[256] W2[256][256] b2[256] W3[80][256] b3[80].
@@ -191,7 +192,7 @@ __device__ __forceinline__ bool product(Ring& ring, int& q, uint32_t a, uint32_t
 
 // Features of rows [m0, m0 + 128) in A, by threads `who` of `of`: card c of owner s is column
 // 4 c + s, then strain and leader; one 16-byte vector holds the owners of two cards.
-__device__ __forceinline__ void tile_features(const MlpArgs& g, int m0, unsigned char* sA, int who, int of) {
+__device__ __forceinline__ void tile_features(const MlpArgs& g, int64_t m0, unsigned char* sA, int who, int of) {
   const int row = who & (TILE_M - 1);
   const int64_t r = m0 + row;
   const int64_t e = g.rows ? g.rows[r] : (r < g.n ? r : -1);
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tslot, a_addr = smem_u32(sA);
   const int per_tile = TRAIN ? 18 : 12;
-  const int mine = blockIdx.x < (unsigned)g.tiles ? (g.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int block = (int)blockIdx.x, grid = (int)gridDim.x, mine = block_tiles(g.tiles, block, grid);
   Ring ring = {smem_u32(sm + SM_RING), bars, bars + 32, g.packed, mine * per_tile, per_tile, 0};
   int q = 0;  // chunks used (thread 0)
   if (tid == 0)
@@ -259,10 +260,9 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
   const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
   uint32_t phase = 0;
   bool ok = true;
-  if (mine) tile_features(g, (int)blockIdx.x * TILE_M, sA, tid, THREADS);
+  if (mine) tile_features(g, first_row(0, block, grid), sA, tid, THREADS);
   for (int t = 0; t < mine && ok; t++) {
-    const int tile = (int)blockIdx.x + t * (int)gridDim.x, m0 = tile * TILE_M;
-    const int64_t at = m0 + row;  // this thread's row
+    const int64_t m0 = first_row(t, block, grid), at = m0 + row;  // the tile's rows, this thread's
     bool good = true;
     // A is written: visible to the tensor cores; the accumulators of before are read.
     auto run = [&](int col, int chunks, int n) {
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
           if (g.hint20) g.hint20[e] = (int8_t)best;
         }
       } else if (t + 1 < mine) {  // meanwhile the other warps make the next tile's features
-        tile_features(g, (tile + (int)gridDim.x) * TILE_M, sA, tid - TILE_M, THREADS - TILE_M);
+        tile_features(g, first_row(t + 1, block, grid), sA, tid - TILE_M, THREADS - TILE_M);
       }
     } else {
       if (tid < TILE_M) {
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
       if (!ok) break;
       if (t + 1 < mine) {
         __syncthreads();
-        tile_features(g, (tile + (int)gridDim.x) * TILE_M, sA, tid, THREADS);
+        tile_features(g, first_row(t + 1, block, grid), sA, tid, THREADS);
       }
     }
   }

@@ -215,7 +215,7 @@ static int guide_predict_on(ddg_guide* g, const uint64_t* d_hands, int64_t n, in
     memset(&a, 0, sizeof(a));
     a.hands = d_hands;
     a.n = total;
-    a.tiles = (int)((total + TILE_M - 1) / TILE_M);
+    a.tiles = (int)tiles_of(total);
     a.packed = g->packed;
     a.master = g->master;
     a.seed20 = d_seed20;
