@@ -175,7 +175,10 @@ __device__ __forceinline__ bool product(Ring& ring, int& q, uint32_t a, uint32_t
   asm volatile("tcgen05.fence::after_thread_sync;");
   for (int c = 0; c < chunks; c++) {
     const int slot = (q + c) & 3;
-    if (!mbar_wait(ring.full + slot * 8, (uint32_t)((q + c) >> 2) & 1)) return false;
+    if (!mbar_wait(ring.full + slot * 8, (uint32_t)((q + c) >> 2) & 1)) {
+      commit(done);  // for the last wait on what was issued
+      return false;
+    }
     for (int j = 0; j < KCHUNK / 16; j++)
       mma(d, smem_desc(a + (c * (KCHUNK / 16) + j) * 2 * lbo_a, lbo_a, 128),
           smem_desc(ring.slots + slot * CHUNK + 2 * j * lbo_b, lbo_b, 128), idesc, c > 0 || j > 0);
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
   const int quarter = warp & 3, group = warp >> 2;  // tensor-memory lanes 32 * quarter.., columns COLS * group..
   const int row = quarter * 32 + lane;
   const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-  uint32_t phase = 0;
+  uint32_t waits = 0;  // for products
   bool ok = true;
   if (mine) tile_features(g, first_row(0, block, grid), sA, tid, THREADS);
   for (int t = 0; t < mine && ok; t++) {
@@ -272,8 +275,7 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
       if (tid == 0) good = product(ring, q, a_addr, tmem + (uint32_t)col, chunks, n, done);
     };
     auto wait = [&]() {  // until the product is done; false on every thread when a wait gave up
-      const bool w = mbar_wait(done, phase);
-      phase ^= 1;
+      const bool w = mbar_wait(done, wait_parity(waits++));
       ok = __syncthreads_and(w && good);
       asm volatile("tcgen05.fence::after_thread_sync;");
       return ok;
@@ -452,10 +454,11 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
     }
   }
   if (!ok && tid == 0) {
-    // A wait gave up: the copies in flight land before their shared memory goes (bounded).
+    // A wait gave up: the copies in flight land before their shared memory goes, the products
+    // before their tensor memory does (bounded).
     atomicExch(g.err, 1);
     for (int c = q; c < ring.issued; c++) mbar_wait(ring.full + (c & 3) * 8, (uint32_t)(c >> 2) & 1);
-    mbar_wait(done, phase);
+    mbar_wait(done, again_parity(waits));
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();

@@ -47,3 +47,29 @@ def test_kernel_takes_its_rows_from_there():
     src = open(os.path.join(CSRC, "ddg_guide.cuh")).read()
     assert not re.search(r"\bint m0\b|\* TILE_M, sA|tile \* TILE_M", src)
     assert len(re.findall(r"\bfirst_row\(", src)) == 4
+
+
+@pytest.mark.parametrize("done_before", [0, 1, 2, 5, 12])
+def test_the_last_wait_is_for_the_product_that_did_not_finish(rows_lib, done_before):
+    """A wait for parity p returns while the phase under way has the other parity. After
+    `done_before` products one does not complete in time: its wait gives up, and so must the
+    wait that is made before the kernel frees what the product uses, until it completes."""
+    class Barrier:
+        phase = 0
+
+        def ready(self, parity):
+            return self.phase & 1 != parity
+
+    bar, waits = Barrier(), 0
+    for _ in range(done_before):
+        assert not bar.ready(rows_lib.rows_wait_parity(waits))
+        bar.phase += 1
+        assert bar.ready(rows_lib.rows_wait_parity(waits))
+        waits += 1
+    assert not bar.ready(rows_lib.rows_wait_parity(waits))  # gives up
+    waits += 1
+    assert not bar.ready(rows_lib.rows_again_parity(waits))
+    bar.phase += 1
+    assert bar.ready(rows_lib.rows_again_parity(waits))
+    src = open(os.path.join(CSRC, "ddg_guide.cuh")).read()
+    assert re.findall(r"mbar_wait\(done, (\w+)", src) == ["wait_parity", "again_parity"]
