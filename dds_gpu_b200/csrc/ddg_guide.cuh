@@ -119,7 +119,7 @@ constexpr int MLP_THREADS = TRAIN ? 512 : 1024;
 constexpr int SM_A = 0, A_BYTES = TILE_M * HID * 2 + 1024;  // activations; training: logits in its upper half
 constexpr int SM_LOGITS = TILE_M * HID;                     // 66 x 128 fp32
 constexpr int SM_RING = A_BYTES, SM_BIAS = SM_RING + 4 * CHUNK, SM_BAR = SM_BIAS + (HID + HID + OUT_PAD) * 4;
-constexpr int MLP_SMEM = SM_BAR + 10 * 8;
+constexpr int MLP_SMEM = SM_BAR + 11 * 8;
 static_assert(SM_LOGITS + OUT * TILE_M * 4 <= A_BYTES && SM_RING % 128 == 0 && SM_BAR % 8 == 0, "shared-memory layout");
 
 __device__ __forceinline__ int chunk_at(int c) {
@@ -175,10 +175,7 @@ __device__ __forceinline__ bool product(Ring& ring, int& q, uint32_t a, uint32_t
   asm volatile("tcgen05.fence::after_thread_sync;");
   for (int c = 0; c < chunks; c++) {
     const int slot = (q + c) & 3;
-    if (!mbar_wait(ring.full + slot * 8, (uint32_t)((q + c) >> 2) & 1)) {
-      commit(done);  // for the last wait on what was issued
-      return false;
-    }
+    if (!mbar_wait(ring.full + slot * 8, (uint32_t)((q + c) >> 2) & 1)) return false;
     for (int j = 0; j < KCHUNK / 16; j++)
       mma(d, smem_desc(a + (c * (KCHUNK / 16) + j) * 2 * lbo_a, lbo_a, 128),
           smem_desc(ring.slots + slot * CHUNK + 2 * j * lbo_b, lbo_b, 128), idesc, c > 0 || j > 0);
@@ -236,14 +233,14 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* sA = sm + SM_A;
   float* bias = reinterpret_cast<float*>(sm + SM_BIAS);
-  const uint32_t bars = smem_u32(sm + SM_BAR), done = bars + 64;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + SM_BAR + 72);
+  const uint32_t bars = smem_u32(sm + SM_BAR), done = bars + 64, last = bars + 72;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + SM_BAR + 80);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(512));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    for (int b = 0; b < 9; b++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + b * 8));
+    for (int b = 0; b < 10; b++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + b * 8));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   for (int k = tid; k < HID + HID + OUT_PAD; k += THREADS)
@@ -261,7 +258,7 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
   const int quarter = warp & 3, group = warp >> 2;  // tensor-memory lanes 32 * quarter.., columns COLS * group..
   const int row = quarter * 32 + lane;
   const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-  uint32_t waits = 0;  // for products
+  uint32_t phase = 0;
   bool ok = true;
   if (mine) tile_features(g, first_row(0, block, grid), sA, tid, THREADS);
   for (int t = 0; t < mine && ok; t++) {
@@ -275,7 +272,8 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
       if (tid == 0) good = product(ring, q, a_addr, tmem + (uint32_t)col, chunks, n, done);
     };
     auto wait = [&]() {  // until the product is done; false on every thread when a wait gave up
-      const bool w = mbar_wait(done, wait_parity(waits++));
+      const bool w = mbar_wait(done, phase);
+      phase ^= 1;
       ok = __syncthreads_and(w && good);
       asm volatile("tcgen05.fence::after_thread_sync;");
       return ok;
@@ -458,7 +456,8 @@ __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
     // before their tensor memory does (bounded).
     atomicExch(g.err, 1);
     for (int c = q; c < ring.issued; c++) mbar_wait(ring.full + (c & 3) * 8, (uint32_t)(c >> 2) & 1);
-    mbar_wait(done, again_parity(waits));
+    commit(last);
+    mbar_wait(last, 0);
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();

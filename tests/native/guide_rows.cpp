@@ -6,6 +6,4 @@ extern "C" {
 int64_t rows_tiles(int64_t rows) { return guide_nn::tiles_of(rows); }
 int rows_block_tiles(int tiles, int block, int grid) { return guide_nn::block_tiles(tiles, block, grid); }
 int64_t rows_first(int t, int block, int grid) { return guide_nn::first_row(t, block, grid); }
-uint32_t rows_wait_parity(uint32_t n) { return guide_nn::wait_parity(n); }
-uint32_t rows_again_parity(uint32_t n) { return guide_nn::again_parity(n); }
 }

@@ -49,27 +49,16 @@ def test_kernel_takes_its_rows_from_there():
     assert len(re.findall(r"\bfirst_row\(", src)) == 4
 
 
-@pytest.mark.parametrize("done_before", [0, 1, 2, 5, 12])
-def test_the_last_wait_is_for_the_product_that_did_not_finish(rows_lib, done_before):
-    """A wait for parity p returns while the phase under way has the other parity. After
-    `done_before` products one does not complete in time: its wait gives up, and so must the
-    wait that is made before the kernel frees what the product uses, until it completes."""
-    class Barrier:
-        phase = 0
-
-        def ready(self, parity):
-            return self.phase & 1 != parity
-
-    bar, waits = Barrier(), 0
-    for _ in range(done_before):
-        assert not bar.ready(rows_lib.rows_wait_parity(waits))
-        bar.phase += 1
-        assert bar.ready(rows_lib.rows_wait_parity(waits))
-        waits += 1
-    assert not bar.ready(rows_lib.rows_wait_parity(waits))  # gives up
-    waits += 1
-    assert not bar.ready(rows_lib.rows_again_parity(waits))
-    bar.phase += 1
-    assert bar.ready(rows_lib.rows_again_parity(waits))
+def test_the_last_wait_is_for_the_products_in_flight():
+    """A wait for a parity returns while the phase under way has the other one, so a wait after
+    one that gave up on a product needs a phase that nothing has completed: a barrier of its
+    own, which a last commit arrives on when all products issued are done."""
     src = open(os.path.join(CSRC, "ddg_guide.cuh")).read()
-    assert re.findall(r"mbar_wait\(done, (\w+)", src) == ["wait_parity", "again_parity"]
+    end = src[src.index("if (!ok && tid == 0) {"):]
+    end = end[:end.index("tcgen05.dealloc")]
+    assert end.index("commit(last);") < end.index("mbar_wait(last, 0);")
+    assert len(re.findall(r"\blast\b[,;)]", src)) == 2  # used nowhere else
+    assert "mbar_wait(done" not in end
+    barriers = int(re.search(r"b < (\d+); b\+\+\) asm volatile\(\"mbarrier.init", src).group(1))
+    assert "done = bars + 64, last = bars + 72" in src and barriers == 72 // 8 + 1
+    assert "sm + SM_BAR + 80)" in src and "MLP_SMEM = SM_BAR + 11 * 8" in src  # then tensor memory's address
