@@ -95,7 +95,9 @@ struct WarpJob {
 struct WarpMem {
   WarpFrame fr[STACK_DEPTH];
   u64 hash[14];         // of the trick starts being searched, by tricks left
-  uint8_t scratch[16];  // candidates, handed to threads 0, 1, 2, ...
+  // Candidates, handed to threads 0, 1, 2, ... A hand of 13 has at most 13, but device-memory
+  // deals come unchecked, and four suits of 13 ranks hold at most 28 runs.
+  uint8_t scratch[32];
   WarpJob job;
 };
 
