@@ -118,6 +118,9 @@ struct WarpState {
   int leader, nplayed, left, need;  // fields of st, as w_unpack() last read them
   u32 nodes;  // nodes since the last flush
   u32 gen;
+#ifdef DDG_BOUNDS_CHECK
+  bool fault;  // a bounds check failed
+#endif
 };
 DDG_W void w_unpack(WarpState& w) {
   w.leader = (int)(w.st & SW_LEADER);
@@ -137,6 +140,23 @@ struct WarpIds {  // what a thread stands for
 DDG_W void w_count(WarpState& w, const WarpIds& id, int what, u32 k) {
   if (id.t == what) w.cnt += k;
 }
+
+// Bounds-checked builds (libddg_check.so): every frame, table bucket, trick hash and candidate
+// slot is checked before its access. A check that fails is counted and the access skipped; the
+// searcher then ends (w_fault), its job's results unsolved, and the call reports the count as an
+// error. (Ways and positions in a bucket are 4-bit fields of 16.) In other builds nothing is left.
+#ifdef DDG_BOUNDS_CHECK
+DDG_W bool w_in_bounds(WarpState& w, const WarpIds& id, bool ok) {
+  if (w_any(!ok)) {
+    w_count(w, id, WCNT_BOUNDS, 1);
+    w.fault = true;
+  }
+  return !w_any(!ok);
+}
+#define W_IN_BOUNDS(ok) w_in_bounds(w, id, ok)
+#else
+#define W_IN_BOUNDS(ok) true
+#endif
 
 // ---- key and owner codes -------------------------------------------------------------------
 
@@ -884,10 +904,11 @@ DDG_W u32 w_follow_floor(const WarpState& w, int n, int seat) {
 
 // Hands the cards of `cm` ([sp], the threads of `seat`) to threads 0, 1, 2, ...: thread
 // t looks at cards t and t + 32. Returns their number; `card` is this thread's.
-DDG_W int w_compact(const WarpIds& id, WarpMem& sm, u32 cm, int seat, int& card) {
+DDG_W int w_compact(WarpState& w, const WarpIds& id, WarpMem& sm, u32 cm, int seat, int& card) {
   const u32 a = w_shfl(cm, 4 * seat + (id.t >> 4)), b = w_shfl(cm, 4 * seat + 2 + (id.t >> 4));
   const bool ha = a >> (id.t & 15) & 1, hb = b >> (id.t & 15) & 1;
   const u32 ma = w_ballot(ha), mb = w_ballot(hb), lt = (1u << id.t) - 1;
+  if (!W_IN_BOUNDS(w_popc(ma) + w_popc(mb) <= 13)) return 0;
   if (ha) sm.scratch[w_popc(ma & lt)] = (uint8_t)id.t;
   if (hb) sm.scratch[w_popc(ma) + w_popc(mb & lt)] = (uint8_t)(id.t + 32);
   w_sync();
@@ -927,6 +948,7 @@ DDG_W int w_lead(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, bool& s
   const WarpLens lens = w_lens(w, id);
   const u64 x = key_hash((u64)lens.hi << 32 | lens.lo, w.leader);
   const WarpKey k = w_key(w, x, env.mask());
+  if (!W_IN_BOUNDS(k.bucket <= env.mask() && w.left < 14)) return 0;
   const TTBucket* b = env.table() + k.bucket;
   const int hit = w_probe(w, id, b, w_tags(b, id), k, w.code, w.need, hint);
   if (W_OFTEN(hit >= 0)) return hit;
@@ -953,7 +975,9 @@ DDG_W int w_lead(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, bool& s
 // cutting card `best` or -1).
 template <class Env>
 DDG_W void w_put(WarpState& w, const WarpIds& id, const WarpMem& sm, Env& env, int v, int best) {
+  if (!W_IN_BOUNDS(w.left < 14)) return;
   const WarpKey k = w_key(w, sm.hash[w.left], env.mask());
+  if (!W_IN_BOUNDS(k.bucket <= env.mask())) return;
   TTBucket* b = env.table() + k.bucket;
   w_store(w, id, b, w_tags(b, id), k, w.code, w.rel, v ? w.need : 0, v ? w.left : w.need - 1, best);
 }
@@ -973,7 +997,7 @@ DDG_W u32 w_expand(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, const
   u32 who = led;  // the threads that stand for a candidate
   int n = w_popc(led), card = ls * 16 + (id.t & 15);  // following suit: thread r for rank r
   if (!led) {
-    n = w_compact(id, sm, cm, seat, card);
+    n = w_compact(w, id, sm, cm, seat, card);
     who = (1u << n) - 1;
   }
   w.at = 0;
@@ -992,6 +1016,7 @@ DDG_W u32 w_expand(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env, const
     weight = w_follow_weight(w, w.nplayed, seat, !led, card);
   }
   const u32 key = who >> id.t & 1 ? (u32)(weight + KEY_BIAS) << 6 | (u32)card : 0;
+  if (!W_IN_BOUNDS((w.st & SW_OFF) < STACK_DEPTH * SW_FRAME)) return 0;
   if (id.t < 16) w_frame(sm, w.st).keys[id.t] = (uint16_t)key;
   return w_max(key);
 }
@@ -1008,6 +1033,7 @@ DDG_W int w_enter_follow(WarpState& w, const WarpIds& id) {
 // Plays the card of `key` from the top frame and pushes the frame (play): at the fourth card the
 // trick is settled and the frame keeps what taking it back needs.
 DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, u32 key) {
+  if (!W_IN_BOUNDS((w.st & SW_OFF) < STACK_DEPTH * SW_FRAME)) return;
   WarpFrame& f = w_frame(sm, w.st);
   const int card = key_card(key), su = card_suit(card), r = card & 15, np8 = (int)(w.st & SW_NP8);
   const u32 bit = 1u << r, code = w.code, st = w.st, trick = w.trick, cards = w.all | w.now << 16;
@@ -1047,6 +1073,7 @@ DDG_W void w_play(WarpState& w, const WarpIds& id, WarpMem& sm, u32 key) {
 // Pops the top frame and takes its card back (node_done, unplay); returns the card.
 DDG_W int w_unplay(WarpState& w, const WarpIds& id, WarpMem& sm) {
   const bool completed = (w.st & SW_NP8) == 0;  // this ply completed a trick
+  if (!W_IN_BOUNDS((w.st & SW_OFF) - SW_FRAME < STACK_DEPTH * SW_FRAME)) return 0;
   const WarpFrame& f = w_frame(sm, w.st - SW_FRAME);
   w.st = f.suit[0].word;
   w.info = f.suit[1].word;
@@ -1147,6 +1174,19 @@ DDG_W void w_flush(WarpState& w, const WarpIds& id, WarpMem& sm) {
   w_sync();
 }
 
+// Ends the searcher after a failed bounds check.
+DDG_W bool w_fault(WarpState& w, const WarpIds& id, WarpMem& sm) {
+#ifdef DDG_BOUNDS_CHECK
+  if (!w_any(w.fault)) return false;
+  w_flush(w, id, sm);
+  if (id.t == 0) sm.job.stage = ST_IDLE;
+  w_sync();
+  return true;
+#else
+  return false;
+#endif
+}
+
 // A root search is done with value v and the root's cutting card `best` (or -1): the next
 // search of the job, or its end (false).
 template <class Env>
@@ -1214,6 +1254,7 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
       bool store = false;
       WarpTop top = {0, 0};
       int v = w.nplayed == 0 ? w_lead(w, id, sm, env, store, top, hint) : w_enter_follow(w, id);
+      if (w_fault(w, id, sm)) return;
       u32 key;  // the next card to play
       if (v < 0) {
         key = w_expand(w, id, sm, env, top, hint);
@@ -1224,6 +1265,7 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
           if (w_any(store)) w_put(w, id, sm, env, v, best);
           if (W_RARE((w.st & SW_OFF) == 0)) goto root_done;
           const int c = w_unplay(w, id, sm);
+          if (w_fault(w, id, sm)) return;
           best = -1;
           if (w_any(v == (int)ns_side(wi_seat(w.info)))) {  // the child cuts
             w.at = (w.at & 0xFFFF0000u) | w.rel;
@@ -1244,14 +1286,7 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
           continue;
         }
       }
-#ifdef DDG_BOUNDS_CHECK
-      if ((w.st & SW_OFF) >= STACK_DEPTH * SW_FRAME) {  // counted, skipped: the warp stops, its results stay unsolved
-        w_count(w, id, WCNT_BOUNDS, 1);
-        w_flush(w, id, sm);
-        if (id.t == 0) sm.job.stage = ST_IDLE;
-        return;
-      }
-#endif
+      if (w_fault(w, id, sm)) return;
       w_play(w, id, sm, key);
     }
     if (w_any(stopped)) return;  // (a return out of both loops would cost ptxas the proof)
