@@ -45,7 +45,7 @@ def measure(cfg, d_hands, n, window_s, torch):
         if st["kernel_ms"] == 0:  # a small set was solved in the warm-up slice: score that one
             st = warm
         sec = st["kernel_ms"] * 1e-3
-        return st["nodes"] / sec, st["jobs_done"] / sec, st["lanes"]
+        return st["nodes"] / sec, st["jobs_done"] / sec, s.lanes
     finally:
         s.close()
 

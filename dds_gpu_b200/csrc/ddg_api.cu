@@ -367,6 +367,9 @@ static int launch_batch(ddg_solver* s, const BatchArgs& a, cudaStream_t stream, 
   return DDG_OK;
 }
 
+// Searches a launch can have under way: a warp each, or a thread each.
+static int launched_lanes(const ddg_solver* s, int grid, int block) { return grid * (s->by_warp ? block / 32 : block); }
+
 static BatchArgs make_args(ddg_solver* s, const uint64_t* d_hands, int64_t n, const int8_t* d_seed20,
                            uint8_t* d_out20, uint64_t* d_job_nodes) {
   BatchArgs a;
@@ -444,7 +447,7 @@ static int take_stats(ddg_solver* s, int grid, int block, ddg_stats* st, const u
   st->kernel_ms = ms;
   st->grid = grid;
   st->block = block;
-  st->lanes = s->lanes;
+  st->lanes = launched_lanes(s, grid, block);
   return DDG_OK;
 }
 
@@ -676,6 +679,7 @@ struct ddg_stream {
   bool launched = false;
   double idle_timeout_s = 30;
   int launches = 0;
+  int grid = 0, block = 0;  // of the kernel
 };
 
 static void stream_free(ddg_stream* st) {
@@ -730,8 +734,7 @@ static int stream_kernel(ddg_stream* st) {
     a.hint20 = st->d_hint;
   }
   *(volatile int*)s->h_stop = 0;
-  int grid = 0, block = 0;
-  int rc = launch_batch(s, a, st->kstream, st->guide ? s->sms - 2 : s->sms, &grid, &block);
+  int rc = launch_batch(s, a, st->kstream, st->guide ? s->sms - 2 : s->sms, &st->grid, &st->block);
   if (rc) return rc;
   CUDA_TRY(cudaEventRecord(st->kdone, st->kstream));
   st->launched = true;
@@ -918,9 +921,9 @@ int ddg_stream_close(ddg_stream* st, int drain, ddg_stats* stats) {
       for (int k = 0; k < 7; k++) stats->enter_exit[k] = c[CNT_EXIT + k];
       stats->jobs_done = (int64_t)c[CNT_JOBS_DONE];
       stats->iterations = c[CNT_ITERS];
-      stats->lanes = st->s->lanes;
-      stats->block = st->s->block;
-      stats->grid = st->s->lanes / st->s->block;
+      stats->lanes = launched_lanes(st->s, st->grid, st->block);
+      stats->block = st->block;
+      stats->grid = st->grid;
       stats->tasks = (uint64_t)st->launches;
     }
     st->s->total_nodes += c[CNT_NODES];

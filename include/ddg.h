@@ -113,7 +113,7 @@ typedef struct ddg_stats {
   uint64_t tasks;          /* sibling-move tasks handed to helping lanes */
   int64_t jobs_done;       /* finished jobs */
   double kernel_ms;        /* device time of the solve kernel (CUDA events) */
-  int lanes;               /* lanes of the solver */
+  int lanes;               /* lanes launched: searches that could run at once */
   int grid, block;         /* launch shape */
   uint64_t tt_entry_reads; /* tag-matched entries read by probes (16 bytes each): the TT's
                               algorithmic bytes are 64 * probes + 16 * entry reads + 80 * stores */
