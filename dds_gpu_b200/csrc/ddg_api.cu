@@ -15,6 +15,7 @@
 
 #include "ddg.h"
 #include "ddg_kernel.cuh"
+#include "ddg_shape.hpp"
 #include "ddg_warp_kernel.cuh"
 
 using namespace ddg;
@@ -338,13 +339,8 @@ static int launch_batch(ddg_solver* s, const BatchArgs& a, cudaStream_t stream, 
   void* params[] = {&args};
 #ifndef DDG_TT_SIG
   if (s->by_warp) {
-    // One block per SM, the lanes' TT slices spread over them; a batch with fewer jobs than
-    // that takes fewer searchers (a stream's jobs are yet to come).
-    const long long want = a.ring || a.n_jobs > s->lanes ? s->lanes : a.n_jobs;
-    const int grid = (int)std::min<long long>(sms, want);
-    const int warps = (int)std::min<long long>(WARP_MAX, a.ring ? want / grid : (want + grid - 1) / grid);
-    const int fit = s->lanes / grid;  // every searcher has a lane
-    const int use = warps < fit ? warps : fit;
+    const WarpShape shape = warp_shape(sms, s->lanes, a.n_jobs, a.ring != nullptr);
+    const int grid = shape.grid, use = shape.warps;
     args.rr_jobs = a.ring ? 0 : std::min<long long>(a.n_jobs, (long long)grid * use);
     *grid_out = grid;
     *block_out = use * 32;
@@ -701,6 +697,17 @@ static void stream_free(ddg_stream* st) {
   delete st;
 }
 
+// Blocks that the pool's lanes make in the lane-per-thread kernels, one to an SM of the default
+// shape: what a pool of `lanes` fills of the GPU.
+static int lane_blocks(const ddg_solver* s) { return (s->lanes + s->block - 1) / s->block; }
+
+// Searches a stream of this solver can have under way.
+static long long stream_searches(const ddg_solver* s) {
+  if (!s->by_warp) return s->lanes;
+  const WarpShape shape = warp_shape(stream_sms(s->sms, lane_blocks(s)), s->lanes, 0, true);
+  return (long long)shape.grid * shape.warps;
+}
+
 // Launches the stream kernel unless it is running; it ends by itself once its lanes found
 // no deal for idle_timeout_s, or once the stream is closing and every deal is done.
 static int stream_kernel(ddg_stream* st) {
@@ -734,7 +741,7 @@ static int stream_kernel(ddg_stream* st) {
     a.hint20 = st->d_hint;
   }
   *(volatile int*)s->h_stop = 0;
-  int rc = launch_batch(s, a, st->kstream, st->guide ? s->sms - 2 : s->sms, &st->grid, &st->block);
+  int rc = launch_batch(s, a, st->kstream, stream_sms(s->sms, lane_blocks(s)), &st->grid, &st->block);
   if (rc) return rc;
   CUDA_TRY(cudaEventRecord(st->kdone, st->kstream));
   st->launched = true;
@@ -751,7 +758,7 @@ int ddg_stream_open_guided(ddg_solver* s, int ring_slots, double idle_timeout_s,
   if (!out) return fail(DDG_E_ARG, "null output");
   *out = nullptr;
   if (!s) return fail(DDG_E_ARG, "null solver");
-  if (guide && (s->lanes + s->block - 1) / s->block > s->sms - 2)
+  if (guide && lane_blocks(s) > s->sms - 2)
     return fail(DDG_E_STATE,
                 "a guided stream needs SMs the solver leaves free for the guide's kernels: create the solver "
                 "with lanes <= (SMs - 2) * block = %d",
@@ -766,11 +773,7 @@ int ddg_stream_open_guided(ddg_solver* s, int ring_slots, double idle_timeout_s,
   st->s = s;
   st->slots = ring_slots;
   st->idle_timeout_s = idle_timeout_s > 0 ? idle_timeout_s : 30;
-  // Admission by TT memory: a deal's jobs each need a lane (and its TT); at most two jobs
-  // per lane are admitted, one running and one waiting.
-  st->admit = (long long)s->lanes * 2 / s->cfg.jobs_per_deal;
-  if (st->admit > ring_slots) st->admit = ring_slots;
-  if (st->admit < 1) st->admit = 1;
+  st->admit = std::min<long long>(stream_deals(stream_searches(s), s->cfg.jobs_per_deal), ring_slots);
   st->slot_busy.assign(ring_slots, 0);
   s->streaming = true;
   cudaError_t e = cudaMalloc(&st->d_ring, (size_t)ring_slots * 32);

@@ -16,17 +16,17 @@
 // batch_kernel stays for helping and for its own options.
 #pragma once
 #include "ddg_kernel.cuh"
+#include "ddg_shape.hpp"
 #include "ddg_warp.cuh"
 
 #ifndef DDG_TT_SIG
 
 namespace ddg {
 
-// Searchers to an SM at most; and at most WARP_FEW in a launch with no more jobs than that,
-// whose kernel may use 104 registers a thread instead of 64. One
-// search alone on an SM 1.31 M against 1.25 M nodes/s; but 16 searchers an SM reached 2.02 G
-// nodes/s where 32 reached 2.30 G, so a launch with more jobs takes 32.
-enum { WARP_MAX = 32, WARP_FEW = 16 };
+// A launch of at most WARP_FEW searchers an SM takes a build with 104 registers a thread instead
+// of 64: one search alone on an SM 1.31 M against 1.25 M nodes/s. At full load 16 searchers an SM
+// reached 2.02 G nodes/s where 32 reached 2.30 G, so a launch with more jobs takes up to WARP_MAX.
+enum { WARP_FEW = 16 };
 
 // A searcher between two slices of a resumable solve (the solver's save area). (The frames
 // below the top go to the lane's stack area.)

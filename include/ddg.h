@@ -204,10 +204,13 @@ int ddg_solve_begin_ex(ddg_solver* s, const uint64_t* d_hands, int64_t n, const 
  * deal's 28-byte record (uint64 0-based submission index, then tricks[strain][declarer],
  * gpu/stream_main.cu:298-302) is available as soon as its last job ends, out of order.
  * ring_slots: power of two, 64..4M (0 = 65,536). Admission: ddg_stream_submit accepts
- * deals only while ring slots are free and at most 2 * lanes jobs are in flight (each job
- * holds a lane and its TT); *accepted says how many of the n it took, in order. Deals wait
- * for nothing but a free lane: requests that arrive while others are on the GPU start as
- * lanes free up. Lanes that find no deal for idle_timeout_s (0 = 30 s) end; the next
+ * deals only while ring slots are free and at most two jobs are in flight for every search
+ * that can be under way (the warp kernel's at most 32 on an SM, or the lanes), one running
+ * and one waiting; *accepted says how many of the n it took, in order. Deals wait for
+ * nothing but a free searcher: requests that arrive while others are on the GPU start as
+ * searchers free up. The kernel stays on the GPU while the stream is open. Of a solver with
+ * at most (SMs - 2) * block lanes it leaves two SMs free for other kernels; of a larger one
+ * it may take every SM. Searchers that find no deal for idle_timeout_s (0 = 30 s) end; the next
  * submit or poll launches the kernel again. While a stream is open the solver's other
  * calls return DDG_E_STATE. Runs on the warp kernel or the block-phase kernel (schedule 0 or
  * 2), helping off. */
@@ -217,7 +220,8 @@ int ddg_stream_open(ddg_solver* s, int ring_slots, double idle_timeout_s, ddg_st
  * device): every submit runs the guide on the new deals before they are published, and
  * each job steps from the guide's NS seed with its lead tried first at the root, as
  * ddg_solve_device_ex. The guide's kernels need SMs the persistent solve kernel leaves
- * free: the solver must have at most (SMs - 2) * block lanes (else DDG_E_STATE). */
+ * free: the solver must have been made with at most (SMs - 2) * block lanes (else
+ * DDG_E_STATE). */
 int ddg_stream_open_guided(ddg_solver* s, int ring_slots, double idle_timeout_s, ddg_guide* guide,
                            ddg_stream** out);
 int ddg_stream_submit(ddg_stream* st, const uint64_t* hands, int64_t n, int64_t* accepted);

@@ -1,13 +1,60 @@
 """What a call reports of its launch is the launch that ran, for the warp kernel (a search to a
 warp) and the lane-per-thread ones (a search to a thread)."""
+import ctypes
+import os
+import subprocess
 import time
 
 import numpy as np
 import pytest
 
-from conftest import load_golden
+from conftest import NATIVE, ROOT, load_golden
 
-pytestmark = pytest.mark.gpu
+
+@pytest.fixture(scope="module")
+def shape_lib():
+    out = os.path.join(NATIVE, "_build", "libshape.so")
+    os.makedirs(os.path.dirname(out), exist_ok=True)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I" + os.path.join(ROOT, "dds_gpu_b200", "csrc"), "-o",
+                    out + ".tmp", os.path.join(NATIVE, "shape.cpp")], check=True)
+    os.replace(out + ".tmp", out)
+    lib = ctypes.CDLL(out)
+    lib.shape_stream_deals.restype = ctypes.c_longlong
+    lib.shape_stream_deals.argtypes = [ctypes.c_longlong, ctypes.c_int]
+    return lib
+
+
+def shape(lib, sms, lanes, jobs, stream=0):
+    grid, warps = ctypes.c_int(), ctypes.c_int()
+    lib.shape_of(sms, lanes, ctypes.c_longlong(jobs), stream, ctypes.byref(grid), ctypes.byref(warps))
+    return grid.value, warps.value
+
+
+@pytest.mark.parametrize("lanes", [512, 2560, 4096, 4736, 75776])
+@pytest.mark.parametrize("sms", [1, 146, 148])
+def test_every_searcher_has_a_table_and_every_sm_its_share(shape_lib, lanes, sms):
+    for jobs in (1, 2, sms - 1, sms, sms + 1, 16 * sms, 16 * sms + 1, 32 * sms, 10 ** 6):
+        if jobs < 1:
+            continue
+        grid, warps = shape(shape_lib, sms, lanes, jobs)
+        assert 1 <= grid <= sms and 1 <= warps <= 32 and grid * warps <= lanes
+        assert grid == min(sms, jobs)
+        assert warps == min(32, lanes // grid, -(-jobs // grid))  # enough for the jobs, where they fit
+    grid, warps = shape(shape_lib, sms, lanes, 0, 1)
+    assert grid == sms and warps == min(32, lanes // sms)
+
+
+@pytest.mark.parametrize("blocks,want", [(1, 146), (32, 146), (146, 146), (147, 147), (148, 148), (500, 148)])
+def test_a_stream_leaves_what_its_pool_leaves_up_to_two(shape_lib, blocks, want):
+    assert shape_lib.shape_stream_sms(148, blocks) == want
+
+
+def test_admission_is_two_jobs_a_search(shape_lib):
+    assert shape_lib.shape_stream_deals(4736, 5) == 1894 and shape_lib.shape_stream_deals(4736, 20) == 473
+    assert shape_lib.shape_stream_deals(4096, 5) == 1638 and shape_lib.shape_stream_deals(3, 20) == 1
+
+
+# ---- on the GPU ------------------------------------------------------------------------------
 
 
 def sm_count():
@@ -22,6 +69,7 @@ def solve(solver, hands):
     return solver.solve_device(d_h.data_ptr(), len(hands), d_o.data_ptr())
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("deals", [1, 31, 600, 4096])
 def test_batch(ddg, deals):
     hands = load_golden("k6_4096.npz")["hands"][:deals]
@@ -35,6 +83,7 @@ def test_batch(ddg, deals):
     assert (st["grid"], st["block"], st["lanes"]) == (min(sms, jobs), 32 * warps, min(sms, jobs) * warps)
 
 
+@pytest.mark.gpu
 def test_lane_per_thread(ddg):
     s = ddg.Solver(lanes=1024, free_below=96)
     try:
@@ -44,6 +93,7 @@ def test_lane_per_thread(ddg):
     assert (st["grid"], st["block"], st["lanes"]) == (2, 512, 1024)
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("kw", [{}, {"lanes": 1024, "free_below": 96}])
 def test_stream(ddg, kw):
     g = load_golden("k4_120.npz")
@@ -61,3 +111,41 @@ def test_stream(ddg, kw):
         s.close()
     want = (2, 512, 1024) if kw else (sm_count(), 1024, 32 * sm_count())
     assert seen == 20 and (stats["grid"], stats["block"], stats["lanes"]) == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw,searches", [({}, 148 * 32), ({"jobs_per_deal": 20}, 148 * 32), ({"lanes": 146 * 512}, 146 * 32),
+                                         ({"lanes": 512}, 146 * 3), ({"lanes": 1024, "free_below": 96}, 1024)])
+def test_stream_capacity(ddg, kw, searches):
+    """Two jobs for every search that can be under way, whatever the pool's size."""
+    if sm_count() != 148:
+        pytest.skip("figures for 148 SMs")
+    s = ddg.Solver(**kw)
+    try:
+        st = ddg.Stream(s, ring_slots=65536, idle_timeout_s=1)
+        assert st.capacity == searches * 2 // s.jobs_per_deal
+        stats = st.close()
+        assert stats["lanes"] == searches
+    finally:
+        s.close()
+
+
+@pytest.mark.gpu
+def test_other_kernels_run_beside_a_stream(ddg):
+    """A stream of (SMs - 2) * 512 lanes, busy for minutes, leaves SMs on which another solver's
+    call ends."""
+    hard = load_golden("k13_24.npz")["hands"]
+    g = load_golden("k5_120.npz")
+    s, other = ddg.Solver(lanes=(sm_count() - 2) * 512), ddg.Solver(lanes=512)
+    try:
+        assert (other.solve(g["hands"]) == g["tricks"]).all()  # kernels loaded, buffers there
+        st = ddg.Stream(s, ring_slots=64, idle_timeout_s=5)
+        assert st.submit(hard) == 24
+        t0 = time.time()
+        assert (other.solve(g["hands"]) == g["tricks"]).all()
+        assert st.in_flight > 0 and time.time() - t0 < 20
+        stats = st.close(drain=False)
+        assert stats["grid"] == sm_count() - 2
+    finally:
+        s.close()
+        other.close()
