@@ -94,8 +94,12 @@ def tune(d_hands, n, window_s, torch, log=print):
 def run_batch(cfg, d_hands, n, limit_s, torch, tables=False, help=False):
     """The whole set as one graph-launched persistent solve; completion-time tail (and the
     tables, (n, 5, 4) uint8 with 255 = unsolved, under "tables" when asked)."""
-    s = Solver(tt_log2=cfg["tt_log2"], lanes=cfg["lanes"], block=cfg["block"], min_blocks=cfg["min_blocks"],
-               jobs_per_deal=5, schedule=cfg["schedule"], help=1 if help and cfg["schedule"] != 1 else 0,
+    help = help and cfg["schedule"] != 1
+    # Helping runs on the lane-per-thread kernel: a pool tuned for the warp kernel (a search to a
+    # warp, at most 32 on an SM) would fill few of its blocks, so it takes every lane instead.
+    by_warp = (cfg["block"], cfg["min_blocks"], cfg["schedule"]) == (512, 1, 0)
+    s = Solver(tt_log2=cfg["tt_log2"], lanes=0 if help and by_warp else cfg["lanes"], block=cfg["block"],
+               min_blocks=cfg["min_blocks"], jobs_per_deal=5, schedule=cfg["schedule"], help=1 if help else 0,
                time_limit_s=limit_s)
     try:
         d_out = torch.empty(n * 20, dtype=torch.uint8, device=d_hands.device)

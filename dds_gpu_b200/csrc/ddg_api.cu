@@ -45,6 +45,7 @@ struct KVariant;
 struct ddg_solver {
   ddg_config cfg;
   int device = 0, lanes = 0, block = 128, sms = 0;
+  int blocks = 0;  // that the lanes asked for make in the lane-per-thread kernels, one to an SM of the default shape
   const KVariant* variant = nullptr;
   bool by_warp = false;  // searched by warp_kernel (see warp_route), else by the variant's kernel
   TTBucket* tt = nullptr;
@@ -266,13 +267,16 @@ int ddg_solver_create(const ddg_config* cfg_in, ddg_solver** out) {
     }
     lanes = (long long)(budget / per_lane);
   }
-  lanes = lanes / cfg.block * cfg.block;
-  if (lanes <= 0) {
+  s->by_warp = warp_route(cfg);
+  s->blocks = (int)(lanes / cfg.block);
+  if (s->blocks <= 0) {
     delete s;
     return fail(DDG_E_MEMORY, "no room for one block of lanes");
   }
-  s->lanes = (int)lanes;
-  s->by_warp = warp_route(cfg);
+  // A searcher of the warp kernel has a table to itself and there are no more than 32 to an SM, so
+  // of the lanes asked for no more are allocated (75,776 tables were 24.3 GB, of which 1.5 in use).
+  s->lanes = (int)(s->by_warp ? warp_tables(s->sms, lanes) : (long long)s->blocks * cfg.block);
+  lanes = s->lanes;
 #ifndef DDG_TT_SIG
   if (s->by_warp) {
     const void* kernels[] = {(const void*)warp_kernel<WARP_MAX, false>, (const void*)warp_kernel<WARP_FEW, false>,
@@ -290,7 +294,7 @@ int ddg_solver_create(const ddg_config* cfg_in, ddg_solver** out) {
   size_t st_bytes = (size_t)lanes * sizeof(Frame) * STACK_DEPTH;
 #ifndef DDG_TT_SIG
   if (s->by_warp)  // a searcher's frames leave shared memory only between slices
-    st_bytes = (size_t)std::min<long long>(lanes, (long long)s->sms * WARP_MAX) * sizeof(WarpFrame) * STACK_DEPTH;
+    st_bytes = (size_t)lanes * sizeof(WarpFrame) * STACK_DEPTH;
 #endif
   e = cudaMalloc(&s->tt, tt_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&s->stacks, st_bytes);
@@ -579,7 +583,7 @@ int ddg_solve_begin_ex(ddg_solver* s, const uint64_t* d_hands, int64_t n, const 
   if (!s->save) {
     size_t bytes = (size_t)s->lanes * sizeof(LaneSave);
 #ifndef DDG_TT_SIG
-    if (s->by_warp) bytes = (size_t)std::min(s->lanes, s->sms * WARP_MAX) * sizeof(WarpSave);
+    if (s->by_warp) bytes = (size_t)s->lanes * sizeof(WarpSave);
 #endif
     cudaError_t e = cudaMalloc(&s->save, bytes);
     if (e != cudaSuccess) {
@@ -697,14 +701,10 @@ static void stream_free(ddg_stream* st) {
   delete st;
 }
 
-// Blocks that the pool's lanes make in the lane-per-thread kernels, one to an SM of the default
-// shape: what a pool of `lanes` fills of the GPU.
-static int lane_blocks(const ddg_solver* s) { return (s->lanes + s->block - 1) / s->block; }
-
 // Searches a stream of this solver can have under way.
 static long long stream_searches(const ddg_solver* s) {
   if (!s->by_warp) return s->lanes;
-  const WarpShape shape = warp_shape(stream_sms(s->sms, lane_blocks(s)), s->lanes, 0, true);
+  const WarpShape shape = warp_shape(stream_sms(s->sms, s->blocks), s->lanes, 0, true);
   return (long long)shape.grid * shape.warps;
 }
 
@@ -741,7 +741,7 @@ static int stream_kernel(ddg_stream* st) {
     a.hint20 = st->d_hint;
   }
   *(volatile int*)s->h_stop = 0;
-  int rc = launch_batch(s, a, st->kstream, stream_sms(s->sms, lane_blocks(s)), &st->grid, &st->block);
+  int rc = launch_batch(s, a, st->kstream, stream_sms(s->sms, s->blocks), &st->grid, &st->block);
   if (rc) return rc;
   CUDA_TRY(cudaEventRecord(st->kdone, st->kstream));
   st->launched = true;
@@ -758,7 +758,7 @@ int ddg_stream_open_guided(ddg_solver* s, int ring_slots, double idle_timeout_s,
   if (!out) return fail(DDG_E_ARG, "null output");
   *out = nullptr;
   if (!s) return fail(DDG_E_ARG, "null solver");
-  if (guide && lane_blocks(s) > s->sms - 2)
+  if (guide && s->blocks > s->sms - 2)
     return fail(DDG_E_STATE,
                 "a guided stream needs SMs the solver leaves free for the guide's kernels: create the solver "
                 "with lanes <= (SMs - 2) * block = %d",

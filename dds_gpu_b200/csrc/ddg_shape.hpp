@@ -7,6 +7,9 @@ namespace ddg {
 // Searchers to an SM at most.
 enum { WARP_MAX = 32 };
 
+// Tables of a pool of `lanes` lanes: those that a launch can use.
+inline long long warp_tables(int sms, long long lanes) { return std::min<long long>(lanes, (long long)sms * WARP_MAX); }
+
 struct WarpShape {
   int grid, warps;  // blocks, one to an SM; searchers to a block
 };

@@ -39,14 +39,15 @@ typedef struct ddg_guide ddg_guide; /* the learned guide (below) */
  * TIME_LIMIT (gpu/gpu_main.cu:247).
  *
  * Two kernels search. With the defaults it is the warp kernel: a warp to a search, at most 32
- * searches on an SM (so of a full pool of lanes at most 32 * SMs are in use). Helping, another
+ * searches on an SM (so of the lanes asked for at most 32 * SMs are allocated). Helping, another
  * block shape or schedule, and any value given to free_below, free_steps, free_pack,
  * phase_spread, cheap_limit or flat_moves ask for the lane-per-thread kernels, which
  * these options belong to (a thread to a search, block lanes on an SM); so does
  * libddg_sig.so. Tricks are the same, and with help = 0 so are the nodes of every job. */
 typedef struct ddg_config {
   int tt_log2;          /* TT buckets per lane = 2^tt_log2, 9..20; default 10 (320 KB per lane) */
-  int lanes;            /* solver lanes, one TT each: the most searches at once; default: fill the GPU */
+  int lanes;            /* solver lanes, one TT each: the most searches at once; default: fill the GPU.
+                           At least one block's; the lane-per-thread kernels' pools are whole blocks */
   int block;            /* threads per block (lanes per block): 64, 128, 256 or 512; default 512
                            (64 to 256: the lane-per-thread kernels) */
   int jobs_per_deal;    /* 5 = one job per strain, the 4 leads share a TT; 20 = one per lead */
@@ -127,7 +128,8 @@ void ddg_config_default(ddg_config* cfg);
 
 /* Creates a solver on cfg->device: allocates the per-lane TTs and search stacks once
  * (lanes * (320 << tt_log2) bytes, and stacks: 6.9 KB for each of the warp kernel's at
- * most 32 * SMs searchers, or 2.6 KB a lane) and clears the TT tags. */
+ * most 32 * SMs lanes, or 2.6 KB a lane) and clears the TT tags. A pool whose lanes asked
+ * for do not fit the memory is refused, also where fewer would be allocated. */
 int ddg_solver_create(const ddg_config* cfg, ddg_solver** out);
 void ddg_solver_destroy(ddg_solver* s);
 /* Lanes actually allocated, and the bytes of device memory the pool holds. */

@@ -8,6 +8,7 @@ void shape_of(int sms, int lanes, long long n_jobs, int stream, int* grid, int* 
   *grid = s.grid;
   *warps = s.warps;
 }
+long long shape_tables(int sms, long long lanes) { return ddg::warp_tables(sms, lanes); }
 int shape_stream_sms(int sms, int blocks) { return ddg::stream_sms(sms, blocks); }
 long long shape_stream_deals(long long searches, int jpd) { return ddg::stream_deals(searches, jpd); }
 }

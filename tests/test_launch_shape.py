@@ -19,6 +19,8 @@ def shape_lib():
                     out + ".tmp", os.path.join(NATIVE, "shape.cpp")], check=True)
     os.replace(out + ".tmp", out)
     lib = ctypes.CDLL(out)
+    lib.shape_tables.restype = ctypes.c_longlong
+    lib.shape_tables.argtypes = [ctypes.c_int, ctypes.c_longlong]
     lib.shape_stream_deals.restype = ctypes.c_longlong
     lib.shape_stream_deals.argtypes = [ctypes.c_longlong, ctypes.c_int]
     return lib
@@ -52,6 +54,16 @@ def test_a_stream_leaves_what_its_pool_leaves_up_to_two(shape_lib, blocks, want)
 def test_admission_is_two_jobs_a_search(shape_lib):
     assert shape_lib.shape_stream_deals(4736, 5) == 1894 and shape_lib.shape_stream_deals(4736, 20) == 473
     assert shape_lib.shape_stream_deals(4096, 5) == 1638 and shape_lib.shape_stream_deals(3, 20) == 1
+
+
+def test_tables_are_those_a_launch_can_use(shape_lib):
+    for lanes, want in ((512, 512), (600, 600), (4735, 4735), (4736, 4736), (4737, 4736), (75776, 4736), (1 << 34, 4736)):
+        assert shape_lib.shape_tables(148, lanes) == want
+        # with fewer tables a launch of any size is the same as with all that were asked for
+        for jobs in (1, 147, 149, 2000, 4700, 10 ** 6):
+            assert shape(shape_lib, 148, want, jobs) == shape(shape_lib, 148, min(lanes, 10 ** 6), jobs)
+        for sms in (146, 148):
+            assert shape(shape_lib, sms, want, 0, 1) == shape(shape_lib, sms, min(lanes, 10 ** 6), 0, 1)
 
 
 # ---- on the GPU ------------------------------------------------------------------------------
@@ -149,3 +161,47 @@ def test_other_kernels_run_beside_a_stream(ddg):
     finally:
         s.close()
         other.close()
+
+
+@pytest.mark.gpu
+def test_pool(ddg):
+    """The warp kernel's pool has a table a searcher; the other kernels' pools are whole blocks."""
+    most = 32 * sm_count()
+    tt = 320 << 10
+    for kw, lanes in (({}, most), ({"lanes": 4 * most}, most), ({"lanes": most}, most), ({"lanes": 700}, 700),
+                      ({"lanes": 700, "free_below": 96}, 512), ({"lanes": 4 * most, "free_below": 96}, 4 * most // 512 * 512)):
+        s = ddg.Solver(**kw)
+        try:
+            assert s.lanes == lanes and lanes * tt <= s.nbytes < lanes * (tt + 8192)
+            g = load_golden("k5_120.npz")
+            assert (s.solve(g["hands"]) == g["tricks"]).all()
+        finally:
+            s.close()
+    for kw in ({"lanes": 511}, {"lanes": 511, "free_below": 96}, {"lanes": 10 ** 7}):  # less than a block; 3.3 TB
+        with pytest.raises(ddg.DDGError):
+            ddg.Solver(**kw)
+
+
+@pytest.mark.gpu
+def test_tuned_pool_with_helping(ddg):
+    """A setting tuned on the warp kernel, run with helping: on every lane of the other kernel."""
+    import torch
+    from dds_gpu_b200 import autotune
+    g = load_golden("k6_120.npz")
+    d_h = torch.from_numpy(g["hands"].view(np.int64)).cuda()
+    made = []
+
+    class Recorded(ddg.Solver):
+        def __init__(self, **kw):
+            super().__init__(**kw)
+            made.append(self.lanes)
+
+    solver, autotune.Solver = autotune.Solver, Recorded
+    try:
+        cfg = {"block": 512, "min_blocks": 1, "schedule": 0, "tt_log2": 10, "lanes": 32 * sm_count()}
+        for help in (False, True):
+            rep = autotune.run_batch(cfg, d_h, 120, 60.0, torch, tables=True, help=help)
+            assert (rep["tables"] == g["tricks"]).all()
+    finally:
+        autotune.Solver = solver
+    assert made == [32 * sm_count(), 512 * sm_count()]
