@@ -9,8 +9,9 @@ The tuner sweeps the launch shape (512 threads x 1 block or 256 x 2 per SM), sol
 and the kernel's stage schedule (block phases or per-warp queues) at one TT size; each
 candidate runs a short resumable slice of the same set and is scored by the search nodes
 it covers per second. The TT size (2^9..2^12 buckets per lane) is then the largest that
-fits beside the chosen lanes (tune() says why node rates do not rank TT sizes). The
-chosen setting then solves the whole set as one CUDA-graph launch of the persistent kernel
+fits beside the chosen lanes (tune() says why node rates do not rank TT sizes). Lane counts
+that make the same pool (of the warp kernel, which 512 x 1 with block phases runs: at most 32
+an SM) are one candidate. The chosen setting then solves the whole set as one CUDA-graph launch of the persistent kernel
 (optionally with helping: idle lanes split the last hard jobs in shared TTs; --help-lanes),
 with per-job completion times for the tail.
 """
@@ -30,14 +31,17 @@ SCHEDULES = (0, 1)
 SEED = 7
 
 
-def measure(cfg, d_hands, n, window_s, torch):
-    """Search nodes and finished jobs per second in one slice of `window_s` after a 1 s
+def measure(cfg, d_hands, n, window_s, torch, seen=()):
+    """Search nodes and finished jobs per second, and the pool's lanes (None for the rates of a
+    pool whose lanes are among `seen`), in one slice of `window_s` after a 1 s
     warm-up slice. Nodes per second scores a setting: a short slice's finished jobs
     favour settings that turn over the smallest jobs quickly, while the batch's end is set
     by how fast the search work as a whole goes."""
     s = Solver(tt_log2=cfg["tt_log2"], lanes=cfg["lanes"], block=cfg["block"], min_blocks=cfg["min_blocks"],
                jobs_per_deal=5, schedule=cfg["schedule"])
     try:
+        if s.lanes in seen:
+            return None, None, s.lanes
         d_out = torch.empty(n * 20, dtype=torch.uint8, device=d_hands.device)
         s.begin(d_hands.data_ptr(), n, d_out.data_ptr())
         _, warm = s.resume(1.0)
@@ -57,15 +61,20 @@ def tune(d_hands, n, window_s, torch, log=print):
     TT sizes are not comparable (a larger table answers more positions, so the same job
     takes fewer nodes: 1.5-2.5x fewer for hard 13-card jobs at 2^12 than at 2^10, at about
     the same node rate), so they are measured and reported, not used to rank."""
-    results = []
+    results, seen = [], {}
     base_tt = 10 if 10 in TT_LOG2 else TT_LOG2[0]
     for (block, minb), lanes, sch in itertools.product(SHAPES, LANES, SCHEDULES):
         cfg = {"block": block, "min_blocks": minb, "lanes": lanes, "tt_log2": base_tt, "schedule": sch}
+        pools = seen.setdefault((block, minb, sch), set())
         try:
-            rate, jobs_rate, used = measure(cfg, d_hands, n, window_s, torch)
+            rate, jobs_rate, used = measure(cfg, d_hands, n, window_s, torch, pools)
         except DDGError as e:  # e.g. the TTs do not fit
             log(f"  {cfg}: {e}")
             continue
+        if rate is None:
+            log(f"  {cfg}: the pool of {used} lanes again")
+            continue
+        pools.add(used)
         cfg["lanes"] = used
         cfg["jobs_per_s"] = jobs_rate
         results.append((rate, cfg))
