@@ -290,7 +290,7 @@ class Stream:
 
     def __init__(self, solver, ring_slots=0, idle_timeout_s=0.0, guide=None):
         """`guide`: a Guide on the solver's device whose seeds and root leads steer every
-        deal's search (the solver then needs at most (SMs - 2) * block lanes)."""
+        deal's search (the solver then has to be made with at most (SMs - 2) * block lanes)."""
         self._lib = solver._lib
         self._h = P()
         _check(self._lib.ddg_last_error,

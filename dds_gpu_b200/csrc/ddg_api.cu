@@ -82,9 +82,11 @@ struct ddg_solver {
 };
 
 // Pinned staging for a host-memory call on at most IO_DEALS deals: its copies and its launch
-// are queued together and waited for once. Pageable copies wait one by one, some 10 us each
-// (the call for one lead of a five-card ending: 173 us with four waits). Larger calls copy
-// straight from and to the caller's memory.
+// are queued together and waited for once. Pageable copies wait one by one, which larger calls'
+// do, straight from and to the caller's memory. Measured on three-card deals, staged against
+// pageable: 1 deal 134 against 152 us, 128: 186 / 203, 1,024: 395 / 409, 2,048: 609 / 624, 4,096:
+// 1,031 / 1,053, 16,384: 3,739 / 3,755 us, 65,536: 14.44 / 14.41 ms. Some 15 us at each size, 4 % of
+// the call at 1,024; for more deals the buffer (107 KB a solver) would grow for less.
 enum { IO_DEALS = 1024 };
 struct HostIo {
   unsigned long long counters[CNT_WORDS];

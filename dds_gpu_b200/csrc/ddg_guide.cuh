@@ -221,11 +221,11 @@ __device__ __forceinline__ void tile_features(const MlpArgs& g, int64_t m0, unsi
 // time): 32 warps an SM, 0.52 ms for the rows below against 0.55 with 16. Two CTAs an SM
 // with a ring of their own each, 40 or 32 KB of it, were slower (0.90, 0.60 ms: the weights
 // come too late). A training step's 32 tiles use 32 SMs and are bound by one tile's chain;
-// 32 warps (64 registers, a few spilled) changed nothing there. Measured, against one kernel per layer with its activations in HBM and its
-// weights loaded through registers, chunk by chunk: the 400,000 rows of 20,000 deals 0.52
-// against 14.2 ms; a step of 4,096 rows with its gradients copied out 0.27 against 1.76 ms
-// (5 launches against 28; the three weight gradients 160 us each there, two CTAs walking
-// the whole batch).
+// 32 warps (64 registers, a few spilled) changed nothing there. Measured, against one kernel
+// per layer with its activations in HBM and its weights loaded through registers, chunk by
+// chunk: the 400,000 rows of 20,000 deals 0.52 against 14.2 ms; a step of 4,096 rows with its
+// gradients copied out 0.27 against 1.76 ms (5 launches against 28; the three weight gradients
+// 160 us each there, two CTAs walking the whole batch).
 template <bool TRAIN>
 __global__ void __launch_bounds__(MLP_THREADS<TRAIN>, 1) mlp_rows(MlpArgs g) {
   constexpr int THREADS = MLP_THREADS<TRAIN>, COLS = HID / (THREADS / TILE_M);  // a thread's columns

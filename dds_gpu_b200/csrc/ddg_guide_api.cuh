@@ -231,6 +231,3 @@ static int guide_predict_on(ddg_guide* g, const uint64_t* d_hands, int64_t n, in
   return DDG_OK;
 }
 
-extern "C" {
-
-}  // extern "C"

@@ -31,10 +31,10 @@ DDG_W u32 w_max(u32 v) { return __reduce_max_sync(0xFFFFFFFFu, v); }
 DDG_W u32 w_min(u32 v) { return __reduce_min_sync(0xFFFFFFFFu, v); }
 DDG_W u32 w_add(u32 v) { return __reduce_add_sync(0xFFFFFFFFu, v); }
 DDG_W bool w_any(bool p) { return __any_sync(0xFFFFFFFFu, p); }
-// The same value in all threads, said so to the compiler: ptxas follows uniformity from a
-// vote, a reduction, a shuffle from one thread or a shared-memory load at a uniform
-// address, but not around a loop. Where it cannot tell that a branch is uniform it guards
-// every collective behind it (a divergence test, and a slow path of some ten instructions).
+// The same value in all threads, said so to the compiler: what goes around the search's loops
+// passes through this shuffle, and branches on it through a vote, so that it can see that the
+// warp stays together. Measured against the same build without them (hard 13-card deals): one
+// search alone on an SM 1.35 against 1.17 M nodes/s, every SM full 2.38 against 2.20 G.
 DDG_W u32 w_uni(u32 v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
 DDG_W void w_sync() { __syncwarp(); }
 DDG_W int w_top(u32 x) { return 31 - __clz((int)x); }   // highest set bit, -1 for 0
@@ -1289,7 +1289,7 @@ DDG_W void w_run(WarpState& w, const WarpIds& id, WarpMem& sm, Env& env) {
       if (w_fault(w, id, sm)) return;
       w_play(w, id, sm, key);
     }
-    if (w_any(stopped)) return;  // (a return out of both loops would cost ptxas the proof)
+    if (w_any(stopped)) return;
   }
 }
 

@@ -5,9 +5,8 @@
 // barrier in the loop and the SM's schedulers always have the other warps to issue from.
 // Searcher w of block b owns the TT slice, stack area and save slot number b * warps + w.
 //
-// What bounds it: on a full SM the integer pipe and instruction fetch (about 2.6 instructions
-// a cycle; the code a node may run is some 36 KB, the SM's instruction cache holds 32 KB);
-// alone on an SM one warp's chain of instructions, 1,500 cycles a node, of which the
+// What bounds it: on a full SM the integer pipe (85 % of its cycles busy) and instruction fetch
+// (2.6 of 11.2 stall cycles an issue; 2.76 instructions a cycle); alone on an SM one warp's chain of instructions, 1,500 cycles a node, of which the
 // table's memory is a twentieth. Measured against batch_kernel (block phases, 512 lanes to
 // an SM): random 13-card deals with every SM full 2.36 against 0.70 G nodes/s; one job
 // alone on an SM 1.3 M against 0.15 M nodes/s; 240 quick 13-card deals 75 against 1,381 ms;
@@ -24,8 +23,10 @@
 namespace ddg {
 
 // A launch of at most WARP_FEW searchers an SM takes a build with 104 registers a thread instead
-// of 64: one search alone on an SM 1.31 M against 1.25 M nodes/s. At full load 16 searchers an SM
-// reached 2.02 G nodes/s where 32 reached 2.30 G, so a launch with more jobs takes up to WARP_MAX.
+// of 64. Measured on hard 13-card deals, nodes/s of the GPU with n searches on each of 148 SMs,
+// this build against the other: n = 1: 200 against 193 M, 4: 784 / 748, 8: 1,375 / 1,348, 12: 1,817
+// / 1,772, 16: 2,045 / 2,004. From 17 on the other's further searches are worth more than 16 of
+// these with the rest waiting (2,050 M): 17: 2,073, 20: 2,172, 24: 2,263, 32: 2,384.
 enum { WARP_FEW = 16 };
 
 // A searcher between two slices of a resumable solve (the solver's save area). (The frames
@@ -54,10 +55,11 @@ struct WarpBlock {
 };
 inline size_t warp_smem(int warps) { return sizeof(WarpBlock) + sizeof(WarpMem) * (size_t)(warps - 1); }
 
-// Is the slice over, or the solve stopped by the host? In one thread. The host's flag is a
-// read over the bus, and the GPU does about 1.15 M of those a second however many SMs ask: a
-// read by every searcher every 1,024 nodes held the whole GPU at 1.18 G nodes/s. So one
-// question of a block in 64 reads it, and the others see what that one found.
+// Is the slice over, or the solve stopped by the host? In one thread, asked at the first trick
+// start after 256 nodes. The host's flag is a read over the bus, and the GPU does about 1.15 M
+// of those a second however many SMs ask: one read by every searcher each 1,024 nodes held the
+// whole GPU at 1.18 G nodes/s. So one question of a block in 64 reads it, and the others see
+// what that one found.
 __device__ __forceinline__ int warp_ask(WarpBlock* sh, u64 t_end) {
   const BatchArgs& a = sh->args;
   volatile int* halt = &sh->halt;
@@ -141,14 +143,13 @@ __device__ __forceinline__ void warp_job_done(WarpBlock* sh, WarpJob* j) {
   }
 }
 
-// STREAM: the jobs come from a stream's ring. (A kernel of its own: what it takes to wait for
-// deals would cost every other launch the compiler's proof that warps stay together.)
+// STREAM: the jobs come from a stream's ring. (A kernel of its own, so that other launches carry
+// nothing of the waiting for deals.)
 template <bool STREAM>
 struct WarpEnv {
   WarpBlock* sh;
   TTBucket* tt;
   u64 t_end;
-  long long lane;
   int wid;
 
   __device__ __forceinline__ TTBucket* table() { return tt; }
@@ -198,8 +199,7 @@ struct WarpEnv {
     }
     if (id.t == 0) j.stage = got == 0 ? ST_IDLE : ST_TAKE;
     if (got != 1) return false;
-    // By all threads, which write the same values: nested branches in a one-thread region
-    // would cost the compiler its proof that the warp is together afterwards.
+    // By all threads, which write the same values: no branch takes the warp apart here.
     warp_set_job(a, j, (unsigned long long)w_uni((u32)(job >> 32)) << 32 | w_uni((u32)job), id.t);
     __syncwarp();
     const long long row = STREAM ? (j.deal & a.ring_mask) : j.deal;
@@ -285,7 +285,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) warp_kernel(BatchArgs a) {
   env.sh = &sh;
   env.tt = a.tt + (lane << a.tt_log2);
   env.t_end = t_end;
-  env.lane = lane;
   env.wid = wid;
   if (sm.job.stage != ST_IDLE) w_run(w, id, sm, env);
   __syncwarp();

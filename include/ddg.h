@@ -262,8 +262,8 @@ int ddg_ns_tricks(ddg_solver* s, const uint64_t* hands4, int strain, int leader,
  * b1[256], W2[256][256], b2[256], W3[80][256] (outputs padded to 80), b3[80]. An example
  * is (deal, strain, declarer) = index deal*20 + strain*4 + declarer, leader = declarer+1. */
 int64_t ddg_guide_param_count(void);
-/* max_rows: examples per training step / inference pass, a multiple of 128. params: the
- * initial parameters (NULL = zeros). */
+/* max_rows: examples per training step, a multiple of 128 (inference takes any number).
+ * params: the initial parameters (NULL = zeros). */
 int ddg_guide_create(int device, int max_rows, const float* params, ddg_guide** out);
 void ddg_guide_destroy(ddg_guide* g);
 int ddg_guide_get_params(ddg_guide* g, float* params);
