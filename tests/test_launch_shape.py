@@ -205,3 +205,31 @@ def test_tuned_pool_with_helping(ddg):
     finally:
         autotune.Solver = solver
     assert made == [32 * sm_count(), 512 * sm_count()]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [{}, {"free_below": 96}])
+def test_guided_stream(ddg, kw):
+    """The guide's kernels get the two SMs that a stream leaves, beside the warp kernel and beside
+    the lane-per-thread one (any of whose options asks for it)."""
+    from dds_gpu_b200 import guide as ddg_guide
+    params = ddg_guide.load_weights()
+    if params is None:
+        pytest.skip("no guide weights file")
+    g = load_golden("k7_120.npz")
+    guide, s = ddg.Guide(max_rows=4096, params=params), ddg.Solver(lanes=(sm_count() - 2) * 512, **kw)
+    try:
+        st = ddg.Stream(s, ring_slots=64, idle_timeout_s=2, guide=guide)
+        got, sent, seen, t0 = np.full_like(g["tricks"], 255), 0, 0, time.time()
+        while seen < 120 and time.time() - t0 < 60:
+            if sent < 120:
+                sent += st.submit(g["hands"][sent:])
+            idx, tab = st.poll()
+            got[idx.astype(int)] = tab
+            seen += len(idx)
+        stats = st.close()
+    finally:
+        s.close()
+        guide.close()
+    assert seen == 120 and (got == g["tricks"]).all()
+    assert stats["grid"] == sm_count() - 2 and stats["block"] == (512 if kw else 1024)
