@@ -106,9 +106,9 @@ __device__ __forceinline__ int warp_stream_look(WarpBlock* sh, unsigned long lon
 // The next job of a batch, in one thread: 1 taken, 0 none left, -1 stopped.
 __device__ __forceinline__ int warp_next_job(WarpBlock* sh, const WarpJob& j, int wid, u64 t_end, unsigned long long& job) {
   const BatchArgs& a = sh->args;
-  // A searcher that has not searched in this launch takes a job unasked: a slice that is over
+  // A searcher that has not searched in this launch takes a job all the same: a slice that is over
   // before the kernel has started up still gets on, by 256 nodes a searcher or a job.
-  if (j.nodes && warp_ask(sh, t_end)) return -1;
+  if (warp_ask(sh, t_end) && j.nodes) return -1;
   // The first job of the launch is dealt round-robin over the blocks, so that a small batch
   // spreads over every SM; later ones come from the shared counter.
   const long long rr = (long long)wid * gridDim.x + blockIdx.x;
