@@ -48,7 +48,7 @@ struct WarpBlock {
   int idle_exit;   // stream: waiting searchers end (1: nothing will come, 2: stopped by the host)
   unsigned polls;  // stream: looks at the ring
   int halt;        // stopped by the host
-  unsigned asks;   // questions whether to stop
+  unsigned turn;   // of the clock, in which the host's flag was last read
   int running;     // searchers that did not end idle
   unsigned long long nodes, jobs_done, total[WCNT_COUNT];
   WarpMem warp[1];  // as many as the block has warps
@@ -56,14 +56,18 @@ struct WarpBlock {
 inline size_t warp_smem(int warps) { return sizeof(WarpBlock) + sizeof(WarpMem) * (size_t)(warps - 1); }
 
 // Is the slice over, or the solve stopped by the host? In one thread, asked at the first trick
-// start after 256 nodes. The host's flag is a read over the bus, and the GPU does about 1.15 M
-// of those a second however many SMs ask: one read by every searcher each 1,024 nodes held the
-// whole GPU at 1.18 G nodes/s. So one question of a block in 64 reads it, and the others see
-// what that one found.
+// start after 256 nodes and before a job is taken. The host's flag is a read over the bus, and the
+// GPU does about 1.15 M of those a second however many SMs ask (one read by every searcher each
+// 1,024 nodes held the whole GPU at 1.18 G nodes/s). So a block reads it once in 2^FLAG_SHIFT
+// clock cycles, about a millisecond: the first question after that does, and the others see what
+// it found. Counted in questions instead, one in 64, it held sets of small endings at 74 M jobs/s.
+enum { FLAG_SHIFT = 21 };
+__device__ __forceinline__ u32 flag_turn() { return (u32)(clock64() >> FLAG_SHIFT); }
 __device__ __forceinline__ int warp_ask(WarpBlock* sh, u64 t_end) {
   const BatchArgs& a = sh->args;
   volatile int* halt = &sh->halt;
-  if ((atomicAdd(&sh->asks, 1u) & 63u) == 63u && a.stop && *a.stop) *halt = 1;
+  const u32 turn = flag_turn();
+  if (turn != *reinterpret_cast<volatile u32*>(&sh->turn) && atomicExch(&sh->turn, turn) != turn && a.stop && *a.stop) *halt = 1;
   return *halt | (int)(t_end && global_ns() > t_end);
 }
 
@@ -243,7 +247,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) warp_kernel(BatchArgs a) {
     sh.args = a;
     sh.idle_since = 0;
     sh.polling = sh.busy = sh.idle_exit = sh.running = 0;
-    sh.polls = sh.asks = 0;
+    sh.polls = 0;
+    sh.turn = flag_turn();
     sh.halt = 0;
     sh.nodes = sh.jobs_done = 0;
     for (int k = 0; k < WCNT_COUNT; k++) sh.total[k] = 0;
