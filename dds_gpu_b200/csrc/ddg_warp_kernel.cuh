@@ -59,9 +59,10 @@ inline size_t warp_smem(int warps) { return sizeof(WarpBlock) + sizeof(WarpMem) 
 // start after 256 nodes and before a job is taken. The host's flag is a read over the bus, and the
 // GPU does about 1.15 M of those a second however many SMs ask (one read by every searcher each
 // 1,024 nodes held the whole GPU at 1.18 G nodes/s). So a block reads it once in 2^FLAG_SHIFT
-// clock cycles, about a millisecond: the first question after that does, and the others see what
-// it found. Counted in questions instead, one in 64, it held sets of small endings at 74 M jobs/s.
-enum { FLAG_SHIFT = 21 };
+// clock cycles, about four milliseconds: the first question after that does, and the others see
+// what it found. Counted in questions instead, one in 64, it held sets of small endings at 74 M
+// jobs/s; read each millisecond, a search alone on an SM was 0.1 % slower (29.82 against 29.77 ms).
+enum { FLAG_SHIFT = 23 };
 __device__ __forceinline__ u32 flag_turn() { return (u32)(clock64() >> FLAG_SHIFT); }
 __device__ __forceinline__ int warp_ask(WarpBlock* sh, u64 t_end) {
   const BatchArgs& a = sh->args;
